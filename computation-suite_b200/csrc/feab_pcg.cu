@@ -14,6 +14,7 @@
 // results are bit-reproducible.  A chunk of steps is captured once in a CUDA graph and replayed;
 // kernels return at once when the state says done, and the host polls the done flag one chunk
 // behind, so there is no host sync per iteration.
+// Sliced operators of up to 8 slices per SM run as one kernel instead (feab_pcg_resident.cuh).
 //
 // Precisions (feab_pcg_params.precision):
 //   FEAB_PREC_FP64   the reference recurrence (iterative_solvers.py:434-481) in FP64.
@@ -69,6 +70,7 @@ struct PcgArgs {
   double *x64a, *x64b, *r64;         // fp32 mode: FP64 solution ping-pong + FP64 residual
   float *r32, *z32, *q0, *q1, *Ap32, *x32;  // fp32 mode vectors (q = p)
   int use_dinv;
+  ulonglong2* inbox;       // the resident solve's inboxes (NULL: none in the workspace)
 };
 
 __device__ __forceinline__ bool last_block_of(uint32_t* ticket) {
@@ -737,6 +739,14 @@ __global__ void __launch_bounds__(kThreads) k_build_diff(int32_t n_groups, const
   }
 }
 
+}  // namespace
+}  // namespace feab
+
+#include "feab_pcg_resident.cuh"
+
+namespace feab {
+namespace {
+
 size_t a256(size_t b) { return (b + 255) & ~size_t(255); }
 
 int max_grid() { return sm_count() * 8; }
@@ -838,6 +848,89 @@ void launch_step_sell(const PcgArgs& A, const Grids& gr, cudaStream_t s) {
   k_step_b<PREC><<<gr.b, kThreads, 0, s>>>(A);
 }
 
+// The resident solve's inboxes (after the work vectors), for the sizes it can take.
+size_t resident_bytes(int32_t n, int32_t precision) {
+  if (precision == FEAB_PREC_FP32 || n > 96 * kResMaxSlices * std::min(sm_count(), kResMaxCtas)) return 0;
+  return 2 * sizeof(ulonglong2) * (size_t)kResMaxCtas * (size_t)kResMaxCtas;
+}
+
+// How an operator of ns slices is spread: one cluster of up to 16 CTAs for up to 48 slices (3 per
+// CTA), whose sums cost half of a grid-wide one (measured: 1,700 cycles with 16 CTAs, against 3,700
+// with 16, 4,200 with 64 and 5,500 with 148 CTAs across the grid); else two slices per CTA while
+// that takes fewer CTAs than there are SMs.  0 CTAs: too large.
+struct ResShape {
+  int ctas;
+  bool cluster;
+};
+
+ResShape resident_shape(int ns) {
+  if (ns <= 3 * kResMaxCluster) return {std::min(ns, kResMaxCluster), true};
+  const int sms = std::min(sm_count(), kResMaxCtas), ctas = std::min(sms, (ns + 1) / 2);
+  return {(ns + ctas - 1) / ctas <= kResMaxSlices ? ctas : 0, false};
+}
+
+template <int KIND, bool IDX16>
+const void* resident_kernel(bool cluster, int slices) {
+  if (cluster) return (const void*)k_pcg_resident<KIND, IDX16, true, 1>;
+  return 96 * slices <= kResThreads ? (const void*)k_pcg_resident<KIND, IDX16, false, 1>
+                                    : (const void*)k_pcg_resident<KIND, IDX16, false, 2>;
+}
+
+constexpr int kResSteps = 4096;   // iterations of one launch (at most some 0.1 s)
+
+// Launches the resident solve of A (setup done) with at most kResSteps iterations; `resume` continues
+// an earlier launch.  cudaErrorNotSupported: use the step kernels.
+cudaError_t launch_resident(const PcgArgs& A, int prec, bool resume, cudaStream_t s) {
+  if (!A.inbox || (reinterpret_cast<uintptr_t>(A.z) & 15u)) return cudaErrorNotSupported;
+  ResShape shape = resident_shape(A.sell.n_slices);
+  if (shape.ctas == 0) return cudaErrorNotSupported;
+  ResArgs Q{};
+  Q.inbox = A.inbox;
+  Q.zp[0] = reinterpret_cast<double2*>(A.z);
+  Q.zp[1] = reinterpret_cast<double2*>(A.p1);
+  Q.resume = resume ? 1 : 0;
+  Q.max_steps = kResSteps;
+  Q.smem_bytes = kResSmem;
+  const bool i16 = A.sell.tcol16 != nullptr;
+  const int per = (A.sell.n_slices + shape.ctas - 1) / shape.ctas;
+  const void* fn;
+  if (prec == FEAB_PREC_MIXED)
+    fn = i16 ? resident_kernel<FEAB_PREC_MIXED, true>(shape.cluster, per)
+             : resident_kernel<FEAB_PREC_MIXED, false>(shape.cluster, per);
+  else
+    fn = i16 ? resident_kernel<FEAB_PREC_FP64, true>(shape.cluster, per)
+             : resident_kernel<FEAB_PREC_FP64, false>(shape.cluster, per);
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem);
+  if (e == cudaSuccess && shape.cluster) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess && !shape.cluster)
+    e = cudaMemsetAsync(A.inbox, 0, 2 * sizeof(ulonglong2) * (size_t)shape.ctas * (size_t)shape.ctas, s);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(shape.ctas);
+  cfg.blockDim = dim3(kResThreads);
+  cfg.dynamicSmemBytes = kResSmem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  if (shape.cluster) {
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = shape.ctas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  } else {
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+  }
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  void* args[2] = {const_cast<PcgArgs*>(&A), &Q};
+  e = cudaLaunchKernelExC(&cfg, fn, args);
+  if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorInvalidClusterSize || e == cudaErrorLaunchOutOfResources) {
+    cudaGetLastError();   // a device with fewer SMs at hand: the step kernels run on any
+    return cudaErrorNotSupported;
+  }
+  if (e == cudaSuccess) count_launches(1);
+  return e;
+}
+
 int normalize_lpg(int lpg) { return lpg == 4 || lpg == 8 || lpg == 16 || lpg == 32 ? lpg : 16; }
 
 int32_t run_pcg(const PcgArgs& A, int prec, int chunk, int maxiter, int lpg, feab_pcg_result* result,
@@ -860,7 +953,33 @@ int32_t run_pcg(const PcgArgs& A, int prec, int chunk, int maxiter, int lpg, fea
     if (e != cudaSuccess && rc == FEAB_OK) rc = FEAB_CUDA_ERROR;
     return e != cudaSuccess;
   };
-  do {
+  bool resident = A.use_sell != 0;
+  // every launch runs kResSteps iterations unless the solve ends, so maxiter bounds the launches
+  for (int64_t it = 0; resident && it <= maxiter; it += kResSteps) {
+    const cudaError_t e = launch_resident(A, prec, it > 0, s);
+    if (e == cudaErrorNotSupported && it == 0) {
+      resident = false;
+      break;
+    }
+    if (fail(e)) break;
+    ++launched;
+    if (fail(cudaMemcpyAsync((void*)flag.ptr, &A.S_->done, sizeof(int32_t), cudaMemcpyDeviceToHost, s))) break;
+    if (fail(cudaStreamSynchronize(s))) break;
+    if (flag.ptr[0] == kResMisfit) {
+      // a CTA's rows refer to more of p than its shared memory holds: nothing was done, but z and
+      // p were written over
+      resident = false;
+      launched = 0;
+      if (fail(cudaMemsetAsync(&A.S_->done, 0, sizeof(int32_t), s))) break;
+      if (prec == FEAB_PREC_MIXED) k_setup_b<FEAB_PREC_MIXED><<<gr.b, kThreads, 0, s>>>(A);
+      else k_setup_b<FEAB_PREC_FP64><<<gr.b, kThreads, 0, s>>>(A);
+      count_launches(1);
+      fail(cudaGetLastError());
+      break;
+    }
+    if (flag.ptr[0] != 0) break;
+  }
+  if (!resident && rc == FEAB_OK) do {
     if (fail(graphs.events(ev))) break;
     // the chunk's launches bake in A, the launch shapes and the chunk length
     const uint64_t topo = topo_signature({prec, chunk, lpg, A.use_sell, gr.a, gr.b, A.use_sell ? sell_grid(A) : 0,
@@ -1009,7 +1128,7 @@ using namespace feab;
 
 extern "C" size_t feab_pcg_workspace_bytes(int32_t n, int32_t precision) {
   if (n < 0 || precision < FEAB_PREC_FP64 || precision > FEAB_PREC_FP32) return 0;
-  return layout(n, precision, nullptr, nullptr);
+  return layout(n, precision, nullptr, nullptr) + resident_bytes(n, precision);
 }
 
 extern "C" size_t feab_diff_operator_bytes(int32_t n, int64_t nnz, int32_t n_groups) {
@@ -1062,7 +1181,10 @@ extern "C" int32_t feab_pcg_solve(const feab_csr* M, const feab_sell_operator* s
   if (M->group_ptr && M->n_groups <= 0) return FEAB_BAD_ARG;
   if (!(prm->tol >= 0.0)) return FEAB_BAD_ARG;
   PcgArgs A{};
-  if (layout(M->n, prec, static_cast<char*>(workspace), &A) > workspace_bytes) return FEAB_BAD_ARG;
+  const size_t used = layout(M->n, prec, static_cast<char*>(workspace), &A), inbox = resident_bytes(M->n, prec);
+  if (used > workspace_bytes) return FEAB_BAD_ARG;
+  if (inbox && used + inbox <= workspace_bytes)
+    A.inbox = reinterpret_cast<ulonglong2*>(static_cast<char*>(workspace) + used);
   fill_matrix(M, &A);
   if (sell && prec != FEAB_PREC_FP32) fill_sell(M, sell, &A);
   A.dinv64 = dinv64;
