@@ -1212,22 +1212,25 @@ int32_t run_block(BArgs A, int prec, int chunk, int maxiter, cudaStream_t s, int
           k_bstep_b<K, false><<<grid_pb, kThreads, 0, cs>>>(A);
         }
       }
-      cudaMemcpyAsync((void*)hflag, A.remaining, sizeof(int32_t), cudaMemcpyDeviceToHost, cs);
+    };
+    // the copy of the counter stays out of the cached graph (see run_pcg)
+    auto launch_chunk = [&](cudaEvent_t behind) {
+      return fail(cudaGraphLaunch(exec, s)) ||
+             fail(cudaMemcpyAsync((void*)hflag, A.remaining, sizeof(int32_t), cudaMemcpyDeviceToHost, s)) ||
+             fail(cudaEventRecord(behind, s));
     };
     if (fail(graphs.acquire(&A, sizeof(A), topo_signature({K, prec, chunk, grid, grid_pb, tiles ? 1 : 0}), record, &exec))) break;
     // iterations and reliable steps per problem are bounded by maxiter each
     const int64_t max_launch = (2 * (int64_t)maxiter + 2 + chunk - 1) / chunk + 1;
     hflag[0] = np;
     int64_t launched = 0;
-    if (fail(cudaGraphLaunch(exec, s))) break;
-    if (fail(cudaEventRecord(ev[0], s))) break;
+    if (launch_chunk(ev[0])) break;
     launched = 1;
     count_launches(3 * (uint64_t)chunk);
     while (true) {
       const bool more = launched < max_launch;
       if (more) {
-        if (fail(cudaGraphLaunch(exec, s))) break;
-        if (fail(cudaEventRecord(ev[launched & 1], s))) break;
+        if (launch_chunk(ev[launched & 1])) break;
         ++launched;
         count_launches(3 * (uint64_t)chunk);
       }

@@ -991,7 +991,14 @@ int32_t run_pcg(const PcgArgs& A, int prec, int chunk, int maxiter, int lpg, fea
         else if (A.use_sell) launch_step_sell<FEAB_PREC_FP64>(A, gr, cs);
         else launch_step<FEAB_PREC_FP64>(A, gr, lpg, cs);
       }
-      cudaMemcpyAsync((void*)flag.ptr, &A.S_->done, sizeof(int32_t), cudaMemcpyDeviceToHost, cs);
+    };
+    // one chunk and, behind it, the copy of the done flag.  The copy is not part of the graph: a
+    // cached graph outlives the workspace, and updating a graph whose copy reads memory that has
+    // been given back to the driver since crashes in cudaGraphExecUpdate.
+    auto launch_chunk = [&](cudaEvent_t behind) {
+      return fail(cudaGraphLaunch(exec, s)) ||
+             fail(cudaMemcpyAsync((void*)flag.ptr, &A.S_->done, sizeof(int32_t), cudaMemcpyDeviceToHost, s)) ||
+             fail(cudaEventRecord(behind, s));
     };
     if (fail(graphs.acquire(&A, sizeof(A), topo, record, &exec))) break;
 
@@ -999,16 +1006,14 @@ int32_t run_pcg(const PcgArgs& A, int prec, int chunk, int maxiter, int lpg, fea
     // 2*maxiter + 2 steps always suffice: the host loop is bounded.
     const int64_t max_launch = (2 * (int64_t)maxiter + 2 + chunk - 1) / chunk + 1;
     flag.ptr[0] = 0;
-    if (fail(cudaGraphLaunch(exec, s))) break;
-    if (fail(cudaEventRecord(ev[0], s))) break;
+    if (launch_chunk(ev[0])) break;
     launched = 1;
     const uint64_t per_step = A.use_sell ? (FEAB_SELL_FUSED_P ? 2 : 3) : 2;
     count_launches(per_step * (uint64_t)chunk);
     while (true) {
       const bool more = launched < max_launch;
       if (more) {
-        if (fail(cudaGraphLaunch(exec, s))) break;
-        if (fail(cudaEventRecord(ev[launched & 1], s))) break;
+        if (launch_chunk(ev[launched & 1])) break;
         ++launched;
         count_launches(per_step * (uint64_t)chunk);
       }

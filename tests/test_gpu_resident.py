@@ -85,3 +85,18 @@ def test_start_vector_and_iteration_limit():
     assert warm.status == 0 and warm.iters <= 2
     rest, more = pcg_solve(op, b, tol=1e-10, x0=half)
     assert more.status == 0 and float((rest - x).norm() / x.norm()) < 1e-6
+
+
+def test_solves_after_memory_went_back_to_the_driver():
+    """A cached graph outlives the workspace it was captured with."""
+    from feab200.batched import block_pcg
+    from feab200.device import pcg_solve
+    for shape in ((20, 4, 4), (20, 4, 5), (20, 4, 4)):
+        op = _operator(*shape)
+        b = torch.as_tensor(np.random.default_rng(9).standard_normal(op.n)).cuda()
+        x, info = pcg_solve(op, b, tol=1e-9, layout="csr", lanes_per_group=8)
+        X, res = block_pcg(op, [0, op.n], b[:, None].repeat(1, 16), [16], tol=1e-9, tune=False)
+        assert info.status == 0 and (res.status == 0).all()
+        assert float((X - x[:, None]).norm() / X.norm()) < 1e-6
+        del op, b, x, X
+        torch.cuda.empty_cache()
