@@ -8,15 +8,10 @@
 // The caller renumbers the rows (a bandwidth-reducing order) so that every nonzero lies within
 // `bandwidth` of the diagonal.  The lower band is kept as 64 x 64 tiles: block row I holds the
 // tiles of block columns I - bands .. I, tile (I, d) being block column I - d.  The fill of a
-// Cholesky factor stays inside the band, so the factorisation is a right-looking tile algorithm
-// over block columns K = 0 .. n_tiles - 1:
-//   1. factor the diagonal tile (K, K) in shared memory (k_band_potrf);
-//      and invert its factor, Linv_KK = L_KK^{-1} (kept beside the band);
-//   2. form the tiles below it, L_IK = A_IK Linv_KK^T, one CTA per tile;
-//   3. update the trailing band, A_IJ -= L_IK L_JK^T for K < J <= I <= K + bands, one CTA per
-//      tile (k_band_tile_gemm: 64 x 64 x 64 FP64 products on the FP64 tensor path, mma.sync).
-// Applying the inverted 64 x 64 diagonal factors (as blocked GPU triangular solvers do) turns the
-// per-column triangular solves into tile products, so only step 1 is sequential within a column.
+// Cholesky factor stays inside the band, so the factorisation is a tile algorithm over block columns
+// J = 0 .. n_tiles - 1: the diagonal tile is factored and its factor inverted (Linv_JJ, kept beside
+// the band), and the tiles below it are L_IJ = (A_IJ - sum_K L_IK L_JK^T) Linv_JJ^T, products of 64 x
+// 64 tiles on the FP64 tensor path (mma.sync).  It runs as one kernel (k_band_factor).
 // The solves walk the block rows forward (L y = b) and backward (L^T x = y), one kernel per block
 // row: each CTA forms the block's y_K = Linv_KK w_K (or x_K = Linv_KK^T w_K) and then applies one
 // off-diagonal tile to a later (earlier) block of the right-hand side.
@@ -30,7 +25,6 @@ namespace {
 
 constexpr int kT = FEAB_BAND_TILE;       // tile edge
 constexpr int kTile = kT * kT;           // doubles per tile
-constexpr int kLd = kT + 1;              // shared-memory row stride of a staged triangle
 
 __host__ __device__ inline size_t tile_index(int I, int d, int bands) {
   return ((size_t)I * (size_t)(bands + 1) + (size_t)d) * (size_t)kTile;
@@ -104,162 +98,41 @@ struct BandState {
 };
 static_assert(sizeof(BandState) <= FEAB_BAND_HEADER_BYTES, "band header");
 
-// Cholesky of the diagonal tile (K, K), then the inverse of its factor.  The tile lives in
-// registers, a 4 x 4 block per thread (16 x 16 threads).  The right-looking elimination keeps the
-// columns unscaled (A_ij -= A_ik A_jk / p_k for j > k): the owners of column k + 1 copy it into a
-// shared double buffer after their step-k update, and the owner of its diagonal entry stores
-// 1 / p_{k+1}, so one barrier separates the steps.  The columns are scaled by 1 / sqrt(p_k) at the
-// end.  Pivots of rows < n are recorded (a pivot <= 0 sets FEAB_NOT_SPD and is replaced by 1 so the
-// kernel finishes).  Linv = L_KK^{-1} (lower triangular) is then formed the same way: X = I in
-// registers, and for each row m, X_m = X_m / L_mm is published and X_i -= L_im X_m for i > m.
-__global__ void __launch_bounds__(256) k_band_potrf(double* __restrict__ tiles, double* __restrict__ inv, int bands,
-                                                   int K, int32_t n, BandState* st) {
-  __shared__ double colbuf[2][kT];
-  __shared__ double rpbuf[2];
-  __shared__ double piv[kT];
-  __shared__ double rowbuf[2][kT];
-  extern __shared__ __align__(16) double psm[];  // the factor L (dynamic: 33 KB)
-  double (*Ls)[kLd] = reinterpret_cast<double (*)[kLd]>(psm);
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  double* T = tiles + tile_index(K, 0, bands);
-  double a[4][4];
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const double2 p0 = *reinterpret_cast<const double2*>(T + (4 * ty + u) * kT + 4 * tx);
-    const double2 p1 = *reinterpret_cast<const double2*>(T + (4 * ty + u) * kT + 4 * tx + 2);
-    a[u][0] = p0.x;
-    a[u][1] = p0.y;
-    a[u][2] = p1.x;
-    a[u][3] = p1.y;
-  }
-  // a[u][v] for run-time u, v, selected without indexing the register array
-  auto row = [&](int u, int v) {
-    return v == 0 ? a[u][0] : v == 1 ? a[u][1] : v == 2 ? a[u][2] : a[u][3];
-  };
-  auto sel = [&](int u, int v) {
-    return u == 0 ? row(0, v) : u == 1 ? row(1, v) : u == 2 ? row(2, v) : row(3, v);
-  };
-  if (tx == 0) {
-#pragma unroll
-    for (int u = 0; u < 4; ++u) colbuf[0][4 * ty + u] = a[u][0];
-    if (ty == 0) {
-      const double p = a[0][0] > 0.0 ? a[0][0] : 1.0;
-      rpbuf[0] = 1.0 / p;
-    }
-  }
-  double pmin = INFINITY, pmax = 0.0;
-  bool bad = false;
-  for (int k = 0; k < kT; ++k) {
-    __syncthreads();
-    const double* col = colbuf[k & 1];
-    const double rp = rpbuf[k & 1];
-    if (tid == 0) {
-      const double p0 = col[k];
-      if (K * kT + k < n) {
-        if (p0 > 0.0) {
-          pmin = fmin(pmin, p0);
-          pmax = fmax(pmax, p0);
-        } else {
-          bad = true;
-        }
-      }
-      piv[k] = p0 > 0.0 ? p0 : 1.0;
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int i = 4 * ty + u;
-      const double ci = col[i] * rp;
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const int jj = 4 * tx + v;
-        if (jj > k && i >= jj) a[u][v] -= ci * col[jj];
-      }
-    }
-    const int k1 = k + 1;
-    if (k1 < kT && tx == (k1 >> 2)) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) colbuf[k1 & 1][4 * ty + u] = sel(u, k1 & 3);
-      if (ty == (k1 >> 2)) {
-        const double p = sel(k1 & 3, k1 & 3);
-        rpbuf[k1 & 1] = 1.0 / (p > 0.0 ? p : 1.0);
-      }
-    }
-  }
-  if (tid == 0) {
-    if (pmax > 0.0) {
-      atomicMin(&st->piv_min, (unsigned long long)__double_as_longlong(pmin));
-      atomicMax(&st->piv_max, (unsigned long long)__double_as_longlong(pmax));
-    }
-    if (bad) atomicCAS(&st->status, FEAB_OK, FEAB_NOT_SPD);
-  }
-  __syncthreads();
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int i = 4 * ty + u;
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int jj = 4 * tx + v;
-      const double l = i > jj ? a[u][v] * rsqrt(piv[jj]) : (i == jj ? sqrt(piv[jj]) : 0.0);
-      Ls[i][jj] = l;
-      a[u][v] = l;
-    }
-    // the whole tile is written, with zeros above the diagonal
-    *reinterpret_cast<double2*>(T + i * kT + 4 * tx) = make_double2(a[u][0], a[u][1]);
-    *reinterpret_cast<double2*>(T + i * kT + 4 * tx + 2) = make_double2(a[u][2], a[u][3]);
-  }
-  // Linv: X = I; row m final after dividing by L_mm; rows below take X_i -= L_im X_m
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v) a[u][v] = (4 * ty + u == 4 * tx + v) ? 1.0 : 0.0;
-  __syncthreads();
-  if (ty == 0) {
-    const double rl = 1.0 / Ls[0][0];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) rowbuf[0][4 * tx + v] = a[0][v] * rl;
-  }
-  for (int m = 0; m < kT; ++m) {
-    __syncthreads();
-    const double* xm = rowbuf[m & 1];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int i = 4 * ty + u;
-      if (i == m) {
-#pragma unroll
-        for (int v = 0; v < 4; ++v) a[u][v] = xm[4 * tx + v];
-      } else if (i > m) {
-        const double lim = Ls[i][m];
-#pragma unroll
-        for (int v = 0; v < 4; ++v) a[u][v] -= lim * xm[4 * tx + v];
-      }
-    }
-    const int m1 = m + 1;
-    if (m1 < kT && ty == (m1 >> 2)) {
-      const double rl = 1.0 / Ls[m1][m1];
-      const int u = m1 & 3;
-#pragma unroll
-      for (int v = 0; v < 4; ++v) rowbuf[m1 & 1][4 * tx + v] = sel(u, v) * rl;
-    }
-  }
-  double* Iv = inv + (size_t)K * kTile;
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int i = 4 * ty + u;
-    *reinterpret_cast<double2*>(Iv + i * kT + 4 * tx) = make_double2(a[u][0], a[u][1]);
-    *reinterpret_cast<double2*>(Iv + i * kT + 4 * tx + 2) = make_double2(a[u][2], a[u][3]);
-  }
-}
+// The factorisation is one cooperative kernel, so that a block column costs what its dependences
+// cost and not three launches.  CTA 0 walks the diagonal (the chain): for block row J it forms
+// L_{J,J-1} = C_{J,J-1} Linv_{J-1}^T, takes it from the diagonal tile, factors that tile and inverts
+// the factor.  The other CTAs (workers) draw tasks, each one tile of the band brought up to date
+// left-looking, in one go: C_IJ = A_IJ - sum_K L_IK L_JK^T, and for tiles at least two below the
+// diagonal L_IJ = C_IJ Linv_J^T.  The two tiles of a row that the chain needs next are left as C
+// (without the last term, which the chain adds).  Progress is published per block row: progress[I]
+// = K + 1 once L_IK is stored (a row's tiles finish in order of K), prepared[I] counts the two
+// tiles left for the chain.  Tasks are drawn in an order in which each depends only on tasks before
+// it and on the chain, and all CTAs run at once, so every wait ends; each is bounded all the same
+// and a CTA whose wait runs out makes all leave with an error.
+//
+// What bounds it: the chain, as long as the workers keep up (b (b + 1) / 2 tile products per block
+// column over 147 SMs), else the FP64 tensor path.  Of the chain's 14.5 us per block column the 64
+// pivots take 6.5 (a reciprocal square root, a product and a difference, 16 cycles each, one after
+// the other), the two products 3.2, the inverse 2.7.  Measured, three launches per block column ->
+// one kernel: 64x16x16 elements (867 block columns, 28 bands) 74.2 -> 12.6 ms, 96x24x24 (2,813, 59
+// bands, bound by the workers at 22 TFLOP/s) 335 -> 118 ms, 33x9x8 (140, 9 bands) 10.6 -> 2.0 ms.
 
-// C (op)= A B^T for 64 x 64 tiles on the FP64 tensor path (mma.sync m8n8k4), one CTA per output
-// tile: warp w owns rows 8 w .. 8 w + 7 and all 64 columns (eight 8 x 8 accumulators), and walks k
-// in steps of 4.  Fragments (m8n8k4, .f64): A row-major 8 x 4, lane l holds (l / 4, l % 4); B
-// column-major 4 x 8, lane l holds (l % 4, l / 4); C 8 x 8, lane l holds (l / 4, 2 (l % 4) + i).
-// Both factors are staged row-major in shared memory with a padded row (kMmaLd doubles), so each
-// fragment load of a half-warp touches 16 distinct banks.
-//   UPDATE: the trailing update of block column K, CTA a -> (I, J) with K < J <= I, a = (I - K - 1)
-//           (I - K) / 2 + (J - K - 1): A_IJ -= L_IK L_JK^T;
-//   PANEL:  the panel below the diagonal tile, CTA b -> I = K + 1 + b: L_IK = A_IK Linv_KK^T.
-constexpr int kMmaLd = kT + 4;
+struct BandWork {
+  double* tiles;
+  double* inv;
+  BandState* st;
+  int32_t* progress;   // n_tiles
+  int32_t* prepared;   // n_tiles
+  int32_t* next_task;
+  int32_t* abort_flag;
+  int32_t n, n_tiles, bands;
+};
+
+constexpr int kBandThreads = 256;
+constexpr int kMmaLd = kT + 4;                 // row stride of a staged tile: no bank conflicts between fragments
+constexpr int kStage = kT * kMmaLd;            // doubles of a staged tile
+constexpr size_t kFactorSmem = 6 * kStage * sizeof(double);   // of the chain; the workers use four stages
+constexpr int kBandSpinLimit = 1 << 22;        // polls before a wait gives up (seconds)
 
 __device__ __forceinline__ void dmma884(double (&d)[2], double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
@@ -267,68 +140,529 @@ __device__ __forceinline__ void dmma884(double (&d)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
-template <bool PANEL>
-__global__ void __launch_bounds__(256) k_band_tile_gemm(double* __restrict__ tiles, const double* __restrict__ inv,
-                                                       int bands, int K) {
-  extern __shared__ __align__(16) double gsm[];
-  double* As = gsm;                  // As[r * kMmaLd + k] = A[r][k]
-  double* Bs = gsm + kT * kMmaLd;    // Bs[c * kMmaLd + k] = B[c][k]
-  const double* Ap;
-  const double* Bp;
-  double* Cp;
-  if (PANEL) {
-    const int I = K + 1 + blockIdx.x;
-    Ap = tiles + tile_index(I, I - K, bands);
-    Bp = inv + (size_t)K * kTile;
-    Cp = tiles + tile_index(I, I - K, bands);
-  } else {
-    const int a = blockIdx.x;
-    int io = (int)((sqrt(8.0 * a + 1.0) - 1.0) * 0.5);
-    while ((io + 1) * (io + 2) / 2 <= a) ++io;
-    while (io * (io + 1) / 2 > a) --io;
-    const int jo = a - io * (io + 1) / 2;
-    const int I = K + 1 + io, J = K + 1 + jo;
-    Ap = tiles + tile_index(I, I - K, bands);
-    Bp = tiles + tile_index(J, J - K, bands);
-    Cp = tiles + tile_index(I, I - J, bands);
-  }
-  for (int q = threadIdx.x; q < kTile / 2; q += blockDim.x) {
-    const int row = q / (kT / 2), k2 = q % (kT / 2);
-    *reinterpret_cast<double2*>(As + row * kMmaLd + 2 * k2) = reinterpret_cast<const double2*>(Ap)[q];
-    *reinterpret_cast<double2*>(Bs + row * kMmaLd + 2 * k2) = reinterpret_cast<const double2*>(Bp)[q];
-  }
+__device__ __forceinline__ int32_t ld_relaxed(const int32_t* p) {
+  int32_t v;
+  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_relaxed(int32_t* p, int32_t v) {
+  asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
+// All threads, after their stores: `where` becomes `value` (0: it is counted up) once the stores are
+// visible to every CTA.  One thread of warp 1 waits for that (a thousand cycles); the others go on.
+__device__ __forceinline__ void publish(int32_t* where, int32_t value) {
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  double acc[8][2];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) acc[j][0] = acc[j][1] = 0.0;
-  const double* Arow = As + (8 * warp + g) * kMmaLd + t;
-  const double* Bcol = Bs + g * kMmaLd + t;
-#pragma unroll 4
-  for (int k0 = 0; k0 < kT; k0 += 4) {
-    const double a = Arow[k0];
-    double b[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) b[j] = Bcol[8 * j * kMmaLd + k0];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) dmma884(acc[j], a, b[j]);
+  if (threadIdx.x == 32) {
+    fence_gpu();
+    if (value) st_relaxed(where, value);
+    else atomicAdd(where, 1);
   }
-  const int r = 8 * warp + g;
+}
+
+// One thread: waits until *p >= want.  False (and every CTA told) when that takes too long.
+__device__ __forceinline__ bool wait_for(const int32_t* p, int32_t want, int32_t* abort_flag) {
+  for (int spin = 0; ld_relaxed(p) < want; ++spin) {
+    if (spin >= kBandSpinLimit) atomicExch(abort_flag, 1);
+    if ((spin & 255) == 255 && ld_relaxed(abort_flag)) return false;
+  }
+  fence_gpu();
+  return true;
+}
+
+// Asynchronous copy of a tile into its padded stage (all threads; commit and wait are the caller's).
+__device__ __forceinline__ void stage_tile(double* dst, const double* src) {
+  for (int q = threadIdx.x; q < kTile / 2; q += kBandThreads) {
+    const int row = q / (kT / 2), k2 = q % (kT / 2);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(dst + row * kMmaLd + 2 * k2)),
+                 "l"(src + 2 * (size_t)q)
+                 : "memory");
+  }
+}
+__device__ __forceinline__ void stage_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void stage_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// acc += A B^T of two staged 64 x 64 tiles, on the FP64 tensor path: warp w owns rows 16 (w / 2) .. + 15
+// and 32 columns as 2 x 4 accumulators; the column half changes sides at warp 4, so that each
+// scheduler (warps w and w + 4) has one warp of either half.  TRI: B is lower triangular, columns k
+// past the output column are zero and left out.  LOWER: only blocks on or below the diagonal.  Fragments (m8n8k4): A
+// row-major 8 x 4, lane l holds (l / 4, l % 4); B column-major 4 x 8, lane l holds (l % 4, l / 4); C
+// 8 x 8, lane l holds (l / 4, 2 (l % 4) + i).
+typedef double TileAcc[2][4][2];
+
+__device__ __forceinline__ void tile_zero(TileAcc& acc) {
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    double2* c = reinterpret_cast<double2*>(Cp + (size_t)r * kT + 8 * j + 2 * t);
-    if (PANEL) {
-      *c = make_double2(acc[j][0], acc[j][1]);
-    } else {
-      double2 cv = *c;
-      cv.x -= acc[j][0];
-      cv.y -= acc[j][1];
-      *c = cv;
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+}
+
+__device__ __forceinline__ int tile_row0() { return 16 * (threadIdx.x >> 6); }
+__device__ __forceinline__ int tile_col0() { return 32 * (((threadIdx.x >> 5) ^ (threadIdx.x >> 7)) & 1); }
+
+template <bool TRI, bool LOWER>
+__device__ __forceinline__ void tile_mma(const double* As, const double* Bs, TileAcc& acc) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, row0 = tile_row0(), col0 = tile_col0();
+  if (LOWER && col0 > row0 + 15) return;
+  const double* Ar = As + (row0 + g) * kMmaLd + t;
+  const double* Br = Bs + (col0 + g) * kMmaLd + t;
+  const int kend = TRI ? col0 + 32 : kT;
+#pragma unroll 4
+  for (int k0 = 0; k0 < kend; k0 += 4) {
+    const double a0 = Ar[k0], a1 = Ar[8 * kMmaLd + k0];
+    double b[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) b[j] = Br[8 * j * kMmaLd + k0];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (TRI && k0 >= col0 + 8 * j + 8) continue;
+      if (!LOWER || col0 + 8 * j <= row0) dmma884(acc[0][j], a0, b[j]);
+      if (!LOWER || col0 + 8 * j <= row0 + 8) dmma884(acc[1][j], a1, b[j]);
     }
   }
 }
-constexpr size_t kGemmSmem = 2 * kT * kMmaLd * sizeof(double);
-constexpr size_t kPotrfSmem = kT * kLd * sizeof(double);
+
+// The accumulators' places in a tile of row stride ld: fn(offset of two adjacent columns, i, j).
+template <typename F>
+__device__ __forceinline__ void tile_each(int ld, F fn) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) fn((tile_row0() + 8 * i + g) * ld + tile_col0() + 8 * j + 2 * t, i, j);
+}
+
+// C -= L L^T on the blocks on or below the diagonal: warp w < 4 block row w, warp w >= 4 block row
+// 11 - w, so that each scheduler has nine blocks.  NB: blocks of the block row.
+template <int NB>
+__device__ __forceinline__ void syrk_row(const double* Ls, double* C) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  double acc[NB][2];
+#pragma unroll
+  for (int j = 0; j < NB; ++j) acc[j][0] = acc[j][1] = 0.0;
+  const double* Ar = Ls + (8 * (NB - 1) + g) * kMmaLd + t;
+  const double* Br = Ls + g * kMmaLd + t;
+#pragma unroll 4
+  for (int k0 = 0; k0 < kT; k0 += 4) {
+    const double a = Ar[k0];
+    double b[NB];
+#pragma unroll
+    for (int j = 0; j < NB; ++j) b[j] = Br[8 * j * kMmaLd + k0];
+#pragma unroll
+    for (int j = 0; j < NB; ++j) dmma884(acc[j], a, b[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < NB; ++j) {
+    double2* c = reinterpret_cast<double2*>(C + (8 * (NB - 1) + g) * kMmaLd + 8 * j + 2 * t);
+    double2 v = *c;
+    v.x -= acc[j][0];
+    v.y -= acc[j][1];
+    *c = v;
+  }
+}
+
+__device__ __forceinline__ void tile_syrk(const double* Ls, double* C) {
+  switch (threadIdx.x >> 5) {
+    case 0: syrk_row<1>(Ls, C); break;
+    case 1: syrk_row<2>(Ls, C); break;
+    case 2: syrk_row<3>(Ls, C); break;
+    case 3: syrk_row<4>(Ls, C); break;
+    case 4: syrk_row<8>(Ls, C); break;
+    case 5: syrk_row<7>(Ls, C); break;
+    case 6: syrk_row<6>(Ls, C); break;
+    default: syrk_row<5>(Ls, C); break;
+  }
+}
+
+// C B^T of an 8 x 8 block: rows at A, columns' rows at B, eight columns of k; one warp.
+__device__ __forceinline__ void mma8(double (&c)[2], const double* A, const double* B, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int k0 = 0; k0 < 8; k0 += 4) dmma884(c, A[g * kMmaLd + k0 + t], B[g * kMmaLd + k0 + t]);
+}
+
+// Cholesky of the staged tile C (lower part), L in its place with zeros above the diagonal, and the
+// inverse of L in X (W: scratch).  Panels of 8 columns: warp 0 factors a panel in registers, a lane
+// per two rows, every lane carrying the 8 x 8 diagonal block along so that no pivot crosses lanes,
+// while the other warps apply the panel before it to the columns behind.  pivot[] takes the pivots; one
+// that is not > 0 counts as 1.  The inverse is put together from the inverses of the 8 x 8 diagonal
+// blocks, doubling the block: X_21 = -X_22 (L_21 X_11).  after_panels() runs between the two parts.
+struct TileScratch {
+  double pivot[kT];
+  double rsq[kT];   // pivot^(-1/2)
+};
+
+// One doubling: off-diagonal squares of H x H blocks.
+template <int H>
+__device__ __forceinline__ void inverse_double(const double* C, double* X, double* W) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  constexpr int kBlocks = 4 / H * H * H;                 // 8 x 8 output blocks of a pass: 4, 8, 16
+  constexpr int kPer = (kBlocks + 7) / 8;                // of one warp
+#pragma unroll
+  for (int pass = 0; pass < 2; ++pass) {
+    double c[kPer][2];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      c[u][0] = c[u][1] = 0.0;
+      const int q = warp + 8 * u;
+      if (q < kBlocks) {
+        const int pr = q / (H * H), bi = (q % (H * H)) / H, bj = q % H;
+        const int r0 = 8 * (2 * H * pr + H), c0 = 8 * 2 * H * pr;   // first row of block 2, first column of block 1
+        const double* A = (pass == 0 ? C + (r0 + 8 * bi) * kMmaLd + c0 : X + (r0 + 8 * bi) * kMmaLd + r0) + g * kMmaLd + t;
+        const double* B = (pass == 0 ? X + c0 * kMmaLd + c0 : W + r0 * kMmaLd + c0) + 8 * bj + t * kMmaLd + g;
+        double a[2 * H], b[2 * H];
+#pragma unroll
+        for (int k = 0; k < 2 * H; ++k) {
+          a[k] = A[4 * k];
+          b[k] = B[4 * k * kMmaLd];
+        }
+#pragma unroll
+        for (int k = 0; k < 2 * H; ++k) dmma884(c[u], a[k], b[k]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int q = warp + 8 * u;
+      if (q < kBlocks) {
+        const int pr = q / (H * H), bi = (q % (H * H)) / H, bj = q % H;
+        const int r0 = 8 * (2 * H * pr + H), c0 = 8 * 2 * H * pr;
+        double2* out = reinterpret_cast<double2*>((pass == 0 ? W : X) + (r0 + 8 * bi + g) * kMmaLd + c0 + 8 * bj + 2 * t);
+        *out = pass == 0 ? make_double2(c[u][0], c[u][1]) : make_double2(-c[u][0], -c[u][1]);
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// last_panel() runs in warp 7 beside the last panel.
+template <typename P, typename F>
+__device__ __forceinline__ void tile_cholesky(double* C, double* X, double* W, TileScratch& sc, P last_panel,
+                                              F after_panels) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll 1   // the body is long: eight copies would not stay in the instruction cache
+  for (int p = 0; p < 8; ++p) {
+    const int base = 8 * p;
+    if (p > 0) {
+      // column block p takes panel p - 1 first: warp w the block in block row p + w
+      if (p + warp < 8) {
+        double c[2] = {0.0, 0.0};
+        double2* d = reinterpret_cast<double2*>(C + (8 * (p + warp) + g) * kMmaLd + base + 2 * t);
+        double2 v = *d;
+        mma8(c, C + 8 * (p + warp) * kMmaLd + base - 8, C + base * kMmaLd + base - 8, lane);
+        v.x -= c[0];
+        v.y -= c[1];
+        *d = v;
+      }
+      __syncthreads();
+    }
+    if (warp == 0) {
+      double d[8][8], a1[8], a2[8];
+      const int r1 = base + lane, r2 = base + 32 + lane;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int k = 0; k <= i; k += 2) {
+          const double2 u = *reinterpret_cast<const double2*>(C + (base + i) * kMmaLd + base + k);
+          d[i][k] = u.x;
+          d[i][k + 1] = u.y;
+        }
+#pragma unroll
+      for (int k = 0; k < 8; k += 2) {
+        const double2 u = r1 < kT ? *reinterpret_cast<const double2*>(C + r1 * kMmaLd + base + k) : make_double2(0.0, 0.0);
+        const double2 w = r2 < kT ? *reinterpret_cast<const double2*>(C + r2 * kMmaLd + base + k) : make_double2(0.0, 0.0);
+        a1[k] = u.x;
+        a1[k + 1] = u.y;
+        a2[k] = w.x;
+        a2[k + 1] = w.y;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const double pj = d[j][j];
+        const double pv = pj > 0.0 ? pj : 1.0;
+        const double rs = rsqrt(pv);
+        if (lane == 0) {
+          sc.pivot[base + j] = pj;
+          sc.rsq[base + j] = rs;
+        }
+#pragma unroll
+        for (int i = j + 1; i < 8; ++i) d[i][j] *= rs;
+        a1[j] = lane > j ? a1[j] * rs : (lane == j ? pv * rs : 0.0);
+        a2[j] *= rs;
+#pragma unroll
+        for (int k = j + 1; k < 8; ++k) {
+#pragma unroll
+          for (int i = k; i < 8; ++i) d[i][k] -= d[i][j] * d[k][j];
+          a1[k] -= a1[j] * d[k][j];
+          a2[k] -= a2[j] * d[k][j];
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 8; k += 2) {
+        if (r1 < kT) *reinterpret_cast<double2*>(C + r1 * kMmaLd + base + k) = make_double2(a1[k], a1[k + 1]);
+        if (r2 < kT) *reinterpret_cast<double2*>(C + r2 * kMmaLd + base + k) = make_double2(a2[k], a2[k + 1]);
+      }
+    } else {
+      if (p > 0) {
+        // panel p - 1 on the columns behind block p: the blocks (i, k), p < k <= i < 8
+        const int m = 7 - p;
+        for (int q = warp - 1; q < m * (m + 1) / 2; q += 7) {
+          int i = 0;
+          while ((i + 1) * (i + 2) / 2 <= q) ++i;
+          const int k = q - i * (i + 1) / 2, bi = 8 * (p + 1 + i), bk = 8 * (p + 1 + k);
+          double c[2] = {0.0, 0.0};
+          mma8(c, C + bi * kMmaLd + base - 8, C + bk * kMmaLd + base - 8, lane);
+          double2* d = reinterpret_cast<double2*>(C + (bi + g) * kMmaLd + bk + 2 * t);
+          double2 v = *d;
+          v.x -= c[0];
+          v.y -= c[1];
+          *d = v;
+        }
+      }
+      if (p == 7 && warp == 7) last_panel();
+      // zeros above the diagonal of the inverse: block row p's columns right of the diagonal block
+      const int w = kT - base - 8;
+      for (int q = tid - 32; q < 8 * w; q += kBandThreads - 32) X[(base + q / w) * kMmaLd + base + 8 + q % w] = 0.0;
+    }
+    __syncthreads();
+  }
+  after_panels();
+  // zeros above the diagonal blocks of L
+  for (int q = tid; q < kTile; q += kBandThreads) {
+    const int r = q / kT, c = q % kT;
+    if ((c >> 3) > (r >> 3)) C[r * kMmaLd + c] = 0.0;
+  }
+  // 8 x 8 diagonal inverses: warp w block w, lane c < 8 its column c, by forward substitution
+  if (lane < 8) {
+    const double* Lb = C + 8 * warp * kMmaLd + 8 * warp;
+    double x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      double s = i == lane ? 1.0 : 0.0;
+#pragma unroll
+      for (int k = 0; k < i; ++k) s -= Lb[i * kMmaLd + k] * x[k];
+      x[i] = i < lane ? 0.0 : s * sc.rsq[8 * warp + i];
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) X[(8 * warp + i) * kMmaLd + 8 * warp + lane] = x[i];
+  }
+  __syncthreads();
+  inverse_double<1>(C, X, W);
+  inverse_double<2>(C, X, W);
+  inverse_double<4>(C, X, W);
+}
+
+__device__ __forceinline__ void store_tile(double* dst, const double* src) {
+  for (int q = threadIdx.x; q < kTile / 2; q += kBandThreads)
+    reinterpret_cast<double2*>(dst)[q] =
+        *reinterpret_cast<const double2*>(src + (q / (kT / 2)) * kMmaLd + 2 * (q % (kT / 2)));
+}
+
+// The diagonal, from the first block row to the last.  The next row's two tiles are fetched while
+// this row's factor is inverted, if the workers have them by then.
+__device__ void band_chain(const BandWork& B, double* sm) {
+  double* As = sm;                  // C_{J,J-1}; the next row's at An
+  double* An = sm + kStage;
+  double* Cs = sm + 2 * kStage;     // the diagonal tile, then L_JJ; the next row's at Cn
+  double* Cn = sm + 3 * kStage;
+  double* Ls = sm + 4 * kStage;     // L_{J,J-1}; scratch of the inverse
+  double* Xs = sm + 5 * kStage;     // Linv of the block row before, then this one's
+  __shared__ TileScratch sc;
+  __shared__ int go, early;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const bool sub = B.bands > 0, need = B.bands >= 2;
+  double pmin = INFINITY, pmax = 0.0;
+  bool bad = false;
+  bool fetched = false;
+  if (tid == 0) early = 0;
+  auto fetch = [&](int J, double* A, double* C) {
+    if (sub && J > 0) stage_tile(A, B.tiles + tile_index(J, 1, B.bands));
+    stage_commit();
+    stage_tile(C, B.tiles + tile_index(J, 0, B.bands));
+    stage_commit();
+  };
+  for (int J = 0; J < B.n_tiles; ++J) {
+    if (!fetched) {
+      if (tid == 0) go = J < 2 || !need || wait_for(B.prepared + J, 2, B.abort_flag);
+      __syncthreads();
+      if (!go) break;
+      fetch(J, As, Cs);
+    }
+    stage_wait<1>();
+    __syncthreads();
+    TileAcc acc;
+    if (sub && J > 0) {
+      tile_zero(acc);
+      tile_mma<true, false>(As, Xs, acc);   // Linv is lower triangular
+      double* G = B.tiles + tile_index(J, 1, B.bands);
+      tile_each(kMmaLd, [&](int o, int i, int j) { *reinterpret_cast<double2*>(Ls + o) = make_double2(acc[i][j][0], acc[i][j][1]); });
+      tile_each(kT, [&](int o, int i, int j) { *reinterpret_cast<double2*>(G + o) = make_double2(acc[i][j][0], acc[i][j][1]); });
+    }
+    stage_wait<0>();
+    __syncthreads();
+    if (sub && J > 0) {
+      publish(B.progress + J, J);
+      tile_syrk(Ls, Cs);
+      __syncthreads();
+    }
+    auto look = [&] {   // is the next row prepared?
+      if (lane == 0 && J + 1 < B.n_tiles && (J < 1 || !need || ld_relaxed(B.prepared + J + 1) >= 2)) {
+        fence_gpu();
+        early = J + 1;
+      }
+    };
+    tile_cholesky(Cs, Xs, Ls, sc, look, [&] {
+      fetched = J + 1 < B.n_tiles && early > J;
+      if (fetched) fetch(J + 1, An, Cn);
+    });
+    store_tile(B.inv + (size_t)J * kTile, Xs);
+    publish(B.progress + J, J + 1);
+    store_tile(B.tiles + tile_index(J, 0, B.bands), Cs);
+    if (tid >= kBandThreads - 32) {   // the last warp: the row's pivots
+      for (int i = lane; i < kT; i += 32) {
+        if (J * kT + i < B.n) {
+          const double p = sc.pivot[i];
+          if (p > 0.0) {
+            pmin = fmin(pmin, p);
+            pmax = fmax(pmax, p);
+          } else {
+            bad = true;
+          }
+        }
+      }
+    }
+    if (fetched) {
+      double* a = As;
+      As = An;
+      An = a;
+      double* c = Cs;
+      Cs = Cn;
+      Cn = c;
+    }
+    __syncthreads();
+  }
+  if (tid >= kBandThreads - 32) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      pmin = fmin(pmin, __shfl_xor_sync(FEAB_FULL_MASK, pmin, o));
+      pmax = fmax(pmax, __shfl_xor_sync(FEAB_FULL_MASK, pmax, o));
+    }
+    bad = __any_sync(FEAB_FULL_MASK, bad);
+    if (lane == 0) {
+      B.st->piv_min = (unsigned long long)__double_as_longlong(pmin);
+      B.st->piv_max = (unsigned long long)__double_as_longlong(pmax);
+      if (bad) B.st->status = FEAB_NOT_SPD;
+    }
+  }
+}
+
+// Tasks of slot J (block column J), bands + 1 of them: 0 the tile (J + 2, J); 1 and 2 the tiles (J + 2,
+// J + 1) and (J + 2, J + 2) for the chain; then the tiles (I, J), I = J + 3 .. J + bands.
+__device__ void band_worker(const BandWork& B, double* sm) {
+  __shared__ int task, ready, go;
+  const int tid = threadIdx.x, b = B.bands;
+  const long long tasks = b >= 2 ? (long long)B.n_tiles * (b + 1) : 0;
+  while (true) {
+    if (tid == 0) task = atomicAdd(B.next_task, 1);
+    __syncthreads();
+    const int tk = task;
+    if (tk >= tasks) return;
+    const int J = tk / (b + 1), q = tk - J * (b + 1);
+    const bool chain_tile = q == 1 || q == 2;
+    const int I = J + (q < 3 ? 2 : q);
+    const int col = q == 1 ? J + 1 : (q == 2 ? J + 2 : J);
+    if (I >= B.n_tiles || (!chain_tile && I - J > b)) {
+      __syncthreads();
+      continue;
+    }
+    const int K0 = max(0, I - b), K1 = chain_tile ? J + 1 : J;   // terms K0 .. K1 - 1
+    const bool diag = col == I;
+    double* G = B.tiles + tile_index(I, I - col, b);
+    TileAcc acc;
+    double2 c0[2][4];
+    tile_each(kT, [&](int o, int i, int j) { c0[i][j] = __ldcg(reinterpret_cast<const double2*>(G + o)); });
+    tile_zero(acc);
+    int known = 0;   // thread 0: both rows' tiles of columns < known are stored
+    auto poll = [&](int want) {
+      known = min(ld_relaxed(B.progress + I), ld_relaxed(B.progress + col));
+      return known >= want;
+    };
+    auto block_until = [&](int want) {   // thread 0
+      if (known >= want) return true;
+      const bool ok = wait_for(B.progress + I, want, B.abort_flag) && wait_for(B.progress + col, want, B.abort_flag);
+      known = want;
+      return ok;
+    };
+    auto issue = [&](int K) {
+      double* buf = sm + (K & 1) * 2 * kStage;
+      stage_tile(buf, B.tiles + tile_index(I, I - K, b));
+      if (!diag) stage_tile(buf + kStage, B.tiles + tile_index(col, col - K, b));
+      stage_commit();
+    };
+    bool issued = false;   // the next term's copies are on their way
+    for (int K = K0; K < K1; ++K) {
+      if (!issued) {
+        if (tid == 0) go = block_until(K + 1);
+        __syncthreads();
+        if (!go) return;
+        issue(K);
+      }
+      if (tid == 0) {
+        ready = K + 1 < K1 && known >= K + 2;
+        if (!ready && K + 1 < K1 && poll(K + 2)) {
+          fence_gpu();
+          ready = 1;
+        }
+      }
+      __syncthreads();
+      issued = ready;
+      if (issued) {
+        issue(K + 1);
+        stage_wait<1>();
+      } else {
+        stage_wait<0>();
+      }
+      __syncthreads();
+      const double* buf = sm + (K & 1) * 2 * kStage;
+      if (!diag) tile_mma<false, false>(buf, buf + kStage, acc);
+      else tile_mma<false, true>(buf, buf, acc);
+      __syncthreads();
+    }
+    if (chain_tile) {
+      tile_each(kT, [&](int o, int i, int j) {
+        *reinterpret_cast<double2*>(G + o) = make_double2(c0[i][j].x - acc[i][j][0], c0[i][j].y - acc[i][j][1]);
+      });
+      publish(B.prepared + I, 0);
+    } else {
+      tile_each(kMmaLd, [&](int o, int i, int j) {
+        *reinterpret_cast<double2*>(sm + o) = make_double2(c0[i][j].x - acc[i][j][0], c0[i][j].y - acc[i][j][1]);
+      });
+      if (tid == 0) go = wait_for(B.progress + J, J + 1, B.abort_flag);
+      __syncthreads();
+      if (!go) return;
+      stage_tile(sm + kStage, B.inv + (size_t)J * kTile);
+      stage_commit();
+      stage_wait<0>();
+      __syncthreads();
+      tile_zero(acc);
+      tile_mma<true, false>(sm, sm + kStage, acc);   // Linv is lower triangular
+      tile_each(kT, [&](int o, int i, int j) {
+        *reinterpret_cast<double2*>(G + o) = make_double2(acc[i][j][0], acc[i][j][1]);
+      });
+      publish(B.progress + I, J + 1);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kBandThreads, 1) k_band_factor(BandWork B) {
+  extern __shared__ __align__(16) double fsm[];
+  if (blockIdx.x == 0) band_chain(B, fsm);
+  else band_worker(B, fsm);
+}
 
 // ---------------------------------------------------------------- solves
 // Forward step K of L y = b: every CTA forms y_K = Linv_KK w_K (two threads per row), CTA 0 writes
@@ -405,6 +739,9 @@ double* band_tiles(const feab_band* B) {
 double* band_inv(const feab_band* B) {
   return band_tiles(B) + (size_t)B->n_tiles * (size_t)(B->bands + 1) * kTile;
 }
+// After the inverses: progress and prepared per block row, the next task and the abort flag.
+size_t band_flag_bytes(int32_t n_tiles) { return (2 * (size_t)n_tiles + 2) * sizeof(int32_t); }
+int32_t* band_flags(const feab_band* B) { return reinterpret_cast<int32_t*>(band_inv(B) + (size_t)B->n_tiles * kTile); }
 bool band_ok(const feab_band* B) {
   return B && B->storage && B->n > 0 && B->bands >= 0 && B->n_tiles == (B->n + kT - 1) / kT &&
          (reinterpret_cast<uintptr_t>(B->storage) & 255) == 0;
@@ -414,7 +751,7 @@ bool band_ok(const feab_band* B) {
 extern "C" size_t feab_band_bytes(int32_t n, int32_t bandwidth) {
   if (n <= 0 || bandwidth < 0) return 0;
   const size_t nt = (size_t)(n + kT - 1) / kT, bands = (size_t)(bandwidth + kT - 1) / kT;
-  return FEAB_BAND_HEADER_BYTES + nt * (bands + 2) * (size_t)kTile * sizeof(double);
+  return FEAB_BAND_HEADER_BYTES + nt * (bands + 2) * (size_t)kTile * sizeof(double) + band_flag_bytes((int32_t)nt);
 }
 
 extern "C" int32_t feab_band_width(const feab_csr* A, const int32_t* iperm, int32_t* scratch, int32_t* bandwidth_out,
@@ -462,27 +799,31 @@ extern "C" int32_t feab_band_cholesky(feab_band* B, double* pivots_out, cudaStre
   init.piv_max = 0ull;
   BandState* st = band_state(B);
   FEAB_CUDA(cudaMemcpyAsync(st, &init, sizeof(BandState), cudaMemcpyHostToDevice, s));
-  FEAB_CUDA(cudaFuncSetAttribute(k_band_potrf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPotrfSmem));
-  FEAB_CUDA(cudaFuncSetAttribute(k_band_tile_gemm<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kGemmSmem));
-  FEAB_CUDA(cudaFuncSetAttribute(k_band_tile_gemm<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kGemmSmem));
-  double* tiles = band_tiles(B);
-  double* inv = band_inv(B);
-  const int NT = B->n_tiles, bands = B->bands;
-  uint64_t launches = 0;
-  for (int K = 0; K < NT; ++K) {
-    k_band_potrf<<<1, 256, kPotrfSmem, s>>>(tiles, inv, bands, K, B->n, st);
-    const int below = std::min(bands, NT - 1 - K);
-    if (below > 0) {
-      k_band_tile_gemm<true><<<below, 256, kGemmSmem, s>>>(tiles, inv, bands, K);
-      k_band_tile_gemm<false><<<below * (below + 1) / 2, 256, kGemmSmem, s>>>(tiles, inv, bands, K);
-      launches += 2;
-    }
-    launches += 1;
-  }
-  count_launches(launches);
+  FEAB_CUDA(cudaMemsetAsync(band_flags(B), 0, band_flag_bytes(B->n_tiles), s));
+  BandWork W{};
+  W.tiles = band_tiles(B);
+  W.inv = band_inv(B);
+  W.st = st;
+  W.progress = band_flags(B);
+  W.prepared = W.progress + B->n_tiles;
+  W.next_task = W.prepared + B->n_tiles;
+  W.abort_flag = W.next_task + 1;
+  W.n = B->n;
+  W.n_tiles = B->n_tiles;
+  W.bands = B->bands;
+  FEAB_CUDA(cudaFuncSetAttribute(k_band_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFactorSmem));
+  // one CTA per SM: the chain and, with two bands or more, at least one worker
+  int resident = 0;
+  FEAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_band_factor, kBandThreads, kFactorSmem));
+  const int64_t tasks = B->bands >= 2 ? (int64_t)B->n_tiles * (B->bands + 1) : 0;
+  const int grid = (int)std::min<int64_t>((int64_t)sm_count() * std::min(resident, 1), 1 + tasks);
+  if (grid < (tasks > 0 ? 2 : 1)) return FEAB_CUDA_ERROR;
+  void* args[1] = {&W};
+  FEAB_CUDA(cudaLaunchCooperativeKernel((const void*)k_band_factor, dim3(grid), dim3(kBandThreads), args, kFactorSmem, s));
+  count_launches(1);
   FEAB_CHECK_LAUNCH();
+  int32_t aborted = 0;
+  FEAB_CUDA(cudaMemcpyAsync(&aborted, W.abort_flag, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
   BandState h{};
   FEAB_CUDA(cudaMemcpyAsync(&h, st, sizeof(BandState), cudaMemcpyDeviceToHost, s));
   FEAB_CUDA(cudaStreamSynchronize(s));
@@ -493,6 +834,7 @@ extern "C" int32_t feab_band_cholesky(feab_band* B, double* pivots_out, cudaStre
     pivots_out[0] = lo;
     pivots_out[1] = hi;
   }
+  if (aborted) return FEAB_CUDA_ERROR;
   return h.status == FEAB_OK ? FEAB_OK : h.status;
 }
 
