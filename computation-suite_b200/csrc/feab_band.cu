@@ -12,9 +12,8 @@
 // J = 0 .. n_tiles - 1: the diagonal tile is factored and its factor inverted (Linv_JJ, kept beside
 // the band), and the tiles below it are L_IJ = (A_IJ - sum_K L_IK L_JK^T) Linv_JJ^T, products of 64 x
 // 64 tiles on the FP64 tensor path (mma.sync).  It runs as one kernel (k_band_factor).
-// The solves walk the block rows forward (L y = b) and backward (L^T x = y), one kernel per block
-// row: each CTA forms the block's y_K = Linv_KK w_K (or x_K = Linv_KK^T w_K) and then applies one
-// off-diagonal tile to a later (earlier) block of the right-hand side.
+// The solves walk the block rows forward (L y = b) and backward (L^T x = y) with the inverted diagonal
+// factors, in one kernel of one cluster (k_band_solve).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -665,6 +664,371 @@ __global__ void __launch_bounds__(kBandThreads, 1) k_band_factor(BandWork B) {
 }
 
 // ---------------------------------------------------------------- solves
+// Both triangular solves in one kernel of one cluster.  CTA c of C owns the block rows J = c (mod C).
+// Forward, w_J = b_J - sum_K L_JK y_K grows in registers as the y_K come in (each thread keeps its
+// share of the sums of its CTA's next P rows, unreduced), and when y_{J-1} is in, the owner of J
+// reduces w_J, forms y_J = Linv_JJ w_J and writes it into every CTA's shared memory (st.async, which
+// counts the bytes on the receiver's barrier).  Backward the same with L_IJ^T and Linv_JJ^T.  A tile
+// is used once, so one more warp streams the tiles in the order of their use through a ring in shared
+// memory (bulk copies).
+// Vector q + 32 goes where vector q was: every CTA sends a vector between the two (it has a row among
+// any 16, and at most 31 vectors lie between its last row forward and its first backward), and it
+// has taken in all vectors before the one that it sends.  Every wait is bounded: a warp whose wait
+// runs out goes on without waiting, so that barriers stay matched, and sends NaN.
+//
+// What bounds it: latency, 1.1 us per block row (two 64 x 64 products by 512 threads, each with its
+// reduction, and one hop to another SM), while a CTA's tiles per block row (bands / C) come in
+// faster than that; wide bands are bound by what 16 SMs read (about 1.4 TB/s).  Measured, two
+// launches per block row -> one kernel, both directions: 64x16x16 elements (867 block rows, 28
+// bands) 19.0 -> 2.1 ms, 96x24x24 (2,813, 59 bands) 63.3 -> 8.3 ms, 33x9x8 (140, 9) 2.07 -> 0.36 ms.
+constexpr int kSolveWarps = 16;
+constexpr int kSolveThreads = 32 * kSolveWarps;       // that compute; one more warp fetches the tiles
+constexpr int kSolveCta = kSolveThreads + 32;
+constexpr int kSolveRing = 6;                          // tiles
+constexpr int kSolveSlots = 32;                        // vectors on their way
+constexpr int kSolveMaxCluster = 16;
+constexpr int kSolveMaxRows = 8;                       // P: pending rows of a CTA
+constexpr int kPartLd = kT + 2;
+
+struct SolveShared {
+  double ring[kSolveRing][kTile];
+  double vec[kSolveSlots][kT];
+  double part[kSolveWarps][kPartLd];
+  double w[kT];
+  unsigned long long full[kSolveRing], empty[kSolveRing], arrived[kSolveSlots];
+  int abort_flag;
+};
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(unsigned long long* m, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(m)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(unsigned long long* m, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(m)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned long long* m) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(m)) : "memory");
+}
+__device__ __forceinline__ unsigned long long now_ns() {
+  unsigned long long v;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(v));
+  return v;
+}
+constexpr unsigned long long kSolveLimitNs = 4000000000ull;
+
+// False when the phase does not end within kSolveLimitNs, or another wait of the CTA has given up.
+__device__ __forceinline__ bool mbar_wait(unsigned long long* m, uint32_t parity, volatile int* abort_flag) {
+  const uint32_t a = smem_u32(m);
+  unsigned long long began = 0;
+  while (true) {
+    uint32_t done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(done)
+        : "r"(a), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if (*abort_flag) return false;
+    if (began == 0) began = now_ns();
+    else if (now_ns() - began > kSolveLimitNs) break;
+  }
+  *abort_flag = 1;
+  return false;
+}
+__device__ __forceinline__ void solve_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+struct SolveArgs {
+  const double* tiles;
+  const double* inv;
+  const double* b;
+  double* x;      // y after the forward pass, then the solution
+  int32_t bands, n_tiles;
+};
+
+// The tiles that CTA c uses, in order, passed to fn(address): forward, for each K, the tiles (J, K) of
+// its rows J > K, nearest first, Linv_JJ behind the tile (K + 1, K); backward the mirror image.
+template <typename F>
+__device__ __forceinline__ void solve_tiles(const SolveArgs& A, int c, int C, F fn) {
+  const int b = A.bands, NT = A.n_tiles;
+  if (c == 0) fn(A.inv);
+  for (int K = 0; K < NT - 1; ++K) {
+    int J = K + 1 + (c - (K + 1) % C + C) % C;
+    if (J == K + 1) {
+      if (b > 0) fn(A.tiles + tile_index(J, 1, b));
+      fn(A.inv + (size_t)J * kTile);
+      J += C;
+    }
+    for (; J <= min(K + b, NT - 1); J += C) fn(A.tiles + tile_index(J, J - K, b));
+  }
+  if (c == (NT - 1) % C) fn(A.inv + (size_t)(NT - 1) * kTile);
+  for (int K = NT - 1; K > 0; --K) {
+    int J = K - 1 - ((K - 1) % C - c + C) % C;
+    if (J == K - 1) {
+      if (b > 0) fn(A.tiles + tile_index(K, 1, b));
+      fn(A.inv + (size_t)J * kTile);
+      J -= C;
+    }
+    for (; J >= max(K - b, 0); J -= C) fn(A.tiles + tile_index(K, K - J, b));
+  }
+}
+
+// A thread's eight values of a tile.
+struct TilePart {
+  double2 t[4];
+};
+// Forward: thread (rp = tid / 16, h = tid % 16) holds rows 2 rp and 2 rp + 1, columns 2 h + {0, 1, 32, 33}.
+__device__ __forceinline__ TilePart fwd_part(const double* T) {
+  const int rp = threadIdx.x >> 4, h = threadIdx.x & 15;
+  TilePart p;
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+    p.t[u] = *reinterpret_cast<const double2*>(T + (2 * rp + (u >> 1)) * kT + 32 * (u & 1) + 2 * h);
+  return p;
+}
+__device__ __forceinline__ void fwd_product(const TilePart& p, const double2 (&y)[2], double (&a)[2]) {
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const double s = fma(p.t[2 * u].x, y[0].x, p.t[2 * u].y * y[0].y);
+    a[u] = fma(p.t[2 * u + 1].x, y[1].x, fma(p.t[2 * u + 1].y, y[1].y, a[u])) + s;
+  }
+}
+// Sums over the 16 lanes of a row pair: row 2 rp in lanes h < 8, row 2 rp + 1 in the others.
+__device__ __forceinline__ double fwd_reduce(const double (&a)[2]) {
+  const bool up = (threadIdx.x & 8) != 0;
+  double s = (up ? a[1] : a[0]) + __shfl_xor_sync(FEAB_FULL_MASK, up ? a[0] : a[1], 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(FEAB_FULL_MASK, s, o);
+  return s;
+}
+// Backward: lane l holds columns 2 l, 2 l + 1 of rows 4 w .. 4 w + 3 (warp w).
+__device__ __forceinline__ TilePart bwd_part(const double* T) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  TilePart p;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) p.t[u] = *reinterpret_cast<const double2*>(T + (4 * warp + u) * kT + 2 * lane);
+  return p;
+}
+__device__ __forceinline__ void bwd_product(const TilePart& p, const double (&x)[4], double (&a)[2]) {
+  const double s0 = fma(p.t[0].x, x[0], p.t[1].x * x[1]), s1 = fma(p.t[0].y, x[0], p.t[1].y * x[1]);
+  a[0] = fma(p.t[2].x, x[2], fma(p.t[3].x, x[3], a[0])) + s0;
+  a[1] = fma(p.t[2].y, x[2], fma(p.t[3].y, x[3], a[1])) + s1;
+}
+// Sums over the warps: column tid / 8, in its eight lanes.
+__device__ __forceinline__ double bwd_reduce(SolveShared& S, const double (&a)[2]) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = threadIdx.x >> 3, h = threadIdx.x & 7;
+  *reinterpret_cast<double2*>(&S.part[warp][2 * lane]) = make_double2(a[0], a[1]);
+  solve_sync();
+  double s = S.part[h][col] + S.part[h + 8][col];
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(FEAB_FULL_MASK, s, o);
+  return s;
+}
+
+template <int P>
+__global__ void __launch_bounds__(kSolveCta, 1) k_band_solve(SolveArgs A) {
+  extern __shared__ __align__(128) unsigned char solve_dyn[];
+  SolveShared& S = *reinterpret_cast<SolveShared*>(solve_dyn);
+  const int tid = threadIdx.x, C = gridDim.x, c = blockIdx.x, b = A.bands, NT = A.n_tiles;
+  volatile int* abort_flag = &S.abort_flag;
+  if (tid == 0) {
+    S.abort_flag = 0;
+    for (int i = 0; i < kSolveRing; ++i) {
+      mbar_init(&S.full[i], 1);
+      mbar_init(&S.empty[i], kSolveWarps);
+    }
+    for (int i = 0; i < kSolveSlots; ++i) {
+      mbar_init(&S.arrived[i], 1);
+      mbar_expect(&S.arrived[i], kT * 8);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  cluster_sync_all();
+  if (tid >= kSolveThreads) {
+    // the tiles, each into the next free place of the ring
+    if ((tid & 31) == 0) {
+      int slot = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      solve_tiles(A, c, C, [&](const double* src) {
+        if (!ok) return;
+        ok = mbar_wait(&S.empty[slot], phase ^ 1, abort_flag);
+        if (!ok) return;
+        mbar_expect(&S.full[slot], kTile * 8);
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         smem_u32(S.ring[slot])),
+                     "l"(src), "r"((uint32_t)(kTile * 8)), "r"(smem_u32(&S.full[slot]))
+                     : "memory");
+        if (++slot == kSolveRing) {
+          slot = 0;
+          phase ^= 1;
+        }
+      });
+    }
+  } else {
+    const int warp = tid >> 5, lane = tid & 31, rp = tid >> 4, h = tid & 15;
+    int slot = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    auto tile = [&] {
+      ok = ok && mbar_wait(&S.full[slot], phase, abort_flag);
+      return (const double*)S.ring[slot];
+    };
+    auto release = [&] {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&S.empty[slot]);
+      if (++slot == kSolveRing) {
+        slot = 0;
+        phase ^= 1;
+      }
+    };
+    // vector number q of the solve (y_0 .. y_{NT-1}, then x_{NT-1} .. x_0), entry i = v of this thread's
+    // eight lanes, to every CTA: with the neighbours' entry, each of the 16 lanes of two entries sends
+    // both to one CTA
+    auto send = [&](int q, int i, double v) {
+      const double other = __shfl_xor_sync(FEAB_FULL_MASK, v, 8);
+      const int r = lane & 15;
+      const bool up = (lane & 8) != 0;
+      if (r < C) {
+        const uint32_t dst = smem_u32(&S.vec[q % kSolveSlots][i & ~1]), bar = smem_u32(&S.arrived[q % kSolveSlots]);
+        uint32_t rd, rb;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rd) : "r"(dst), "r"(r));
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rb) : "r"(bar), "r"(r));
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(rd),
+                     "l"(__double_as_longlong(up ? other : v)), "l"(__double_as_longlong(up ? v : other)), "r"(rb)
+                     : "memory");
+      }
+    };
+    auto receive = [&](int q) {
+      ok = ok && mbar_wait(&S.arrived[q % kSolveSlots], (q / kSolveSlots) & 1, abort_flag);
+      if (tid == 0 && ok) mbar_expect(&S.arrived[q % kSolveSlots], kT * 8);
+      return (const double*)S.vec[q % kSolveSlots];
+    };
+    double acc[P][2];
+    auto shift = [&] {
+#pragma unroll
+      for (int p = 0; p + 1 < P; ++p) {
+        acc[p][0] = acc[p + 1][0];
+        acc[p][1] = acc[p + 1][1];
+      }
+      acc[P - 1][0] = acc[P - 1][1] = 0.0;
+    };
+#pragma unroll
+    for (int p = 0; p < P; ++p) acc[p][0] = acc[p][1] = 0.0;
+    // ---- forward
+    // The tile (J, J - 1) and Linv_JJ are in registers before y_{J-1} arrives.
+    const int frow = 2 * rp + (h >> 3);
+    double rhs = c < NT ? A.b[(size_t)c * kT + frow] : 0.0;   // of the CTA's next row
+    TilePart sub{}, diag{};
+    auto load_fwd = [&](bool with_sub) {
+      if (with_sub) {
+        sub = fwd_part(tile());
+        release();
+      }
+      diag = fwd_part(tile());
+      release();
+    };
+    auto finish_fwd = [&](int J) {
+      const double wv = rhs - fwd_reduce(acc[0]);
+      if ((h & 7) == 0) S.w[frow] = wv;
+      solve_sync();
+      const double2 w2[2] = {*reinterpret_cast<const double2*>(&S.w[2 * h]),
+                             *reinterpret_cast<const double2*>(&S.w[32 + 2 * h])};
+      double a[2] = {0.0, 0.0};
+      fwd_product(diag, w2, a);
+      const double sum = fwd_reduce(a), y = ok ? sum : __longlong_as_double(0x7ff8000000000000ll);
+      send(J, frow, y);
+      if ((h & 7) == 0) A.x[(size_t)J * kT + frow] = y;
+      shift();
+      if (J + C < NT) rhs = A.b[(size_t)(J + C) * kT + frow];
+    };
+    if (c == 0) {
+      load_fwd(false);
+      finish_fwd(0);
+    }
+    for (int K = 0; K < NT; ++K) {
+      int J = K + 1 + (c - (K + 1) % C + C) % C;
+      const bool mine = J == K + 1 && J < NT;
+      if (mine) load_fwd(b > 0);
+      const double* v = receive(K);
+      if (K == NT - 1) break;
+      const double2 y[2] = {*reinterpret_cast<const double2*>(v + 2 * h),
+                            *reinterpret_cast<const double2*>(v + 32 + 2 * h)};
+      if (mine) {
+        if (b > 0) fwd_product(sub, y, acc[0]);
+        finish_fwd(J);
+        J += C;
+      }
+      const int last = min(K + b, NT - 1);
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        if (J + p * C <= last) {
+          fwd_product(fwd_part(tile()), y, acc[p]);
+          release();
+        }
+      }
+    }
+    // ---- backward
+    asm volatile("bar.sync 1, 512;" ::: "memory");
+#pragma unroll
+    for (int p = 0; p < P; ++p) acc[p][0] = acc[p][1] = 0.0;
+    const int col = tid >> 3;
+    const int top = NT - 1 - ((NT - 1) % C - c + C) % C;   // the CTA's last row (negative: none)
+    if (top >= 0) rhs = __ldcg(A.x + (size_t)top * kT + col);
+    auto load_bwd = [&](bool with_sub) {
+      if (with_sub) {
+        sub = bwd_part(tile());
+        release();
+      }
+      diag = bwd_part(tile());
+      release();
+    };
+    auto finish_bwd = [&](int J) {
+      const double wv = rhs - bwd_reduce(S, acc[0]);
+      if ((tid & 7) == 0) S.w[col] = wv;
+      solve_sync();
+      const double wr[4] = {S.w[4 * warp], S.w[4 * warp + 1], S.w[4 * warp + 2], S.w[4 * warp + 3]};
+      double a[2] = {0.0, 0.0};
+      bwd_product(diag, wr, a);
+      const double sum = bwd_reduce(S, a), xv = ok ? sum : __longlong_as_double(0x7ff8000000000000ll);
+      send(2 * NT - 1 - J, col, xv);
+      if ((tid & 7) == 0) A.x[(size_t)J * kT + col] = xv;
+      shift();
+      if (J - C >= 0) rhs = __ldcg(A.x + (size_t)(J - C) * kT + col);
+    };
+    if (top == NT - 1) {
+      load_bwd(false);
+      finish_bwd(NT - 1);
+    }
+    for (int K = NT - 1; K > 0; --K) {
+      int J = K - 1 - ((K - 1) % C - c + C) % C;
+      const bool mine = J == K - 1;
+      if (mine) load_bwd(b > 0);
+      const double* v = receive(2 * NT - 1 - K);
+      const double xr[4] = {v[4 * warp], v[4 * warp + 1], v[4 * warp + 2], v[4 * warp + 3]};
+      if (mine) {
+        if (b > 0) bwd_product(sub, xr, acc[0]);
+        finish_bwd(J);
+        J -= C;
+      }
+      const int last = max(K - b, 0);
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        if (J - p * C >= last) {
+          bwd_product(bwd_part(tile()), xr, acc[p]);
+          release();
+        }
+      }
+    }
+    receive(2 * NT - 1);   // x_0: nothing is on its way to this CTA when it leaves
+  }
+  __syncwarp();
+  cluster_sync_all();
+}
+
+// Wider bands than the cluster kernel's pending rows: one launch per block row.
 // Forward step K of L y = b: every CTA forms y_K = Linv_KK w_K (two threads per row), CTA 0 writes
 // it, and CTA i < n_below applies tile (K + 1 + i, i + 1): w_{K+1+i} -= L_{K+1+i,K} y_K.
 __global__ void __launch_bounds__(128) k_band_fwd(const double* __restrict__ tiles, const double* __restrict__ inv,
@@ -843,6 +1207,31 @@ extern "C" int32_t feab_band_solve(const feab_band* B, const double* b, double* 
   const double* tiles = band_tiles(B);
   const double* inv = band_inv(B);
   const int NT = B->n_tiles, bands = B->bands;
+  // A CTA's pending rows, bands / C, are registers; up to 8 bands one portable cluster has a tile per
+  // CTA and block row.
+  const int C = bands > 8 ? kSolveMaxCluster : 8, rows = (bands + C - 1) / C;
+  if (rows <= kSolveMaxRows) {
+    SolveArgs A{tiles, inv, b, x, bands, NT};
+    const void* fn = rows <= 1 ? (const void*)k_band_solve<1> : rows <= 2 ? (const void*)k_band_solve<2>
+                   : rows <= 4 ? (const void*)k_band_solve<4> : (const void*)k_band_solve<kSolveMaxRows>;
+    FEAB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SolveShared)));
+    FEAB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(C);
+    cfg.blockDim = dim3(kSolveCta);
+    cfg.dynamicSmemBytes = sizeof(SolveShared);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = C;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    void* args[1] = {&A};
+    FEAB_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
+    count_launches(1);
+    return FEAB_OK;
+  }
   const size_t bytes = (size_t)NT * kT * sizeof(double);
   // forward: work = b, updated in place; y into x
   FEAB_CUDA(cudaMemcpyAsync(work, b, bytes, cudaMemcpyDeviceToDevice, s));

@@ -21,13 +21,12 @@ def _band_matrix(n, bw, seed):
     return sp.csr_matrix(A + sp.diags(1.2 * row.max() + 1.0 + rng.uniform(0.0, 1.0, n)))
 
 
-@pytest.mark.parametrize("n,bw", [(1, 0), (63, 0), (64, 20), (65, 1), (64, 63), (128, 64), (130, 65), (200, 128),
-                                  (500, 129), (449, 192), (700, 699), (1500, 257)])
-def test_band_factor_and_solve(n, bw):
+def _assembled(A, bw):
+    """(feab_band, its storage, stream) of the CSR matrix A with its rows in order."""
     from feab200 import _lib as L
-    A = _band_matrix(n, bw, 100 * n + bw)
     dev = torch.device("cuda")
     t = lambda a, dt: torch.as_tensor(np.ascontiguousarray(a, dtype=dt)).to(dev)  # noqa: E731
+    n = A.shape[0]
     rp, ci, va = t(A.indptr, np.int32), t(A.indices, np.int32), t(A.data, np.float64)
     csr = L.CSR(n, n, int(A.nnz), rp.data_ptr(), ci.data_ptr(), va.data_ptr(), None, None)
     iperm = torch.arange(n, dtype=torch.int32, device=dev)
@@ -35,6 +34,26 @@ def test_band_factor_and_solve(n, bw):
     band = L.Band(0, 0, 0, 0, storage.data_ptr())
     st = L.stream_ptr(dev)
     assert L.lib.feab_band_assemble(C.byref(csr), L.dptr(iperm), bw, C.byref(band), st) == L.FEAB_OK
+    return band, storage, st
+
+
+def _solve(band, b, st):
+    from feab200 import _lib as L
+    bt = torch.zeros(64 * band.n_tiles, dtype=torch.float64, device="cuda")
+    bt[:len(b)] = torch.as_tensor(b).cuda()
+    x, w = torch.empty_like(bt), torch.empty_like(bt)
+    assert L.lib.feab_band_solve(C.byref(band), L.dptr(bt), L.dptr(x), L.dptr(w), st) == L.FEAB_OK
+    x = x.cpu().numpy()
+    assert not x[len(b):].any()
+    return x[:len(b)]
+
+
+@pytest.mark.parametrize("n,bw", [(1, 0), (63, 0), (64, 20), (65, 1), (64, 63), (128, 64), (130, 65), (200, 128),
+                                  (500, 129), (449, 192), (700, 699), (1500, 257)])
+def test_band_factor_and_solve(n, bw):
+    from feab200 import _lib as L
+    A = _band_matrix(n, bw, 100 * n + bw)
+    band, storage, st = _assembled(A, bw)
     piv = (C.c_double * 2)()
     assert L.lib.feab_band_cholesky(C.byref(band), piv, st) == L.FEAB_OK
     full = np.linalg.cholesky(A.toarray())
@@ -50,11 +69,26 @@ def test_band_factor_and_solve(n, bw):
     assert np.abs(got[:n, :n] - full).max() < tol * np.abs(full).max()
     rng = np.random.default_rng(n)
     for _ in range(2):
-        b = np.zeros(64 * nt)
-        b[:n] = rng.standard_normal(n)
-        bt = t(b, np.float64)
-        x, w = torch.empty_like(bt), torch.empty_like(bt)
-        assert L.lib.feab_band_solve(C.byref(band), L.dptr(bt), L.dptr(x), L.dptr(w), st) == L.FEAB_OK
-        want = sl.cho_solve((full, True), b[:n])
-        assert np.linalg.norm(x.cpu().numpy()[:n] - want) < tol * np.linalg.norm(want)
-        assert not x[n:].any()
+        b = rng.standard_normal(n)
+        want = sl.cho_solve((full, True), b)
+        assert np.linalg.norm(_solve(band, b, st) - want) < tol * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("bands", [8, 9, 16, 17, 33, 65, 128, 129])
+def test_wide_band_solve(bands):
+    """Both sides of each form of the solve: a few diagonals, the outermost at the band's edge."""
+    from feab200 import _lib as L
+    bw = 64 * bands
+    n = bw + 200
+    rng = np.random.default_rng(bands)
+    off = sp.diags([rng.uniform(-1.0, 1.0, n - k) for k in (1, 65, bw // 2 + 3, bw)], [1, 65, bw // 2 + 3, bw],
+                   shape=(n, n))
+    A = sp.csr_matrix(off + off.T + sp.diags(10.0 + rng.uniform(0.0, 1.0, n)))
+    band, storage, st = _assembled(A, bw)
+    assert band.bands == bands
+    piv = (C.c_double * 2)()
+    assert L.lib.feab_band_cholesky(C.byref(band), piv, st) == L.FEAB_OK
+    b = rng.standard_normal(n)
+    x = _solve(band, b, st)
+    # condition number below 10, as above
+    assert np.linalg.norm(b - A @ x) < 40.0 * n * 2.0 ** -53 * np.linalg.norm(b)
