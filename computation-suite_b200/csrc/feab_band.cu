@@ -94,6 +94,7 @@ struct BandState {
   unsigned long long piv_min, piv_max;  // bit patterns of positive doubles (order-preserving)
   int32_t status;
   int32_t bad;                          // assembly: an entry outside the band
+  int32_t next_task, abort_flag;        // factorisation
 };
 static_assert(sizeof(BandState) <= FEAB_BAND_HEADER_BYTES, "band header");
 
@@ -504,7 +505,8 @@ __device__ void band_chain(const BandWork& B, double* sm) {
     stage_wait<0>();
     __syncthreads();
     if (sub && J > 0) {
-      publish(B.progress + J, J);
+      if (need) publish(B.progress + J, J);
+      else __syncthreads();
       tile_syrk(Ls, Cs);
       __syncthreads();
     }
@@ -519,7 +521,7 @@ __device__ void band_chain(const BandWork& B, double* sm) {
       if (fetched) fetch(J + 1, An, Cn);
     });
     store_tile(B.inv + (size_t)J * kTile, Xs);
-    publish(B.progress + J, J + 1);
+    if (need) publish(B.progress + J, J + 1);
     store_tile(B.tiles + tile_index(J, 0, B.bands), Cs);
     if (tid >= kBandThreads - 32) {   // the last warp: the row's pivots
       for (int i = lane; i < kT; i += 32) {
@@ -1103,9 +1105,19 @@ double* band_tiles(const feab_band* B) {
 double* band_inv(const feab_band* B) {
   return band_tiles(B) + (size_t)B->n_tiles * (size_t)(B->bands + 1) * kTile;
 }
-// After the inverses: progress and prepared per block row, the next task and the abort flag.
-size_t band_flag_bytes(int32_t n_tiles) { return (2 * (size_t)n_tiles + 2) * sizeof(int32_t); }
-int32_t* band_flags(const feab_band* B) { return reinterpret_cast<int32_t*>(band_inv(B) + (size_t)B->n_tiles * kTile); }
+// progress and prepared, two counters per block row, in use with two bands or more while the factorisation
+// runs: in the tiles of block row 0 that lie left of the matrix (bands tiles, never read), behind the
+// inverses when there are more counters than those hold.
+size_t band_flag_bytes(int32_t n_tiles, int32_t bands) {
+  return bands >= 2 ? 2 * (size_t)n_tiles * sizeof(int32_t) : 0;
+}
+bool band_flags_inside(int32_t n_tiles, int32_t bands) {
+  return band_flag_bytes(n_tiles, bands) <= (size_t)bands * kTile * sizeof(double);
+}
+int32_t* band_flags(const feab_band* B) {
+  return reinterpret_cast<int32_t*>(band_flags_inside(B->n_tiles, B->bands) ? band_tiles(B) + kTile
+                                                                            : band_inv(B) + (size_t)B->n_tiles * kTile);
+}
 bool band_ok(const feab_band* B) {
   return B && B->storage && B->n > 0 && B->bands >= 0 && B->n_tiles == (B->n + kT - 1) / kT &&
          (reinterpret_cast<uintptr_t>(B->storage) & 255) == 0;
@@ -1115,7 +1127,8 @@ bool band_ok(const feab_band* B) {
 extern "C" size_t feab_band_bytes(int32_t n, int32_t bandwidth) {
   if (n <= 0 || bandwidth < 0) return 0;
   const size_t nt = (size_t)(n + kT - 1) / kT, bands = (size_t)(bandwidth + kT - 1) / kT;
-  return FEAB_BAND_HEADER_BYTES + nt * (bands + 2) * (size_t)kTile * sizeof(double) + band_flag_bytes((int32_t)nt);
+  const size_t flags = band_flags_inside((int32_t)nt, (int32_t)bands) ? 0 : band_flag_bytes((int32_t)nt, (int32_t)bands);
+  return FEAB_BAND_HEADER_BYTES + nt * (bands + 2) * (size_t)kTile * sizeof(double) + flags;
 }
 
 extern "C" int32_t feab_band_width(const feab_csr* A, const int32_t* iperm, int32_t* scratch, int32_t* bandwidth_out,
@@ -1163,15 +1176,16 @@ extern "C" int32_t feab_band_cholesky(feab_band* B, double* pivots_out, cudaStre
   init.piv_max = 0ull;
   BandState* st = band_state(B);
   FEAB_CUDA(cudaMemcpyAsync(st, &init, sizeof(BandState), cudaMemcpyHostToDevice, s));
-  FEAB_CUDA(cudaMemsetAsync(band_flags(B), 0, band_flag_bytes(B->n_tiles), s));
+  const size_t flag_bytes = band_flag_bytes(B->n_tiles, B->bands);
+  if (flag_bytes) FEAB_CUDA(cudaMemsetAsync(band_flags(B), 0, flag_bytes, s));
   BandWork W{};
   W.tiles = band_tiles(B);
   W.inv = band_inv(B);
   W.st = st;
   W.progress = band_flags(B);
   W.prepared = W.progress + B->n_tiles;
-  W.next_task = W.prepared + B->n_tiles;
-  W.abort_flag = W.next_task + 1;
+  W.next_task = &st->next_task;
+  W.abort_flag = &st->abort_flag;
   W.n = B->n;
   W.n_tiles = B->n_tiles;
   W.bands = B->bands;
@@ -1186,8 +1200,7 @@ extern "C" int32_t feab_band_cholesky(feab_band* B, double* pivots_out, cudaStre
   FEAB_CUDA(cudaLaunchCooperativeKernel((const void*)k_band_factor, dim3(grid), dim3(kBandThreads), args, kFactorSmem, s));
   count_launches(1);
   FEAB_CHECK_LAUNCH();
-  int32_t aborted = 0;
-  FEAB_CUDA(cudaMemcpyAsync(&aborted, W.abort_flag, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+  if (flag_bytes) FEAB_CUDA(cudaMemsetAsync(band_flags(B), 0, flag_bytes, s));   // left as it was
   BandState h{};
   FEAB_CUDA(cudaMemcpyAsync(&h, st, sizeof(BandState), cudaMemcpyDeviceToHost, s));
   FEAB_CUDA(cudaStreamSynchronize(s));
@@ -1198,7 +1211,7 @@ extern "C" int32_t feab_band_cholesky(feab_band* B, double* pivots_out, cudaStre
     pivots_out[0] = lo;
     pivots_out[1] = hi;
   }
-  if (aborted) return FEAB_CUDA_ERROR;
+  if (h.abort_flag) return FEAB_CUDA_ERROR;
   return h.status == FEAB_OK ? FEAB_OK : h.status;
 }
 
