@@ -6,9 +6,9 @@ splu of K_ff, a singularity test on its pivots (min |U_ii| < tol max |U_ii|, tol
 lu.solve.  K_ff is SPD, so its LU factorisation without pivoting is the Cholesky factorisation
 K_ff = L L^T with U_ii = L_ii^2; the same pivot test is made on the Cholesky pivots.
 
-The free DOFs are renumbered node by node in reverse Cuthill-McKee order of the node graph (the
-ordering is host-side preprocessing, as SuperLU's column ordering is in the reference), so that
-the band of the renumbered K_ff is narrow; the band is factored and solved on the GPU with the
+The free DOFs are renumbered node by node, layer by layer along the mesh's longest extent or in reverse
+Cuthill-McKee order of the node graph (on the host, as SuperLU's column ordering is in the
+reference), so that the band of the renumbered K_ff is narrow; the band is factored and solved on the GPU with the
 feab_band_* kernels (64 x 64 tiles).  The factor of an operator is computed once and reused for
 every right-hand side.
 """
@@ -61,14 +61,46 @@ def coordinate_order(op, coords):
     return np.lexsort((key[:, ax[0]], key[:, ax[1]], key[:, ax[2]])).astype(np.int64)
 
 
+def layer_order(op, coords, sample=2048):
+    """Node row groups sorted layer by layer along the mesh's longest extent, within a layer by the
+    other two, and the number of layers: the coordinates in units of the mesh's own spacing along each
+    axis (the mean length of the longer edges of some nodes), rounded.  Unlike the coordinates
+    themselves, whole layers stay together when the nodes are not exactly in their planes, so the
+    band is one cross-section of nodes wide and not two.  On the operator's device."""
+    p = op.pattern
+    dev = op.vals64.device
+    gp, rp = p.group_ptr.to(torch.int64), p.row_ptr.to(torch.int64)
+    G = gp.numel() - 1
+    dof = torch.nonzero(p.free_map >= 0).flatten()
+    key = torch.as_tensor(np.ascontiguousarray(coords, dtype=float)).to(dev)[dof[gp[:-1]] // 3]
+    some = torch.linspace(0, G - 1, min(G, int(sample)), device=dev).to(torch.int64)
+    start = rp[gp[some]]
+    lens = rp[gp[some] + 1] - start
+    src = torch.repeat_interleave(torch.arange(some.numel(), device=dev), lens)
+    col = torch.arange(src.numel(), device=dev) + (start - torch.cumsum(lens, 0) + lens)[src]
+    nbr = torch.searchsorted(gp, p.col_idx[col].to(torch.int64), right=True) - 1
+    d = (key[nbr] - key[some[src]]).abs()
+    long = d > 0.5 * d.amax(0)
+    h = torch.where(long, d, torch.zeros_like(d)).sum(0) / long.sum(0).clamp_min(1)
+    lo, hi = key.amin(0), key.amax(0)
+    q = ((key - lo) / torch.where(h > 0, h, torch.ones_like(h))).round().to(torch.int64)
+    n_layers = q.amax(0) + 1
+    ext, n_layers = torch.stack([hi - lo, n_layers.to(torch.float64)]).cpu().numpy()     # one read-back
+    ax = np.argsort(ext)
+    code = (q[:, ax[2]] * int(n_layers[ax[1]]) + q[:, ax[1]]) * int(n_layers[ax[0]]) + q[:, ax[0]]
+    return torch.argsort(code, stable=True), int(n_layers[ax[2]])
+
+
 def dof_permutation(op, order):
     """iperm (old reduced row -> new row, int32 device tensor) for the node order `order`."""
-    gp = op.pattern.group_ptr.cpu().numpy().astype(np.int64)
-    sz = (gp[1:] - gp[:-1])[order]
-    old = np.repeat(gp[order], sz) + (np.arange(int(sz.sum())) - np.repeat(np.cumsum(sz) - sz, sz))
-    iperm = np.empty(op.n, np.int32)
-    iperm[old] = np.arange(op.n, dtype=np.int32)
-    return torch.as_tensor(iperm).to(op.vals64.device)
+    dev = op.vals64.device
+    gp = op.pattern.group_ptr.to(torch.int64)
+    order = torch.as_tensor(order).to(dev)
+    sz = gp[1:] - gp[:-1]
+    first = torch.empty_like(sz)
+    first[order] = torch.cumsum(sz[order], 0) - sz[order]
+    group = torch.repeat_interleave(torch.arange(sz.numel(), device=dev), sz, output_size=op.n)
+    return (first[group] + torch.arange(op.n, device=dev) - gp[group]).to(torch.int32)
 
 
 class BandCholesky:
@@ -76,25 +108,37 @@ class BandCholesky:
     would take more than `max_fraction` of the device's free memory."""
 
     def __init__(self, op, coords=None, max_fraction=0.6):
-        """coords: the mesh's node coordinates (N, 3), if known: the ordering along the longest
-        axis is then tried beside reverse Cuthill-McKee, and the narrower band is kept."""
+        """coords: the mesh's node coordinates (N, 3), if known: the ordering in layers along the longest
+        axis is then tried first, and unless its band is about one layer wide, the ordering by
+        coordinates and reverse Cuthill-McKee beside it, and the narrowest band is kept."""
         self.op = op
         dev = op.vals64.device
         if op.pattern.group_ptr is None:
             raise ValueError("the direct solve needs node row groups (an assembled K_ff)")
         csr = op.csr_struct()
         scratch = torch.zeros(2, dtype=torch.int32, device=dev)
-        orders = {"rcm": node_order(op)}
-        if coords is not None:
-            orders["axis"] = coordinate_order(op, coords)
         best = None
-        for name, order in orders.items():
+
+        def consider(name, order):
+            nonlocal best
             iperm = dof_permutation(op, order)
             bw = C.c_int32(0)
             rc = L.lib.feab_band_width(C.byref(csr), L.dptr(iperm), L.dptr(scratch), C.byref(bw), L.stream_ptr(dev))
             L.raise_for(rc, "band width")
             if best is None or bw.value < best[1]:
                 best = (iperm, int(bw.value), name)
+
+        layers = 0
+        if coords is not None:
+            order, layers = layer_order(op, coords)
+            consider("axis", order)
+        # The rows of one layer bound the band of an ordering layer by layer from below.  Within half
+        # as much again the other orderings are not tried: on the box meshes reverse Cuthill-McKee's
+        # band is 2.7 times as wide, and it takes 30 ms of host time at 96x24x24 elements.
+        if coords is None or best[1] > 1.5 * op.n / layers + 6:
+            if coords is not None:
+                consider("axis", coordinate_order(op, coords))
+            consider("rcm", node_order(op))
         self.iperm, self.bandwidth, self.ordering = best
         nbytes = int(L.lib.feab_band_bytes(op.n, self.bandwidth))
         free, _ = torch.cuda.mem_get_info(dev)
