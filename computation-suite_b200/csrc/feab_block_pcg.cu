@@ -26,6 +26,7 @@
 #include <cmath>
 #include "feab_common.cuh"
 #include "feab_graph.cuh"
+#include "feab_pair.cuh"
 
 namespace feab {
 namespace {
@@ -91,6 +92,7 @@ struct BArgs {
   const uint8_t* t_vlo2;
   const int32_t* t_cptr;
   const int32_t* t_chunk;
+  PairView pairs;          // the tiles' pair records (panels of 8 columns or more)
 };
 
 // True in the block that completes the last of problem p's n_items_p work items; `count` items
@@ -120,6 +122,41 @@ __device__ __forceinline__ void block_col_sums(double v, double* sm) {
   for (int s = kThreads / 2; s >= K; s >>= 1) {
     if (threadIdx.x < s) sm[threadIdx.x] += sm[threadIdx.x + s];
     __syncthreads();
+  }
+}
+
+// A problem's per-column totals of NV sums from its items' partial rows (part: 2 K doubles per item), by
+// the whole block: thread t takes every (kThreads / K)-th row of column t % K, eight loads in
+// flight, then the threads of a column are added as a tree; a fixed order.  In threads < K.  One
+// thread per column walking the rows one after the other took longer than the step's vector passes
+// when a problem has many items (250 of 621 us per step at 4,352 items).  HEADS: only the first
+// item of each run of kBRun has a row.
+template <int K, int NV, bool HEADS>
+__device__ __forceinline__ void problem_totals(const double* part, int i0, int i1, double (&s)[NV]) {
+  __shared__ double sm[NV][kThreads];
+  const int c = threadIdx.x % K, h = threadIdx.x / K;
+  constexpr int H = kThreads / K, U = 8;
+  const int rows = HEADS ? (i1 - 1) / kBRun - i0 / kBRun + 1 : i1 - i0;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) s[k] = 0.0;
+  for (int m0 = h; m0 < rows; m0 += U * H) {
+    double v[U][NV];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int m = m0 + u * H;
+      const int row = HEADS && m > 0 ? (i0 / kBRun + m) * kBRun : i0 + m;
+#pragma unroll
+      for (int k = 0; k < NV; ++k) v[u][k] = m < rows ? __ldcg(&part[(int64_t)row * 2 * K + k * K + c]) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int k = 0; k < NV; ++k) s[k] += v[u][k];
+  }
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    block_col_sums<K>(s[k], sm[k]);
+    s[k] = sm[k][c];
   }
 }
 
@@ -635,12 +672,10 @@ __global__ void __launch_bounds__(kThreads) k_bsetup(BArgs A) {
     }
     const int i0 = A.prob_items[p], n_it = A.prob_items[p + 1] - i0;
     if (last_of_problem(&A.ps[p].ticket_a, n_it)) {
+      double tot[2];
+      problem_totals<K, 2, false>(A.part, i0, i0 + n_it, tot);
       if (threadIdx.x < K) {
-        double s0 = 0.0, s1 = 0.0;
-        for (int q = 0; q < n_it; ++q) {
-          s0 += __ldcg(&A.part[(int64_t)(i0 + q) * 2 * K + c]);
-          s1 += __ldcg(&A.part[(int64_t)(i0 + q) * 2 * K + K + c]);
-        }
+        const double s0 = tot[0], s1 = tot[1];
         ColState& C = A.cs[(int64_t)p * K + c];
         double bn = sqrt(s0);
         if (bn == 0.0) bn = 1.0;
@@ -674,6 +709,49 @@ __global__ void __launch_bounds__(kThreads) k_bsetup(BArgs A) {
     }
     __syncthreads();
   }
+}
+
+// The end of a step A over work item it of problem p: the item's per-column sums from the warps' (sm),
+// and by the block that completes the problem, the column's alpha (or, after a reliable step, r.r).
+template <int K>
+__device__ __forceinline__ void finish_step_a(const BArgs& A, int it, int p, bool reliable, const double (*sm)[K]) {
+  if (threadIdx.x < K) {
+    double s = 0.0;
+    for (int q = 0; q < kWarps; ++q) s += sm[q][threadIdx.x];
+    A.part[(int64_t)it * 2 * K + threadIdx.x] = s;
+  }
+  const int i0 = A.prob_items[p], n_it = A.prob_items[p + 1] - i0;
+  if (last_of_problem(&A.ps[p].ticket_a, n_it)) {
+    double tot[1];
+    problem_totals<K, 1, false>(A.part, i0, i0 + n_it, tot);
+    if (threadIdx.x < K) {
+      const int c = threadIdx.x;
+      const double s = tot[0];
+      ColState& C = A.cs[(int64_t)p * K + c];
+      if (reliable) {
+        C.rr = s;
+      } else {
+        C.alpha = 0.0;
+        if (C.active && !C.converged) {
+          if (!(s > 0.0)) atomicCAS(&A.ps[p].status, FEAB_OK, FEAB_NOT_SPD);
+          else C.alpha = C.rz_old / s;
+        }
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      ProbState& Pm = A.ps[p];
+      Pm.ticket_a = 0;
+      if (!reliable) {
+        Pm.pending = 0;
+        if (Pm.status != FEAB_OK) {
+          Pm.done = 1;
+          atomicSub(A.remaining, 1);
+        }
+      }
+    }
+  }
+  __syncthreads();
 }
 
 // Step A: AP = K P (P updated by k_bstep_p; or, in a reliable step, R = B - K64 X);
@@ -762,42 +840,235 @@ __global__ void __launch_bounds__(kThreads, TILES ? FEAB_BLOCK_MINB : FEAB_BLOCK
       for (int q = 0; q < CPL; ++q) sm[w][panel_col<K>(lane, q)] = part[q];
     }
     __syncthreads();
-    if (threadIdx.x < K) {
-      double s = 0.0;
-      for (int q = 0; q < kWarps; ++q) s += sm[q][threadIdx.x];
-      A.part[(int64_t)it * 2 * K + threadIdx.x] = s;
+    finish_step_a<K>(A, it, p, reliable, sm);
+  }
+}
+
+// ---------------------------------------------------------------- pairs on the FP64 tensor path
+// Step A through the tiles' pair records: a warp forms the up to six rows of a pair as an 8 x 8 tile of
+// mma.sync.m8n8k4 per 8 panel columns, four matrix columns at a time.  Fragments: A row-major 8 x 4,
+// lane l holds (l / 4, l % 4): the record's values as they lie (lanes 24 and up hold zero rows); B 4 x
+// 8, lane l holds row l % 4: two adjacent panel columns of that matrix column's panel row by one
+// 16-byte load, one for each of two tiles (an even and an odd one of every 16 columns); C 8 x 8, lane
+// l holds row l / 4, so with both tiles four adjacent panel columns.
+//
+// What bounds it: the FP64 tensor rate (37 TFLOP/s) on the pair's 8 x 108 operand, 56 % of it nonzeros.
+// In the group and tile paths every value reached the lanes as its own shared-memory broadcast, and
+// the L1 data path set the pace; here a value is one lane's register.
+#ifndef FEAB_PAIR_UNROLL
+#define FEAB_PAIR_UNROLL(K) ((K) == 64 ? 2 : ((K) == 32 ? 4 : 8))
+#endif
+#ifndef FEAB_PAIR_MINB
+#define FEAB_PAIR_MINB(K) 2
+#endif
+
+__device__ __forceinline__ void dmma884(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+
+// 16-byte loads of a lane per panel row (K = 8: one 8-byte load).
+constexpr int pair_loads(int K) { return K >= 16 ? K / 16 : 1; }
+
+// Records on their way to a warp: two chunks of up to kPairChunk steps in shared memory, each filled by
+// one bulk copy while the other is applied, so that K's HBM latency is not the gathers'.
+constexpr int kPairChunk = 14;   // a structured pair has 27 steps
+struct __align__(16) PairStage {
+  PairRecord rec[2][kPairChunk];
+  unsigned long long full[2];
+};
+constexpr size_t kPairSmem = kWarps * sizeof(PairStage);
+
+__device__ __forceinline__ void pair_copy(PairStage& st, int buf, const PairRecord* src, int steps) {   // one lane
+  const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&st.full[buf]), bytes = (uint32_t)(steps * sizeof(PairRecord));
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(st.rec[buf])),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+
+// False when the copy does not arrive (some seconds).
+__device__ __forceinline__ bool pair_wait(PairStage& st, int buf, unsigned parity) {
+  const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&st.full[buf]);
+  for (int spin = 0; spin < (1 << 22); ++spin) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
+// acc += the staged records times the panel rows of src.
+template <int K>
+__device__ __forceinline__ void pair_apply(const PairRecord* __restrict__ rec, int steps, int lane,
+                                           const double* __restrict__ src, double (&acc)[K / 8][2]) {
+  constexpr int U = FEAB_PAIR_UNROLL(K), NL = pair_loads(K);
+  const int t = lane & 3, n = lane >> 2;
+  for (int s = 0; s < steps; s += U) {
+    double2 b[U][NL];
+    double a[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (s + u < steps) {   // the same for the whole warp
+        const double* row = src + (int64_t)rec[s + u].col[K >= 16 ? lane >> 3 : t] * K;
+#pragma unroll
+        for (int j = 0; j < NL; ++j) {
+          if (K >= 16) b[u][j] = __ldg(reinterpret_cast<const double2*>(row + 16 * j) + (lane & 7));
+          else b[u][j] = make_double2(__ldg(row + n), 0.0);
+        }
+        a[u] = lane < 24 ? rec[s + u].val[lane] : 0.0;
+      }
     }
-    const int i0 = A.prob_items[p], n_it = A.prob_items[p + 1] - i0;
-    if (last_of_problem(&A.ps[p].ticket_a, n_it)) {
-      if (threadIdx.x < K) {
-        const int c = threadIdx.x;
-        double s = 0.0;
-        for (int q = 0; q < n_it; ++q) s += __ldcg(&A.part[(int64_t)(i0 + q) * 2 * K + c]);
-        ColState& C = A.cs[(int64_t)p * K + c];
-        if (reliable) {
-          C.rr = s;
-        } else {
-          C.alpha = 0.0;
-          if (C.active && !C.converged) {
-            if (!(s > 0.0)) atomicCAS(&A.ps[p].status, FEAB_OK, FEAB_NOT_SPD);
-            else C.alpha = C.rz_old / s;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (s + u < steps) {
+#pragma unroll
+        for (int j = 0; j < NL; ++j) {
+          if constexpr (K >= 16) {
+            // eight lanes read one 128-byte line; the fragment wants row l % 4, columns 2 (l / 4) + {0, 1}
+            const double x = __shfl_sync(FEAB_FULL_MASK, b[u][j].x, 8 * t + n);
+            const double y = __shfl_sync(FEAB_FULL_MASK, b[u][j].y, 8 * t + n);
+            dmma884(acc[2 * j], a[u], x);
+            dmma884(acc[2 * j + 1], a[u], y);
+          } else {
+            dmma884(acc[j], a[u], b[u][j].x);
           }
         }
       }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        ProbState& Pm = A.ps[p];
-        Pm.ticket_a = 0;
-        if (!reliable) {
-          Pm.pending = 0;
-          if (Pm.status != FEAB_OK) {
-            Pm.done = 1;
-            atomicSub(A.remaining, 1);
-          }
+    }
+  }
+}
+
+template <int K, bool MIXED>
+__global__ void __launch_bounds__(kThreads, FEAB_PAIR_MINB(K)) k_bstep_a_pairs(BArgs A) {
+  constexpr int NL = pair_loads(K), W = K >= 16 ? 4 : 2;   // adjacent columns of a lane, NL times
+  __shared__ double sm[kWarps][K];
+  extern __shared__ __align__(16) unsigned char dyn_stage[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, t = lane & 3, r = lane >> 2;
+  PairStage& st = reinterpret_cast<PairStage*>(dyn_stage)[w];
+  if (lane < 2)
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(&st.full[lane])) : "memory");
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  __syncwarp();
+  int buf = 0;
+  unsigned parity[2] = {0u, 0u};
+  for (int it = blockIdx.x; it < A.n_items; it += gridDim.x) {
+    const int p = A.item_problem[it];
+    const ProbState P = A.ps[p];
+    if (P.done) continue;
+    const bool reliable = MIXED && P.mode == kModeReliable;
+    const double* __restrict__ src = reliable ? A.X : A.P0;
+    bool arrived = true;
+    double part[NL][W];
+#pragma unroll
+    for (int j = 0; j < NL; ++j)
+#pragma unroll
+      for (int e = 0; e < W; ++e) part[j][e] = 0.0;
+    int t0, t1;
+    item_tiles(A, it, t0, t1);
+    // the warp's pairs 2 t0 + w, + 8, ..., 32 at a time: lane i holds the i-th one's records and rows
+    for (int q0 = 2 * t0 + w; q0 < 2 * t1; q0 += 32 * kWarps) {
+      const int q = q0 + lane * kWarps;
+      int first = 0, last = 0, row0 = 0, rows = 0;
+      if (q < 2 * t1) {
+        const int g = A.t_g0[q >> 1] + 2 * (q & 1), gn = min(2, A.t_g0[(q >> 1) + 1] - g);
+        if (gn > 0) {
+          first = __ldg(A.pairs.off + q);
+          last = __ldg(A.pairs.off + q + 1);
+          row0 = A.group_ptr[g];
+          rows = A.group_ptr[g + gn] - row0;
         }
       }
+      const int count = min(32, (2 * t1 - q0 + kWarps - 1) / kWarps);
+      int pi = 0, s = 0, e = 0;                              // the next chunk to fetch: pair pi, from record s
+      auto open = [&] {                                      // the first pair from pi on that has records
+        for (; pi < count; ++pi) {
+          s = __shfl_sync(FEAB_FULL_MASK, first, pi);
+          e = __shfl_sync(FEAB_FULL_MASK, last, pi);
+          if (e > s) return;
+        }
+      };
+      auto fetch = [&](int b) {                              // issues the chunk, moves on; its steps (0: none left)
+        if (pi >= count) return 0;
+        const int n = min(kPairChunk, e - s);
+        if (lane == 0) pair_copy(st, b, A.pairs.rec + s, n);
+        s += n;
+        if (s >= e) {
+          ++pi;
+          open();
+        }
+        return n;
+      };
+      open();
+      double acc[K / 8][2];
+#pragma unroll
+      for (int j = 0; j < K / 8; ++j) acc[j][0] = acc[j][1] = 0.0;
+      int cur = pi, steps = fetch(buf);
+      while (steps > 0) {
+        const int nxt = pi, more = fetch(buf ^ 1);           // pair and steps of the chunk behind this one
+        arrived = pair_wait(st, buf, parity[buf]) && arrived;
+        parity[buf] ^= 1u;
+        pair_apply<K>(st.rec[buf], steps, lane, src, acc);
+        __syncwarp();                                        // every lane is done with the chunk
+        if (more == 0 || nxt != cur) {                       // the pair's last chunk: its rows
+          const int r0 = __shfl_sync(FEAB_FULL_MASK, row0, cur), m = __shfl_sync(FEAB_FULL_MASK, rows, cur);
+          if (r < m) {
+            const int64_t base = (int64_t)(r0 + r) * K + W * t;
+#pragma unroll
+            for (int j = 0; j < NL; ++j) {
+              double v[W];
+              if constexpr (K >= 16) {
+                v[0] = acc[2 * j][0];
+                v[1] = acc[2 * j + 1][0];
+                v[2] = acc[2 * j][1];
+                v[3] = acc[2 * j + 1][1];
+              } else {
+                v[0] = acc[j][0];
+                v[1] = acc[j][1];
+              }
+#pragma unroll
+              for (int e2 = 0; e2 < W; e2 += 2) {
+                const int64_t idx = base + 16 * j + e2;
+                if (reliable) {   // R = B - K X and r.r
+                  const double b0 = A.B[idx] - v[e2], b1 = A.B[idx + 1] - v[e2 + 1];
+                  *reinterpret_cast<double2*>(A.R + idx) = make_double2(b0, b1);
+                  part[j][e2] += b0 * b0;
+                  part[j][e2 + 1] += b1 * b1;
+                } else {          // AP and p.Ap
+                  const double2 pv = *reinterpret_cast<const double2*>(A.P0 + idx);
+                  *reinterpret_cast<double2*>(A.AP + idx) = make_double2(v[e2], v[e2 + 1]);
+                  part[j][e2] += pv.x * v[e2];
+                  part[j][e2 + 1] += pv.y * v[e2 + 1];
+                }
+              }
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < K / 8; ++j) acc[j][0] = acc[j][1] = 0.0;
+        }
+        cur = nxt;
+        steps = more;
+        buf ^= 1;
+      }
     }
+    if (!arrived && lane == 0) atomicCAS(&A.ps[p].status, FEAB_OK, FEAB_CUDA_ERROR);
+    // the rows' lanes of each column
+#pragma unroll
+    for (int j = 0; j < NL; ++j)
+#pragma unroll
+      for (int e = 0; e < W; ++e) {
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) part[j][e] += __shfl_xor_sync(FEAB_FULL_MASK, part[j][e], o);
+        if (r == 0) sm[w][16 * j + W * t + e] = part[j][e];
+      }
     __syncthreads();
+    finish_step_a<K>(A, it, p, reliable, sm);
   }
 }
 
@@ -948,7 +1219,6 @@ __global__ void __launch_bounds__(kThreads, FEAB_BLOCK_B_MINB) k_bstep_b(BArgs A
       if (threadIdx.x < K) {
         A.part[(int64_t)it * 2 * K + c] = smv[0][c];
         A.part[(int64_t)it * 2 * K + K + c] = smv[1][c];
-        for (int z = it + 1; z < it2; ++z) A.part[(int64_t)z * 2 * K + c] = A.part[(int64_t)z * 2 * K + K + c] = 0.0;
       }
     } else {
       const double alpha = A.cs[(int64_t)p * K + c].alpha;
@@ -990,7 +1260,6 @@ __global__ void __launch_bounds__(kThreads, FEAB_BLOCK_B_MINB) k_bstep_b(BArgs A
       if (threadIdx.x < K) {
         A.part[(int64_t)it * 2 * K + c] = sm[0][c];
         A.part[(int64_t)it * 2 * K + K + c] = sm[1][c];
-        for (int z = it + 1; z < it2; ++z) A.part[(int64_t)z * 2 * K + c] = A.part[(int64_t)z * 2 * K + K + c] = 0.0;
       }
     }
     const int i0 = A.prob_items[p], n_it = A.prob_items[p + 1] - i0;
@@ -1002,13 +1271,10 @@ __global__ void __launch_bounds__(kThreads, FEAB_BLOCK_B_MINB) k_bstep_b(BArgs A
         flag_any = 0;
         flag_all = 1;
       }
-      __syncthreads();
+      double tot[2];
+      problem_totals<K, 2, true>(A.part, i0, i0 + n_it, tot);
       if (threadIdx.x < K) {
-        double s0 = 0.0, s1 = 0.0;
-        for (int q = 0; q < n_it; ++q) {
-          s0 += __ldcg(&A.part[(int64_t)(i0 + q) * 2 * K + c]);
-          s1 += __ldcg(&A.part[(int64_t)(i0 + q) * 2 * K + K + c]);
-        }
+        const double s0 = tot[0], s1 = tot[1];
         ColState& C = A.cs[(int64_t)p * K + c];
         if (C.active && !C.converged) {
           if (!reliable) C.iters += 1;
@@ -1199,15 +1465,30 @@ int32_t run_block(BArgs A, int prec, int chunk, int maxiter, cudaStream_t s, int
     if (fail(cudaFuncSetAttribute(k_bstep_a<K, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)kStageBytes)))
       break;
+    if constexpr (K >= 8) {
+      if (fail(cudaFuncSetAttribute(k_bstep_a_pairs<K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem)))
+        break;
+      if (fail(cudaFuncSetAttribute(k_bstep_a_pairs<K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem)))
+        break;
+    }
     auto record = [&](cudaStream_t cs) {
       for (int q = 0; q < chunk; ++q) {
         k_bstep_p<K><<<grid_pb, kThreads, 0, cs>>>(A);
+        if constexpr (K >= 8) {
+          if (A.pairs.off) {
+            if (prec == FEAB_PREC_MIXED) k_bstep_a_pairs<K, true><<<grid, kThreads, kPairSmem, cs>>>(A);
+            else k_bstep_a_pairs<K, false><<<grid, kThreads, kPairSmem, cs>>>(A);
+          }
+        }
+        const bool pairs = K >= 8 && A.pairs.off;
         if (prec == FEAB_PREC_MIXED) {
-          if (tiles) k_bstep_a<K, true, true><<<grid, kThreads, smem_a, cs>>>(A);
+          if (pairs) {
+          } else if (tiles) k_bstep_a<K, true, true><<<grid, kThreads, smem_a, cs>>>(A);
           else k_bstep_a<K, true, false><<<grid, kThreads, smem_a, cs>>>(A);
           k_bstep_b<K, true><<<grid_pb, kThreads, 0, cs>>>(A);
         } else {
-          if (tiles) k_bstep_a<K, false, true><<<grid, kThreads, smem_a, cs>>>(A);
+          if (pairs) {
+          } else if (tiles) k_bstep_a<K, false, true><<<grid, kThreads, smem_a, cs>>>(A);
           else k_bstep_a<K, false, false><<<grid, kThreads, smem_a, cs>>>(A);
           k_bstep_b<K, false><<<grid_pb, kThreads, 0, cs>>>(A);
         }
@@ -1219,7 +1500,7 @@ int32_t run_block(BArgs A, int prec, int chunk, int maxiter, cudaStream_t s, int
              fail(cudaMemcpyAsync((void*)hflag, A.remaining, sizeof(int32_t), cudaMemcpyDeviceToHost, s)) ||
              fail(cudaEventRecord(behind, s));
     };
-    if (fail(graphs.acquire(&A, sizeof(A), topo_signature({K, prec, chunk, grid, grid_pb, tiles ? 1 : 0}), record, &exec))) break;
+    if (fail(graphs.acquire(&A, sizeof(A), topo_signature({K, prec, chunk, grid, grid_pb, tiles ? 1 : 0, A.pairs.off ? 1 : 0}), record, &exec))) break;
     // iterations and reliable steps per problem are bounded by maxiter each
     const int64_t max_launch = (2 * (int64_t)maxiter + 2 + chunk - 1) / chunk + 1;
     hflag[0] = np;
@@ -1288,6 +1569,7 @@ bool set_tiles(BArgs& A, const feab_tile_operator* T, int prec) {
   A.t_vlo2 = T->vlo2;
   A.t_cptr = T->cptr;
   A.t_chunk = T->chunk;
+  A.pairs = pair_view(T);
   return true;
 }
 

@@ -12,10 +12,13 @@
 //      a mask), so that the SpMM walks runs of columns shared by the same groups;
 //   5. (build) one warp per group: each list entry finds its mask (binary searches in the tile's
 //      lists), its mask's run and its column there, and writes its rows' values at
-//      3 * (poff + upair + rank of the group among the mask's set bits) + row.
+//      3 * (poff + upair + rank of the group among the mask's set bits) + row;
+//   6. (build) one warp per pair of a tile's groups (0, 1 and 2, 3): the pair records that the
+//      block-PCG's SpMM feeds to the FP64 tensor path (feab_pair.cuh).
 #include <algorithm>
 #include <climits>
 #include "feab_common.cuh"
+#include "feab_pair.cuh"
 #include "feab_scan.cuh"
 
 namespace feab {
@@ -275,12 +278,93 @@ __global__ void __launch_bounds__(kThreads) k_tile_values(int32_t G, Lists Ls, c
   }
 }
 
+// Pair q's groups: 2 (q % 2) and the next of tile q / 2 (count 0 to 2).
+__device__ __forceinline__ int pair_groups(const int32_t* tile_g0, int q, int& count) {
+  const int t = q >> 1, g = tile_g0[t] + 2 * (q & 1);
+  count = min(2, max(0, tile_g0[t + 1] - g));
+  return g;
+}
+
+// First place in cols[0 .. len) whose column is >= c.
+__device__ __forceinline__ int lower_bound(const int32_t* __restrict__ cols, int len, int c) {
+  int lo = 0, hi = len;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (cols[mid] < c) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+
+// One warp per pair, over the CSR's column lists of its one or two groups.  steps == nullptr: the records, at
+// rec + poff[q] (zeroed before); else their number.
+__global__ void __launch_bounds__(kThreads) k_pairs(int32_t n_pairs, const int32_t* __restrict__ group_ptr,
+                                                   const int32_t* __restrict__ row_ptr,
+                                                   const int32_t* __restrict__ col_idx,
+                                                   const double* __restrict__ vals64,
+                                                   const int32_t* __restrict__ tile_g0, int32_t* __restrict__ steps,
+                                                   const int32_t* __restrict__ poff, PairRecord* __restrict__ rec) {
+  const int lane = threadIdx.x & 31;
+  const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (q >= n_pairs) return;
+  int count;
+  const int g = pair_groups(tile_g0, q, count);
+  int r[2] = {0, 0}, f[2] = {0, 0}, len[2] = {0, 0};
+  const int32_t* cols[2] = {col_idx, col_idx};
+  for (int j = 0; j < count; ++j) {
+    r[j] = group_ptr[g + j];
+    f[j] = group_ptr[g + j + 1] - r[j];
+    cols[j] = col_idx + row_ptr[r[j]];
+    len[j] = row_ptr[r[j] + 1] - row_ptr[r[j]];
+  }
+  int common = 0;   // columns of both lists seen so far
+  for (int b = 0; b < len[0]; b += 32) {
+    const int i = b + lane;
+    const int c = i < len[0] ? cols[0][i] : 0;
+    const int at = i < len[0] ? lower_bound(cols[1], len[1], c) : 0;
+    const bool both = i < len[0] && at < len[1] && cols[1][at] == c;
+    const unsigned m = __ballot_sync(FEAB_FULL_MASK, both);
+    if (rec && i < len[0]) {
+      const int pos = i + at - common - __popc(m & ((1u << lane) - 1u));
+      PairRecord& R = rec[(int64_t)poff[q] + (pos >> 2)];
+      R.col[pos & 3] = c;
+      for (int k = 0; k < f[0]; ++k) R.val[4 * k + (pos & 3)] = vals64[row_ptr[r[0] + k] + i];
+      if (both)
+        for (int k = 0; k < f[1]; ++k) R.val[4 * (f[0] + k) + (pos & 3)] = vals64[row_ptr[r[1] + k] + at];
+    }
+    common += __popc(m);
+  }
+  const int total = len[0] + len[1] - common, n_steps = (total + 3) >> 2;
+  if (steps) {
+    if (lane == 0) steps[q] = n_steps;
+    return;
+  }
+  common = 0;
+  for (int b = 0; b < len[1]; b += 32) {
+    const int i = b + lane;
+    const int c = i < len[1] ? cols[1][i] : 0;
+    const int at = i < len[1] ? lower_bound(cols[0], len[0], c) : 0;
+    const bool both = i < len[1] && at < len[0] && cols[0][at] == c;
+    const unsigned m = __ballot_sync(FEAB_FULL_MASK, both);
+    if (i < len[1] && !both) {
+      const int pos = i + at - common - __popc(m & ((1u << lane) - 1u));
+      PairRecord& R = rec[(int64_t)poff[q] + (pos >> 2)];
+      R.col[pos & 3] = c;
+      for (int k = 0; k < f[1]; ++k) R.val[4 * (f[0] + k) + (pos & 3)] = vals64[row_ptr[r[1] + k] + i];
+    }
+    common += __popc(m);
+  }
+  // past the union: the pair's own first row, value 0
+  for (int pos = total + lane; pos < 4 * n_steps; pos += 32) rec[(int64_t)poff[q] + (pos >> 2)].col[pos & 3] = r[0];
+}
+
 struct TileScratch {
   int32_t* pt;      // n_problems + 1
   int32_t* tg0;     // count mode: tile_g0 (n_groups + 1)
   int32_t* ucnt;    // n_groups + 1
   int32_t* pcnt;    // n_groups + 1
   int32_t* ccnt;    // n_groups + 1
+  int32_t* scnt;    // 2 n_groups + 1: steps per pair
   int64_t* scan;
   int64_t* total;   // 1
   int32_t* err;     // 1
@@ -300,7 +384,8 @@ TileScratch scratch_layout(int32_t G, int32_t P, char* base) {
   X.ucnt = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * ((size_t)G + 1)));
   X.pcnt = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * ((size_t)G + 1)));
   X.ccnt = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * ((size_t)G + 1)));
-  const int64_t m = std::max<int64_t>((int64_t)G + 1, (int64_t)P + 1);
+  X.scnt = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * (2 * (size_t)G + 1)));
+  const int64_t m = std::max<int64_t>(2 * (int64_t)G + 1, (int64_t)P + 1);
   X.scan = reinterpret_cast<int64_t*>(take(sizeof(int64_t) * ((size_t)scan_blocks(m) + 2)));
   X.total = reinterpret_cast<int64_t*>(take(sizeof(int64_t)));
   X.err = reinterpret_cast<int32_t*>(take(sizeof(int32_t)));
@@ -308,9 +393,10 @@ TileScratch scratch_layout(int32_t G, int32_t P, char* base) {
   return X;
 }
 
-// Storage layout of the operator for n_tiles tiles, nu union columns and np pairs.
-size_t storage_layout(int32_t n_tiles, int32_t G, int64_t nu, int64_t np, int64_t nch, int prec, char* base,
-                      feab_tile_operator* T) {
+// Storage layout of the operator for n_tiles tiles, nu union columns, np (column, group) pairs and ns
+// steps of pair records.
+size_t storage_layout(int32_t n_tiles, int32_t G, int64_t nu, int64_t np, int64_t nch, int64_t ns, int prec,
+                      char* base, feab_tile_operator* T) {
   size_t off = 0;
   auto take = [&](size_t b) {
     char* p = base ? base + off : nullptr;
@@ -335,7 +421,10 @@ size_t storage_layout(int32_t n_tiles, int32_t G, int64_t nu, int64_t np, int64_
     lo = take(sizeof(uint16_t) * nv);
     lo2 = take(nv);
   }
+  const size_t pairs = off;
+  take(pair_section_bytes(n_tiles, ns));
   if (T) {
+    T->reserved = (int32_t)(pairs / 256);   // see pair_view()
     T->tile_g0 = reinterpret_cast<int32_t*>(tg);
     T->group_tile = reinterpret_cast<int32_t*>(gt);
     T->uoff = reinterpret_cast<int32_t*>(uo);
@@ -412,12 +501,21 @@ extern "C" int32_t feab_tile_operator_build(const feab_csr* M, const feab_diff_o
   FEAB_CUDA(cudaMemcpyAsync(&nch, X.total, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   FEAB_CUDA(cudaStreamSynchronize(s));
   if (nu >= (int64_t)INT32_MAX || 3 * np >= (int64_t)INT32_MAX) return FEAB_CAPACITY;
-  const size_t need = storage_layout(n_tiles, G, nu, np, nch, prec, nullptr, nullptr);
+  const int pw = kThreads / 32, pair_blocks = (2 * n_tiles + pw - 1) / pw;
+  k_pairs<<<pair_blocks, kThreads, 0, s>>>(2 * n_tiles, M->group_ptr, M->row_ptr, M->col_idx, M->vals64, X.tg0, X.scnt,
+                                           nullptr, nullptr);
+  count_launches(1);
+  FEAB_CHECK_LAUNCH();
+  int64_t ns = 0;
+  FEAB_CUDA(scan_exclusive_i32(X.scnt, X.scnt, 2 * (int64_t)n_tiles, X.scan, X.total, s));
+  FEAB_CUDA(cudaMemcpyAsync(&ns, X.total, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  FEAB_CUDA(cudaStreamSynchronize(s));
+  const size_t need = storage_layout(n_tiles, G, nu, np, nch, ns, prec, nullptr, nullptr);
   if (bytes_out) *bytes_out = need;
   if (!storage) return FEAB_OK;
   if (need > storage_bytes) return FEAB_BAD_ARG;
   feab_tile_operator T{};
-  storage_layout(n_tiles, G, nu, np, nch, prec, static_cast<char*>(storage), &T);
+  storage_layout(n_tiles, G, nu, np, nch, ns, prec, static_cast<char*>(storage), &T);
   T.n_tiles = n_tiles;
   T.precision = prec;
   T.n_groups = G;
@@ -432,7 +530,13 @@ extern "C" int32_t feab_tile_operator_build(const feab_csr* M, const feab_diff_o
   k_tile_values<<<(G + wpb - 1) / wpb, kThreads, 0, s>>>(
       G, Ls, M->vals64, D ? D->vhi : nullptr, D ? D->vlo : nullptr, D ? D->vlo2 : nullptr, D ? D->voff : nullptr,
       T.tile_g0, T.group_tile, T.uoff, T.poff, T.ucol, T.umask, T.upair, T.v64, T.vhi, T.vlo, T.vlo2, X.err);
-  count_launches(3);
+  const PairView V = pair_view(&T);
+  FEAB_CUDA(cudaMemcpyAsync(const_cast<int32_t*>(V.off), X.scnt, sizeof(int32_t) * (2 * (size_t)n_tiles + 1),
+                            cudaMemcpyDeviceToDevice, s));
+  FEAB_CUDA(cudaMemsetAsync(const_cast<PairRecord*>(V.rec), 0, sizeof(PairRecord) * (size_t)ns, s));
+  k_pairs<<<pair_blocks, kThreads, 0, s>>>(2 * n_tiles, M->group_ptr, M->row_ptr, M->col_idx, M->vals64, T.tile_g0, nullptr,
+                                           V.off, const_cast<PairRecord*>(V.rec));
+  count_launches(4);
   FEAB_CHECK_LAUNCH();
   FEAB_CUDA(cudaMemcpyAsync(&err, X.err, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
   FEAB_CUDA(cudaStreamSynchronize(s));

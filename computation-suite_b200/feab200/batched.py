@@ -204,7 +204,7 @@ def tuning_cache_path():
 
 
 def tuning_key(device_name, n, nnz, n_problems, k, precision):
-    return f"{device_name}|n={n}|nnz={nnz}|problems={n_problems}|k={k}|{precision}|spmm=tiles{TILE_GROUPS}"
+    return f"{device_name}|n={n}|nnz={nnz}|problems={n_problems}|k={k}|{precision}|spmm=tiles{TILE_GROUPS}p"
 
 
 def load_tuning(path=None):

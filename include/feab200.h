@@ -350,7 +350,8 @@ typedef struct feab_tile_operator {
   int32_t n_tiles;
   int32_t precision;     /* FEAB_PREC_FP64 or FEAB_PREC_MIXED                         */
   int32_t n_groups;
-  int32_t reserved;
+  int32_t reserved;      /* place of the pair records (0: none): block-PCG panels of 8 */
+                         /*   or more columns then run on the FP64 tensor path         */
   int32_t* tile_g0;      /* n_tiles + 1: first row group of each tile                  */
   int32_t* group_tile;   /* n_groups: tile of each row group                           */
   int32_t* uoff;         /* n_tiles + 1: first union column (a multiple of 4)          */
