@@ -600,55 +600,90 @@ __global__ void __launch_bounds__(32 * kReduceWarps) k_gram_reduce(const double*
 }
 
 // One-block cyclic Jacobi eigensolver for a symmetric k x k FP64 matrix (k <= 64), round-robin
-// ordering (k/2 disjoint rotations per round).  Eigenvalues sorted descending into w; A is
-// overwritten.  Bounded by max_sweeps.
-__global__ void k_symeig_jacobi(double* A, int k, double* w, double* V, int max_sweeps, int* sweeps_out) {
+// ordering (k / 2 disjoint rotations per round).  Eigenvalues sorted descending into w; A is read
+// only.  Bounded by max_sweeps.
+//
+// A round is two steps.  The rotations: one thread per pair of indices, c and s from the half-angle
+// formulas cos 2t = |d| / h, sin 2t = b / h, h = sqrt(d^2 + b^2), with d the difference of the two
+// diagonal entries and b twice the off-diagonal one (two reciprocal square roots, no division).  The
+// update: one thread per pair of pairs applies both rotations to its 2 x 2 block, on and above the
+// diagonal, and mirrors it, so that the matrix stays symmetric; every thread turns two rows' pairs
+// of V.  The matrix is first scaled by a power of two to entries of at most one.
+//
+// What bounds it: latency, a round's chain of some 20 dependent FP64 operations (16 cycles each, 45
+// for a reciprocal square root) and two barriers.  Measured at k = 64: 2,366 us before, when one
+// thread added up the off-diagonal before each sweep, sorted and wrote V, and rows and columns were
+// turned in two steps.
+constexpr int kJacThreads = 1024;
+
+// Sum of v over the block, in every thread.
+__device__ __forceinline__ double jac_block_sum(double v, double* sh) {
+  v = warp_sum(v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return warp_sum(sh[threadIdx.x & 31]);
+}
+
+__global__ void __launch_bounds__(kJacThreads) k_symeig_jacobi(const double* A, int k, double* w, double* V,
+                                                              int max_sweeps, int* sweeps_out) {
   extern __shared__ double jac_smem[];
   double (*a)[65] = reinterpret_cast<double (*)[65]>(jac_smem);
   double (*v)[65] = reinterpret_cast<double (*)[65]>(jac_smem + 64 * 65);
-  __shared__ double cs[32], sn[32];
+  __shared__ double cs[32], sn[32], red[32];
   __shared__ int pp[32], qq[32];
-  __shared__ double off;
-  const int tid = threadIdx.x, nt = blockDim.x;
+  const int tid = threadIdx.x;
   const int kk = (k + 1) & ~1;  // even size (a zero row/col pads odd k)
-  for (int i = tid; i < kk * kk; i += nt) {
+  const int half = kk / 2;
+  for (int i = tid; i < kk * kk; i += kJacThreads) {
     const int r = i / kk, c = i % kk;
     a[r][c] = (r < k && c < k) ? A[r * k + c] : 0.0;
     v[r][c] = r == c ? 1.0 : 0.0;
   }
   __syncthreads();
-  double fro = 0.0;
-  if (tid == 0) {
-    for (int r = 0; r < kk; ++r)
-      for (int c = 0; c < kk; ++c) fro += a[r][c] * a[r][c];
-    off = fro;
-  }
+  double big = 0.0;
+  for (int i = tid; i < kk * kk; i += kJacThreads) big = fmax(big, fabs(a[i / kk][i % kk]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(FEAB_FULL_MASK, big, o));
+  if ((tid & 31) == 0) red[tid >> 5] = big;
   __syncthreads();
-  const double tol = 1e-30 * (off > 0 ? off : 1.0);
+  big = red[tid & 31];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(FEAB_FULL_MASK, big, o));
+  int e = 0;
+  if (big > 0.0 && big <= 1.7976931348623157e308) frexp(big, &e);
+  double fro = 0.0;
+  for (int i = tid; i < kk * kk; i += kJacThreads) {
+    const double x = scalbn(a[i / kk][i % kk], -e);
+    a[i / kk][i % kk] = x;
+    fro += x * x;
+  }
+  fro = jac_block_sum(fro, red);
+  const double tol = 1e-30 * (fro > 0 ? fro : 1.0);
   int sweep = 0;
   for (; sweep < max_sweeps; ++sweep) {
-    if (tid == 0) {
-      double o = 0.0;
-      for (int r = 0; r < kk; ++r)
-        for (int c = 0; c < kk; ++c)
-          if (r != c) o += a[r][c] * a[r][c];
-      off = o;
-    }
-    __syncthreads();
+    double off = 0.0;
+    for (int i = tid; i < kk * kk; i += kJacThreads)
+      if (i / kk != i % kk) off += a[i / kk][i % kk] * a[i / kk][i % kk];
+    off = jac_block_sum(off, red);
     if (off <= tol) break;
     for (int round = 0; round < kk - 1; ++round) {
-      if (tid < kk / 2) {
+      if (tid < half) {
         // round-robin pairing: position 0 fixed, others rotate
-        int i1 = tid == 0 ? 0 : ((tid - 1 + round) % (kk - 1)) + 1;
-        int i2 = ((kk - 2 - tid + round) % (kk - 1)) + 1;
+        int i1 = tid - 1 + round, i2 = kk - 2 - tid + round;
+        if (i1 >= kk - 1) i1 -= kk - 1;
+        if (i2 >= kk - 1) i2 -= kk - 1;
+        i1 = tid == 0 ? 0 : i1 + 1;
+        ++i2;
         const int p = min(i1, i2), q = max(i1, i2);
-        const double apq = a[p][q], app = a[p][p], aqq = a[q][q];
+        const double b = 2.0 * a[p][q], d = a[q][q] - a[p][p];
+        const double h2 = fma(d, d, b * b);
         double c = 1.0, s = 0.0;
-        if (apq != 0.0) {
-          const double tau = (aqq - app) / (2.0 * apq);
-          const double t = (tau >= 0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-          c = 1.0 / sqrt(1.0 + t * t);
-          s = t * c;
+        if (b != 0.0 && !(h2 < 1e-290)) {
+          const double rh = rsqrt(h2);
+          const double c2 = fma(0.5 * fabs(d), rh, 0.5), rc = rsqrt(c2);   // cos^2 t >= 1/2
+          c = c2 * rc;
+          s = copysign(0.5, d) * b * rh * rc;
         }
         pp[tid] = p;
         qq[tid] = q;
@@ -656,50 +691,51 @@ __global__ void k_symeig_jacobi(double* A, int k, double* w, double* V, int max_
         sn[tid] = s;
       }
       __syncthreads();
-      // rows: a <- J^T a
-      for (int i = tid; i < (kk / 2) * kk; i += nt) {
-        const int r = i / kk, col = i % kk;
-        const int p = pp[r], q = qq[r];
-        const double c = cs[r], s = sn[r];
-        const double x = a[p][col], y = a[q][col];
-        a[p][col] = c * x - s * y;
-        a[q][col] = s * x + c * y;
+      const int P = tid >> 5, Q = tid & 31;
+      if (P <= Q && Q < half) {
+        const int p = pp[P], q = qq[P], r = pp[Q], u = qq[Q];
+        const double cp = cs[P], sp = sn[P], cq = cs[Q], sq = sn[Q];
+        const double x00 = a[p][r], x01 = a[p][u], x10 = a[q][r], x11 = a[q][u];
+        const double y00 = fma(cp, x00, -(sp * x10)), y10 = fma(sp, x00, cp * x10);
+        const double y01 = fma(cp, x01, -(sp * x11)), y11 = fma(sp, x01, cp * x11);
+        double z00 = fma(cq, y00, -(sq * y01)), z01 = fma(sq, y00, cq * y01);
+        double z10 = fma(cq, y10, -(sq * y11)), z11 = fma(sq, y10, cq * y11);
+        if (P == Q && sp != 0.0) z01 = z10 = 0.0;
+        a[p][r] = z00;
+        a[p][u] = z01;
+        a[q][r] = z10;
+        a[q][u] = z11;
+        if (P != Q) {
+          a[r][p] = z00;
+          a[u][p] = z01;
+          a[r][q] = z10;
+          a[u][q] = z11;
+        }
       }
-      __syncthreads();
-      // columns: a <- a J ; v <- v J
-      for (int i = tid; i < (kk / 2) * kk; i += nt) {
-        const int r = i / kk, row = i % kk;
+      for (int i = tid; i < half * kk; i += kJacThreads) {
+        const int r = i / kk, row = i - r * kk;
         const int p = pp[r], q = qq[r];
         const double c = cs[r], s = sn[r];
-        const double x = a[row][p], y = a[row][q];
-        a[row][p] = c * x - s * y;
-        a[row][q] = s * x + c * y;
         const double vx = v[row][p], vy = v[row][q];
-        v[row][p] = c * vx - s * vy;
-        v[row][q] = s * vx + c * vy;
+        v[row][p] = fma(c, vx, -(s * vy));
+        v[row][q] = fma(s, vx, c * vy);
       }
       __syncthreads();
     }
   }
-  if (tid == 0) {
-    // selection sort of the diagonal, descending (k <= 64)
-    int order[64];
-    for (int i = 0; i < k; ++i) order[i] = i;
-    for (int i = 0; i < k; ++i) {
-      int best = i;
-      for (int j = i + 1; j < k; ++j)
-        if (a[order[j]][order[j]] > a[order[best]][order[best]]) best = j;
-      const int t = order[i];
-      order[i] = order[best];
-      order[best] = t;
-    }
-    for (int i = 0; i < k; ++i) {
-      w[i] = a[order[i]][order[i]];
-      if (V)
-        for (int r = 0; r < k; ++r) V[r * k + i] = v[r][order[i]];
-    }
-    if (sweeps_out) *sweeps_out = sweep;
+  // descending order: an eigenvalue's place is the number of those before it
+  __shared__ int place[64];
+  if (tid < k) {
+    const double x = a[tid][tid];
+    int at = 0;
+    for (int j = 0; j < k; ++j) at += a[j][j] > x || (!(a[j][j] < x) && j < tid) ? 1 : 0;
+    place[tid] = at;
+    w[at] = scalbn(x, e);
   }
+  __syncthreads();
+  if (V)
+    for (int i = tid; i < k * k; i += kJacThreads) V[(i / k) * k + place[i % k]] = v[i / k][i % k];
+  if (tid == 0 && sweeps_out) *sweeps_out = sweep;
 }
 
 // FP64 Gram on the CUDA cores: G = X^T X accumulated in FP64 for X (n x 64, FP32 or FP64, row
@@ -847,7 +883,7 @@ extern "C" int32_t feab_symeig_jacobi(double* A, int32_t k, double* evals, doubl
   if (!A || !evals || k <= 0 || k > 64) return FEAB_BAD_ARG;
   const size_t smem = sizeof(double) * 2 * 64 * 65;
   FEAB_CUDA(cudaFuncSetAttribute(k_symeig_jacobi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_symeig_jacobi<<<1, 256, smem, s>>>(A, k, evals, evecs, max_sweeps > 0 ? max_sweeps : 40, sweeps_out);
+  k_symeig_jacobi<<<1, kJacThreads, smem, s>>>(A, k, evals, evecs, max_sweeps > 0 ? max_sweeps : 40, sweeps_out);
   count_launches(1);
   FEAB_CHECK_LAUNCH();
   return FEAB_OK;

@@ -94,22 +94,74 @@ __global__ void __launch_bounds__(32 * kPReduceWarps) k_panel_gram_reduce(const 
   if (lane == 0) C[idx] = s;
 }
 
-// Z = Y V: V (k x m) staged in shared memory; thread (row, col) of the n x m output.
-__global__ void __launch_bounds__(kPThreads) k_panel_small(const double* __restrict__ Y, int ldy, int64_t n, int k,
-                                                          const double* __restrict__ V, int m,
-                                                          double* __restrict__ Z, int ldz) {
-  __shared__ double vs[kP * kP];
-  for (int e = threadIdx.x; e < k * m; e += kPThreads) vs[e] = V[e];
-  __syncthreads();
-  const int64_t total = n * (int64_t)m;
-  for (int64_t e = (int64_t)blockIdx.x * kPThreads + threadIdx.x; e < total; e += (int64_t)gridDim.x * kPThreads) {
-    const int64_t i = e / m;
-    const int c = (int)(e - i * m);
-    const double* y = Y + i * (int64_t)ldy;
-    double s = 0.0;
-    for (int j = 0; j < k; ++j) s = fma(__ldg(y + j), vs[j * m + c], s);
-    Z[i * (int64_t)ldz + c] = s;
+// Z = Y V, Y of FP64 or FP32 values: a CTA stages 128 rows of Y (padded, so that a warp's 32 rows read
+// one column without bank conflicts) and V in shared memory; thread (row, half) forms eight columns
+// of its row at a time, the sums over j in order.  What bounds it: reading Y once (33 us at 418,176 x
+// 64 FP64) and, close behind, the shared-memory reads (V's values are broadcasts, two per read).
+// Measured there with m = 10: 303 us when every output read its row of Y from L1 by itself.
+constexpr int kSmallRows = 128;
+constexpr int kSmallLd = kP + 1;
+constexpr size_t kSmallSmem = sizeof(double) * (kSmallRows * kSmallLd + kP * kP);
+
+template <typename T>
+__global__ void __launch_bounds__(kPThreads) k_panel_small(const T* __restrict__ Y, int ldy, int64_t n, int k,
+                                                          const double* __restrict__ V, int m, double* __restrict__ Z,
+                                                          int ldz) {
+  extern __shared__ __align__(16) double small_sm[];
+  double* vs = small_sm;                  // vs[j * mp + c], mp = m rounded up to 8, zeros past m
+  double* ys = small_sm + kP * kP;        // ys[r * kSmallLd + j]
+  const int tid = threadIdx.x, mp = (m + 7) & ~7;
+  for (int e = tid; e < k * mp; e += kPThreads) {
+    const int j = e / mp, c = e - j * mp;
+    vs[e] = c < m ? V[j * m + c] : 0.0;
   }
+  const int r = tid & (kSmallRows - 1), h = tid / kSmallRows;
+  for (int64_t r0 = (int64_t)blockIdx.x * kSmallRows; r0 < n; r0 += (int64_t)gridDim.x * kSmallRows) {
+    __syncthreads();
+    const int rows = (int)min((int64_t)kSmallRows, n - r0);
+    for (int e = tid; e < kSmallRows * kP; e += kPThreads) {
+      const int i = e / kP, j = e % kP;
+      if (i < rows && j < k) ys[i * kSmallLd + j] = (double)__ldcs(Y + (r0 + i) * (int64_t)ldy + j);
+    }
+    __syncthreads();
+    if (r < rows) {
+      for (int c0 = 8 * h; c0 < m; c0 += 16) {
+        double s[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) s[c] = 0.0;
+#pragma unroll 4
+        for (int j = 0; j < k; ++j) {
+          const double y = ys[r * kSmallLd + j];
+          const double2* vj = reinterpret_cast<const double2*>(vs + j * mp + c0);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const double2 vv = vj[c];
+            s[2 * c] = fma(y, vv.x, s[2 * c]);
+            s[2 * c + 1] = fma(y, vv.y, s[2 * c + 1]);
+          }
+        }
+        double* z = Z + (r0 + r) * (int64_t)ldz + c0;
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          if (c0 + c < m) z[c] = s[c];
+      }
+    }
+  }
+}
+
+template <typename T>
+int32_t launch_panel_small(const T* Y, int32_t ldy, int64_t n, int32_t k, const double* V, int32_t m, double* Z,
+                           int32_t ldz, cudaStream_t s) {
+  if (!Y || !V || !Z || n <= 0 || k < 1 || k > kP || m < 1 || m > kP || ldy < k || ldz < m ||
+      static_cast<const void*>(Y) == Z)
+    return FEAB_BAD_ARG;
+  FEAB_CUDA(cudaFuncSetAttribute(k_panel_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem));
+  const int64_t tiles = (n + kSmallRows - 1) / kSmallRows;
+  const int grid = (int)std::min<int64_t>(tiles, 2 * (int64_t)sm_count());
+  k_panel_small<T><<<grid, kPThreads, kSmallSmem, s>>>(Y, ldy, n, k, V, m, Z, ldz);
+  count_launches(1);
+  FEAB_CHECK_LAUNCH();
+  return FEAB_OK;
 }
 
 int panel_grid(int64_t n) {
@@ -142,12 +194,10 @@ extern "C" int32_t feab_panel_gram(const double* X, int32_t ldx, const double* Y
 
 extern "C" int32_t feab_panel_small(const double* Y, int32_t ldy, int64_t n, int32_t k, const double* V, int32_t m,
                                     double* Z, int32_t ldz, cudaStream_t s) {
-  if (!Y || !V || !Z || n <= 0 || k < 1 || k > kP || m < 1 || m > kP || ldy < k || ldz < m) return FEAB_BAD_ARG;
-  if (Z == Y) return FEAB_BAD_ARG;  // every output row reads its whole input row
-  const int64_t blocks = (n * (int64_t)m + kPThreads - 1) / kPThreads;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(blocks, (int64_t)sm_count() * 8));
-  k_panel_small<<<grid, kPThreads, 0, s>>>(Y, ldy, n, k, V, m, Z, ldz);
-  count_launches(1);
-  FEAB_CHECK_LAUNCH();
-  return FEAB_OK;
+  return launch_panel_small(Y, ldy, n, k, V, m, Z, ldz, s);
+}
+
+extern "C" int32_t feab_panel_small_f32(const float* Y, int32_t ldy, int64_t n, int32_t k, const double* V, int32_t m,
+                                        double* Z, int32_t ldz, cudaStream_t s) {
+  return launch_panel_small(Y, ldy, n, k, V, m, Z, ldz, s);
 }

@@ -128,6 +128,7 @@ SIGNATURES = {
     "feab_panel_gram_workspace_bytes": (_SZ, [_I64]),
     "feab_panel_gram": (_I32, [_P, _I32, _P, _I32, _I64, _I32, _P, _P, _SZ, _P]),
     "feab_panel_small": (_I32, [_P, _I32, _I64, _I32, _P, _I32, _P, _I32, _P]),
+    "feab_panel_small_f32": (_I32, [_P, _I32, _I64, _I32, _P, _I32, _P, _I32, _P]),
     "feab_gram_workspace_bytes": (_SZ, [_I64, _I32]),
     "feab_gram_bf16x3": (_I32, [_P, _I64, _I32, _P, _P, _SZ, _P, _P]),
     "feab_gram_fp64": (_I32, [_P, _I32, _I64, _I32, _P, _P, _SZ, _P]),

@@ -56,13 +56,21 @@ def panel_gram(X, Y):
 
 def panel_small(Y, V):
     """Y V for an (n, k) device panel and a (k, m) device matrix, k, m <= 64."""
-    Y = _f64_panel(Y, "Y")
+    return _panel_small(_f64_panel(Y, "Y"), V, L.lib.feab_panel_small)
+
+
+def panel_small_f32(Y, V):
+    """panel_small for a float32 panel Y with unit column stride; the sums and the result are float64."""
+    return _panel_small(Y, V, L.lib.feab_panel_small_f32)
+
+
+def _panel_small(Y, V, entry):
     V = _f64_panel(V, "V").contiguous()
     n, k = Y.shape
     if V.shape[0] != k or V.shape[1] > 64 or k > 64:
         raise ValueError(f"panel_small: V must be ({k}, m <= 64), got {tuple(V.shape)}")
     m = V.shape[1]
     Z = torch.empty((n, m), dtype=torch.float64, device=Y.device)
-    rc = L.lib.feab_panel_small(L.dptr(Y), Y.stride(0), n, k, L.dptr(V), m, L.dptr(Z), m, L.stream_ptr(Y.device))
+    rc = entry(L.dptr(Y), Y.stride(0), n, k, L.dptr(V), m, L.dptr(Z), m, L.stream_ptr(Y.device))
     L.raise_for(rc, "panel_small")
     return Z

@@ -28,7 +28,7 @@ import torch
 
 from . import _lib as L
 from .device import cuda_device
-from .panel import panel_small
+from .panel import panel_small, panel_small_f32
 
 MAX_SNAPSHOTS = 64
 
@@ -152,8 +152,11 @@ class PodBasis:
         if gram == "auto":
             gram = "int8" if X.dtype == torch.float32 else "fp64"
         dt = torch.float64 if gram == "fp64" else torch.float32
-        Xp = torch.zeros((n, MAX_SNAPSHOTS), dtype=dt, device=dev)
-        Xp[:, :k] = X.to(dt)
+        if k == MAX_SNAPSHOTS and X.dtype == dt and X.is_contiguous() and X.data_ptr() % 16 == 0:
+            Xp = X                                           # a whole panel as the Gram kernels read it
+        else:
+            Xp = torch.zeros((n, MAX_SNAPSHOTS), dtype=dt, device=dev)
+            Xp[:, :k] = X.to(dt)
         G = {"bf16x3": gram_bf16x3, "int8": gram_int8, "fp64": gram_fp64}[gram](Xp)
         w, V = symeig(G)
         S = torch.sqrt(torch.clamp(w[: min(k, n)], min=0.0))
@@ -162,7 +165,11 @@ class PodBasis:
         Vk = V[:k, :r]                                       # eigenvectors of the k x k Gram block
         inv = torch.where(S[:r] > 0, 1.0 / S[:r], torch.zeros_like(S[:r]))
         # method of snapshots: U = X V / sigma, as one panel product (V scaled by 1 / sigma first)
-        self.V = panel_small(X.to(torch.float64), (Vk * inv[None, :]).contiguous())
+        W = (Vk * inv[None, :]).contiguous()
+        if X.dtype == torch.float32 and X.stride(1) == 1 and X.stride(0) >= k:
+            self.V = panel_small_f32(X, W)                   # the values widen to FP64 in the kernel
+        else:
+            self.V = panel_small(X.to(torch.float64), W)
         self.singular_values = S_host
         self.n_modes = r
         return self

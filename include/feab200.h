@@ -446,10 +446,13 @@ int32_t feab_panel_gram(const double* X, int32_t ldx, const double* Y, int32_t l
  * (rom_engine/src/rom_engine/pod.py:140-160).  Asynchronous. */
 int32_t feab_panel_small(const double* Y, int32_t ldy, int64_t n, int32_t k, const double* V, int32_t m, double* Z,
                          int32_t ldz, cudaStream_t stream);
+/* The same for an FP32 panel Y (the products and sums are FP64). */
+int32_t feab_panel_small_f32(const float* Y, int32_t ldy, int64_t n, int32_t k, const double* V, int32_t m, double* Z,
+                             int32_t ldz, cudaStream_t stream);
 
 /* Cyclic Jacobi eigensolver (one CTA, FP64) for a symmetric k x k matrix (k <= 64) in device
  * memory: eigenvalues descending into evals, eigenvectors (columns) into evecs (may be NULL).
- * A is overwritten.  *sweeps_out (device int, may be NULL) receives the sweeps used. */
+ * A may be overwritten.  *sweeps_out (device int, may be NULL) receives the sweeps used. */
 int32_t feab_symeig_jacobi(double* A, int32_t k, double* evals, double* evecs, int32_t max_sweeps,
                            int32_t* sweeps_out, cudaStream_t stream);
 
