@@ -599,143 +599,249 @@ __global__ void __launch_bounds__(32 * kReduceWarps) k_gram_reduce(const double*
   if (lane == 0) G[idx] = 0.5 * (s + t);
 }
 
-// One-block cyclic Jacobi eigensolver for a symmetric k x k FP64 matrix (k <= 64), round-robin
-// ordering (k / 2 disjoint rotations per round).  Eigenvalues sorted descending into w; A is read
-// only.  Bounded by max_sweeps.
+// Cyclic Jacobi eigensolver for a symmetric k x k FP64 matrix (k <= 64), round-robin ordering (k / 2
+// disjoint rotations per round), on a cluster of three CTAs.  Eigenvalues sorted descending into w; A
+// is read only.  Bounded by max_sweeps.
 //
-// A round is two steps.  The rotations: one thread per pair of indices, c and s from the half-angle
-// formulas cos 2t = |d| / h, sin 2t = b / h, h = sqrt(d^2 + b^2), with d the difference of the two
-// diagonal entries and b twice the off-diagonal one (two reciprocal square roots, no division).  The
-// update: one thread per pair of pairs applies both rotations to its 2 x 2 block, on and above the
-// diagonal, and mirrors it, so that the matrix stays symmetric; every thread turns two rows' pairs
-// of V.  The matrix is first scaled by a power of two to entries of at most one.
+// CTA 0 turns the matrix (its upper triangle).  A round is two steps.  The rotations: one thread per
+// pair of indices, c and s from the half-angle formulas cos 2t = |d| / h, sin 2t = b / h, h = sqrt(d^2 +
+// b^2), with d the difference of the two diagonal entries and b twice the off-diagonal one (two
+// reciprocal square roots, no division).  The update: one thread per pair of pairs applies both
+// rotations to its 2 x 2 block.  The matrix is first scaled by a power of two to entries of at most
+// one.  CTAs 1 and 2 turn half of V's rows each, some rounds behind: a round's (c, s) go into their
+// shared memory (st.async), where a sweep's rounds have a place each, and the CTAs meet after each sweep.
 //
-// What bounds it: latency, a round's chain of some 20 dependent FP64 operations (16 cycles each, 45
-// for a reciprocal square root) and two barriers.  Measured at k = 64: 2,366 us before, when one
-// thread added up the off-diagonal before each sweep, sorted and wrote V, and rows and columns were
-// turned in two steps.
-constexpr int kJacThreads = 1024;
+// What bounds it: a round's chain of some 20 dependent FP64 operations (16 cycles each, 45 for a
+// reciprocal square root), two barriers and the update's shared-memory accesses.  Measured for a POD
+// Gram matrix (k = 64, 12 sweeps): 2,366 us when one thread added up the off-diagonal before each
+// sweep, sorted and wrote V, and rows and columns were turned in two steps; 1,049 us with these in
+// parallel and V turned by the same CTA.
+constexpr int kJacThreads = 544;          // 528 pairs of pairs
+constexpr int kJacCluster = 3;
+constexpr int kJacVRows = 32;             // of V per CTA
+
+struct JacShared {
+  double a[64][65];                       // CTA 0: the matrix (row <= column); the others: their rows of V
+  double2 rot[64][32];                    // a sweep's rounds: (c, s) of each pair
+  double cs[32], sn[32], red[32];
+  int place[64];
+  unsigned long long full[64];
+  int go[2];                              // another sweep? (even and odd sweeps: a slow CTA still reads the last)
+  int bad;                                // a wait ran out
+};
 
 // Sum of v over the block, in every thread.
 __device__ __forceinline__ double jac_block_sum(double v, double* sh) {
+  const int nw = kJacThreads / 32, lane = threadIdx.x & 31;
   v = warp_sum(v);
   __syncthreads();
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  if (lane == 0) sh[threadIdx.x >> 5] = v;
   __syncthreads();
-  return warp_sum(sh[threadIdx.x & 31]);
+  return warp_sum(lane < nw ? sh[lane] : 0.0);
 }
 
-__global__ void __launch_bounds__(kJacThreads) k_symeig_jacobi(const double* A, int k, double* w, double* V,
-                                                              int max_sweeps, int* sweeps_out) {
-  extern __shared__ double jac_smem[];
-  double (*a)[65] = reinterpret_cast<double (*)[65]>(jac_smem);
-  double (*v)[65] = reinterpret_cast<double (*)[65]>(jac_smem + 64 * 65);
-  __shared__ double cs[32], sn[32], red[32];
-  __shared__ int pp[32], qq[32];
-  const int tid = threadIdx.x;
+__device__ __forceinline__ uint32_t jac_map(const void* p, int rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void jac_meet() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The pair at position P of the round-robin schedule: index 0 stays, 1 .. kk - 1 go round.
+struct JacPair {
+  int i1, i2;
+  __device__ __forceinline__ JacPair(int P, int kk) : i1(P), i2(kk - 1 - P) {}
+  __device__ __forceinline__ int lo() const { return min(i1, i2); }
+  __device__ __forceinline__ int hi() const { return max(i1, i2); }
+  __device__ __forceinline__ void next(int kk) {
+    if (i1 != 0) i1 = i1 == kk - 1 ? 1 : i1 + 1;
+    i2 = i2 == kk - 1 ? 1 : i2 + 1;
+  }
+};
+
+__global__ void __cluster_dims__(kJacCluster, 1, 1) __launch_bounds__(kJacThreads, 1)
+    k_symeig_jacobi(const double* A, int k, double* w, double* V, int max_sweeps, int* sweeps_out) {
+  extern __shared__ __align__(16) unsigned char jac_dyn[];
+  JacShared& S = *reinterpret_cast<JacShared*>(jac_dyn);
+  const int tid = threadIdx.x, cta = blockIdx.x;
   const int kk = (k + 1) & ~1;  // even size (a zero row/col pads odd k)
-  const int half = kk / 2;
-  for (int i = tid; i < kk * kk; i += kJacThreads) {
-    const int r = i / kk, c = i % kk;
-    a[r][c] = (r < k && c < k) ? A[r * k + c] : 0.0;
-    v[r][c] = r == c ? 1.0 : 0.0;
+  const int half = kk / 2, rounds = kk - 1;
+  if (cta != 0) {
+    const int row0 = (cta - 1) * kJacVRows;
+    if (tid < 64) {
+      const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&S.full[tid]);
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(16 * half) : "memory");
+    }
+    if (tid == 0) S.bad = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int i = tid; i < kJacVRows * 64; i += kJacThreads) S.a[i / 64][i % 64] = row0 + i / 64 == i % 64 ? 1.0 : 0.0;
   }
-  __syncthreads();
-  double big = 0.0;
-  for (int i = tid; i < kk * kk; i += kJacThreads) big = fmax(big, fabs(a[i / kk][i % kk]));
+  int e = 0, sweep = 0;
+  double tol = 0.0;
+  if (cta == 0) {
+    double big = 0.0;
+    for (int i = tid; i < kk * kk; i += kJacThreads) {
+      const int r = i / kk, c = i % kk;
+      const double x = (r < k && c < k) ? A[r * k + c] : 0.0;
+      S.a[r][c] = x;
+      big = fmax(big, fabs(x));
+    }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(FEAB_FULL_MASK, big, o));
-  if ((tid & 31) == 0) red[tid >> 5] = big;
-  __syncthreads();
-  big = red[tid & 31];
+    for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(FEAB_FULL_MASK, big, o));
+    if ((tid & 31) == 0) S.red[tid >> 5] = big;
+    __syncthreads();
+    big = (tid & 31) < kJacThreads / 32 ? S.red[tid & 31] : 0.0;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(FEAB_FULL_MASK, big, o));
-  int e = 0;
-  if (big > 0.0 && big <= 1.7976931348623157e308) frexp(big, &e);
-  double fro = 0.0;
-  for (int i = tid; i < kk * kk; i += kJacThreads) {
-    const double x = scalbn(a[i / kk][i % kk], -e);
-    a[i / kk][i % kk] = x;
-    fro += x * x;
+    for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(FEAB_FULL_MASK, big, o));
+    if (big > 0.0 && big <= 1.7976931348623157e308) frexp(big, &e);
+    double fro = 0.0;
+    for (int i = tid; i < kk * kk; i += kJacThreads) {
+      const double x = scalbn(S.a[i / kk][i % kk], -e);
+      S.a[i / kk][i % kk] = x;
+      fro += x * x;
+    }
+    fro = jac_block_sum(fro, S.red);
+    tol = 1e-30 * (fro > 0 ? fro : 1.0);
   }
-  fro = jac_block_sum(fro, red);
-  const double tol = 1e-30 * (fro > 0 ? fro : 1.0);
-  int sweep = 0;
-  for (; sweep < max_sweeps; ++sweep) {
-    double off = 0.0;
-    for (int i = tid; i < kk * kk; i += kJacThreads)
-      if (i / kk != i % kk) off += a[i / kk][i % kk] * a[i / kk][i % kk];
-    off = jac_block_sum(off, red);
-    if (off <= tol) break;
-    for (int round = 0; round < kk - 1; ++round) {
-      if (tid < half) {
-        // round-robin pairing: position 0 fixed, others rotate
-        int i1 = tid - 1 + round, i2 = kk - 2 - tid + round;
-        if (i1 >= kk - 1) i1 -= kk - 1;
-        if (i2 >= kk - 1) i2 -= kk - 1;
-        i1 = tid == 0 ? 0 : i1 + 1;
-        ++i2;
-        const int p = min(i1, i2), q = max(i1, i2);
-        const double b = 2.0 * a[p][q], d = a[q][q] - a[p][p];
-        const double h2 = fma(d, d, b * b);
-        double c = 1.0, s = 0.0;
-        if (b != 0.0 && !(h2 < 1e-290)) {
-          const double rh = rsqrt(h2);
-          const double c2 = fma(0.5 * fabs(d), rh, 0.5), rc = rsqrt(c2);   // cos^2 t >= 1/2
-          c = c2 * rc;
-          s = copysign(0.5, d) * b * rh * rc;
-        }
-        pp[tid] = p;
-        qq[tid] = q;
-        cs[tid] = c;
-        sn[tid] = s;
+  jac_meet();   // the receivers' barriers are set up
+  // thread t < half (half + 1) / 2 of CTA 0: its pair of pairs
+  int bp = 0, bq = 0;
+  const bool block = tid < half * (half + 1) / 2;
+  if (block) {
+    while ((bq + 1) * (bq + 2) / 2 <= tid) ++bq;
+    bp = tid - bq * (bq + 1) / 2;
+  }
+  bool more;
+  while (true) {
+    // CTA 0 decides; every sweep's rounds use the same barriers, phase sweep & 1
+    if (cta == 0) {
+      double off = 0.0;
+      for (int i = tid; i < kk * kk; i += kJacThreads) {
+        const int r = i / kk, c = i % kk;
+        if (r < c) off += S.a[r][c] * S.a[r][c];
       }
-      __syncthreads();
-      const int P = tid >> 5, Q = tid & 31;
-      if (P <= Q && Q < half) {
-        const int p = pp[P], q = qq[P], r = pp[Q], u = qq[Q];
-        const double cp = cs[P], sp = sn[P], cq = cs[Q], sq = sn[Q];
-        const double x00 = a[p][r], x01 = a[p][u], x10 = a[q][r], x11 = a[q][u];
-        const double y00 = fma(cp, x00, -(sp * x10)), y10 = fma(sp, x00, cp * x10);
-        const double y01 = fma(cp, x01, -(sp * x11)), y11 = fma(sp, x01, cp * x11);
-        double z00 = fma(cq, y00, -(sq * y01)), z01 = fma(sq, y00, cq * y01);
-        double z10 = fma(cq, y10, -(sq * y11)), z11 = fma(sq, y10, cq * y11);
-        if (P == Q && sp != 0.0) z01 = z10 = 0.0;
-        a[p][r] = z00;
-        a[p][u] = z01;
-        a[q][r] = z10;
-        a[q][u] = z11;
-        if (P != Q) {
-          a[r][p] = z00;
-          a[u][p] = z01;
-          a[r][q] = z10;
-          a[u][q] = z11;
-        }
+      off = 2.0 * jac_block_sum(off, S.red);
+      more = sweep < max_sweeps && !(off <= tol);
+      if (tid < kJacCluster) {
+        const uint32_t dst = jac_map(&S.go[sweep & 1], tid);
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(dst), "r"(more ? 1 : 0) : "memory");
       }
-      for (int i = tid; i < half * kk; i += kJacThreads) {
-        const int r = i / kk, row = i - r * kk;
-        const int p = pp[r], q = qq[r];
-        const double c = cs[r], s = sn[r];
-        const double vx = v[row][p], vy = v[row][q];
-        v[row][p] = fma(c, vx, -(s * vy));
-        v[row][q] = fma(s, vx, c * vy);
+    }
+    jac_meet();
+    more = S.go[sweep & 1] != 0;
+    if (!more) break;
+    if (cta == 0) {
+      JacPair own(min(tid, half - 1), kk), P(bp, kk), Q(bq, kk);
+      for (int round = 0; round < rounds; ++round) {
+        if (tid < half) {
+          const int p = own.lo(), q = own.hi();
+          const double b = 2.0 * S.a[p][q], d = S.a[q][q] - S.a[p][p];
+          const double h2 = fma(d, d, b * b);
+          double c = 1.0, s = 0.0;
+          if (b != 0.0 && !(h2 < 1e-290)) {
+            const double rh = rsqrt(h2);
+            const double c2 = fma(0.5 * fabs(d), rh, 0.5), rc = rsqrt(c2);   // cos^2 t >= 1/2
+            c = c2 * rc;
+            s = copysign(0.5, d) * b * rh * rc;
+          }
+          S.cs[tid] = c;
+          S.sn[tid] = s;
+          if (V) {
+#pragma unroll
+            for (int r = 1; r < kJacCluster; ++r) {
+              const uint32_t dst = jac_map(&S.rot[round][tid], r), bar = jac_map(&S.full[round], r);
+              asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(dst),
+                           "l"(__double_as_longlong(c)), "l"(__double_as_longlong(s)), "r"(bar)
+                           : "memory");
+            }
+          }
+        }
+        __syncthreads();
+        if (block) {
+          const int p = P.lo(), q = P.hi(), r = Q.lo(), u = Q.hi();
+          const double cp = S.cs[bp], sp = S.sn[bp], cq = S.cs[bq], sq = S.sn[bq];
+          double* e00 = &S.a[min(p, r)][max(p, r)];
+          double* e01 = &S.a[min(p, u)][max(p, u)];
+          double* e10 = &S.a[min(q, r)][max(q, r)];
+          double* e11 = &S.a[min(q, u)][max(q, u)];
+          const double x00 = *e00, x01 = *e01, x10 = *e10, x11 = *e11;
+          const double y00 = fma(cp, x00, -(sp * x10)), y10 = fma(sp, x00, cp * x10);
+          const double y01 = fma(cp, x01, -(sp * x11)), y11 = fma(sp, x01, cp * x11);
+          *e00 = fma(cq, y00, -(sq * y01));
+          *e11 = fma(sq, y10, cq * y11);
+          if (bp != bq) {
+            *e01 = fma(sq, y00, cq * y01);
+            *e10 = fma(cq, y10, -(sq * y11));
+          } else if (sp != 0.0) {
+            *e01 = 0.0;   // the rotated pair's own off-diagonal entry
+          }
+        }
+        own.next(kk);
+        P.next(kk);
+        Q.next(kk);
+        __syncthreads();
+      }
+    } else if (V) {
+      // pair tid % 32 of rows tid / 32, + 16 (the first 512 threads)
+      const int pos = tid & 31;
+      JacPair own(min(pos, half - 1), kk);
+      for (int round = 0; round < rounds; ++round) {
+        const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&S.full[round]);
+        for (int spin = 0; !*(volatile int*)&S.bad; ++spin) {
+          uint32_t ok;
+          asm volatile(
+              "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+              : "=r"(ok)
+              : "r"(bar), "r"(sweep & 1)
+              : "memory");
+          if (ok) break;
+          if (spin > (1 << 22)) *(volatile int*)&S.bad = 1;   // seconds: V becomes NaN below
+        }
+        if (tid == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(16 * half) : "memory");
+        if (tid < 512 && pos < half) {
+          const double2 cs = S.rot[round][pos];
+          const int p = own.lo(), q = own.hi();
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            double* v = S.a[(tid >> 5) + 16 * u];
+            const double vx = v[p], vy = v[q];
+            v[p] = fma(cs.x, vx, -(cs.y * vy));
+            v[q] = fma(cs.y, vx, cs.x * vy);
+          }
+        }
+        own.next(kk);
+        __syncwarp();   // a row belongs to one warp
       }
       __syncthreads();
     }
+    ++sweep;
   }
-  // descending order: an eigenvalue's place is the number of those before it
-  __shared__ int place[64];
-  if (tid < k) {
-    const double x = a[tid][tid];
-    int at = 0;
-    for (int j = 0; j < k; ++j) at += a[j][j] > x || (!(a[j][j] < x) && j < tid) ? 1 : 0;
-    place[tid] = at;
-    w[at] = scalbn(x, e);
+  if (cta == 0) {
+    // descending order: an eigenvalue's place is the number of those before it
+    if (tid < k) {
+      const double x = S.a[tid][tid];
+      int at = 0;
+      for (int j = 0; j < k; ++j) at += S.a[j][j] > x || (!(S.a[j][j] < x) && j < tid) ? 1 : 0;
+      w[at] = scalbn(x, e);
+      for (int r = 1; r < kJacCluster; ++r) {
+        const uint32_t dst = jac_map(&S.place[tid], r);
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(dst), "r"(at) : "memory");
+      }
+    }
+    if (tid == 0 && sweeps_out) *sweeps_out = sweep;
   }
-  __syncthreads();
-  if (V)
-    for (int i = tid; i < k * k; i += kJacThreads) V[(i / k) * k + place[i % k]] = v[i / k][i % k];
-  if (tid == 0 && sweeps_out) *sweeps_out = sweep;
+  jac_meet();
+  if (cta != 0 && V) {
+    const int row0 = (cta - 1) * kJacVRows;
+    for (int i = tid; i < kJacVRows * k; i += kJacThreads) {
+      const int r = i / k, c = i % k;
+      if (row0 + r < k)
+        V[(row0 + r) * k + S.place[c]] = S.bad ? __longlong_as_double(0x7ff8000000000000ll) : S.a[r][c];
+    }
+  }
 }
 
 // FP64 Gram on the CUDA cores: G = X^T X accumulated in FP64 for X (n x 64, FP32 or FP64, row
@@ -881,9 +987,9 @@ extern "C" int32_t feab_gram_fp64(const void* X, int32_t x_bytes, int64_t n, int
 extern "C" int32_t feab_symeig_jacobi(double* A, int32_t k, double* evals, double* evecs, int32_t max_sweeps,
                                       int32_t* sweeps_out, cudaStream_t s) {
   if (!A || !evals || k <= 0 || k > 64) return FEAB_BAD_ARG;
-  const size_t smem = sizeof(double) * 2 * 64 * 65;
+  const size_t smem = sizeof(JacShared);
   FEAB_CUDA(cudaFuncSetAttribute(k_symeig_jacobi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_symeig_jacobi<<<1, kJacThreads, smem, s>>>(A, k, evals, evecs, max_sweeps > 0 ? max_sweeps : 40, sweeps_out);
+  k_symeig_jacobi<<<kJacCluster, kJacThreads, smem, s>>>(A, k, evals, evecs, max_sweeps > 0 ? max_sweeps : 40, sweeps_out);
   count_launches(1);
   FEAB_CHECK_LAUNCH();
   return FEAB_OK;

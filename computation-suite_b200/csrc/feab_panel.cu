@@ -94,58 +94,85 @@ __global__ void __launch_bounds__(32 * kPReduceWarps) k_panel_gram_reduce(const 
   if (lane == 0) C[idx] = s;
 }
 
-// Z = Y V, Y of FP64 or FP32 values: a CTA stages 128 rows of Y (padded, so that a warp's 32 rows read
-// one column without bank conflicts) and V in shared memory; thread (row, half) forms eight columns
-// of its row at a time, the sums over j in order.  What bounds it: reading Y once (33 us at 418,176 x
-// 64 FP64) and, close behind, the shared-memory reads (V's values are broadcasts, two per read).
-// Measured there with m = 10: 303 us when every output read its row of Y from L1 by itself.
-constexpr int kSmallRows = 128;
-constexpr int kSmallLd = kP + 1;
-constexpr size_t kSmallSmem = sizeof(double) * (kSmallRows * kSmallLd + kP * kP);
+// Z = Y V, Y of FP64 or FP32 values, on the FP64 tensor path (mma.sync m8n8k4): a warp forms eight rows and
+// up to 16 columns at a time, with V's fragments in registers for the whole launch.  Lane l reads four
+// adjacent values of row l / 4 of Y for each 16 columns of it, from k = 16 kb + 4 (l % 4), and step s of
+// that block multiplies the four lanes' s-th values, k = 16 kb + 4 (l % 4) + s, so a row's 16 values
+// are one or two sectors and nothing passes through shared memory.  More than 16 columns are
+// more column groups (gridDim.y), each of which reads Y.  What bounds it: reading Y once (16 us
+// at 418,176 x 64 FP32) and the tensor rate (23 us).  Measured there with m = 10: 303 us when every
+// output read its row of Y from L1 by itself, 152 us with rows and V staged in shared memory.
+constexpr int kSmallSteps = kP / 4;
 
-template <typename T>
+__device__ __forceinline__ void panel_dmma(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+
+// The lane's 16 values of a row: four adjacent ones of each 16 columns; zeros past column k and for no row.
+// VEC: 64 columns, rows at multiples of 16 bytes.
+template <typename T, bool VEC>
+__device__ __forceinline__ void panel_row(const T* __restrict__ row, bool valid, int k, int t, T (&y)[16]) {
+#pragma unroll
+  for (int kb = 0; kb < 4; ++kb) {
+    const int c = 16 * kb + 4 * t;
+    if constexpr (VEC && sizeof(T) == 4) {
+      const float4 v = valid ? __ldcs(reinterpret_cast<const float4*>(row + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      y[4 * kb] = v.x;
+      y[4 * kb + 1] = v.y;
+      y[4 * kb + 2] = v.z;
+      y[4 * kb + 3] = v.w;
+    } else if constexpr (VEC) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const double2 v = valid ? __ldcs(reinterpret_cast<const double2*>(row + c) + h) : make_double2(0.0, 0.0);
+        y[4 * kb + 2 * h] = v.x;
+        y[4 * kb + 2 * h + 1] = v.y;
+      }
+    } else {
+#pragma unroll
+      for (int s = 0; s < 4; ++s) y[4 * kb + s] = valid && c + s < k ? __ldcs(row + c + s) : T(0);
+    }
+  }
+}
+
+template <typename T, bool VEC>
 __global__ void __launch_bounds__(kPThreads) k_panel_small(const T* __restrict__ Y, int ldy, int64_t n, int k,
                                                           const double* __restrict__ V, int m, double* __restrict__ Z,
                                                           int ldz) {
-  extern __shared__ __align__(16) double small_sm[];
-  double* vs = small_sm;                  // vs[j * mp + c], mp = m rounded up to 8, zeros past m
-  double* ys = small_sm + kP * kP;        // ys[r * kSmallLd + j]
-  const int tid = threadIdx.x, mp = (m + 7) & ~7;
-  for (int e = tid; e < k * mp; e += kPThreads) {
-    const int j = e / mp, c = e - j * mp;
-    vs[e] = c < m ? V[j * m + c] : 0.0;
-  }
-  const int r = tid & (kSmallRows - 1), h = tid / kSmallRows;
-  for (int64_t r0 = (int64_t)blockIdx.x * kSmallRows; r0 < n; r0 += (int64_t)gridDim.x * kSmallRows) {
-    __syncthreads();
-    const int rows = (int)min((int64_t)kSmallRows, n - r0);
-    for (int e = tid; e < kSmallRows * kP; e += kPThreads) {
-      const int i = e / kP, j = e % kP;
-      if (i < rows && j < k) ys[i * kSmallLd + j] = (double)__ldcs(Y + (r0 + i) * (int64_t)ldy + j);
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, c0 = 16 * blockIdx.y;
+  double b[2][kSmallSteps];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int q = 0; q < kSmallSteps; ++q) {
+      const int r = 16 * (q >> 2) + 4 * t + (q & 3), c = c0 + 8 * j + g;
+      b[j][q] = r < k && c < m ? V[r * m + c] : 0.0;
     }
-    __syncthreads();
-    if (r < rows) {
-      for (int c0 = 8 * h; c0 < m; c0 += 16) {
-        double s[8];
+  const int64_t step = 8 * ((int64_t)gridDim.x * (kPThreads / 32));
+  int64_t r = 8 * ((int64_t)blockIdx.x * (kPThreads / 32) + (threadIdx.x >> 5)) + g;
+  T y[16];
+  panel_row<T, VEC>(Y + r * ldy, r < n, k, t, y);
+  for (; r - g < n; r += step) {
+    T next[16];
+    panel_row<T, VEC>(Y + (r + step) * ldy, r + step < n, k, t, next);
+    double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
 #pragma unroll
-        for (int c = 0; c < 8; ++c) s[c] = 0.0;
-#pragma unroll 4
-        for (int j = 0; j < k; ++j) {
-          const double y = ys[r * kSmallLd + j];
-          const double2* vj = reinterpret_cast<const double2*>(vs + j * mp + c0);
+    for (int q = 0; q < kSmallSteps; ++q) {
+      panel_dmma(acc[0], (double)y[q], b[0][q]);
+      panel_dmma(acc[1], (double)y[q], b[1][q]);
+    }
+    if (r < n) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const double2 vv = vj[c];
-            s[2 * c] = fma(y, vv.x, s[2 * c]);
-            s[2 * c + 1] = fma(y, vv.y, s[2 * c + 1]);
-          }
-        }
-        double* z = Z + (r0 + r) * (int64_t)ldz + c0;
-#pragma unroll
-        for (int c = 0; c < 8; ++c)
-          if (c0 + c < m) z[c] = s[c];
+      for (int j = 0; j < 2; ++j) {
+        const int c = c0 + 8 * j + 2 * t;
+        if (c < m) Z[r * ldz + c] = acc[j][0];
+        if (c + 1 < m) Z[r * ldz + c + 1] = acc[j][1];
       }
     }
+#pragma unroll
+    for (int q = 0; q < 16; ++q) y[q] = next[q];
   }
 }
 
@@ -155,10 +182,11 @@ int32_t launch_panel_small(const T* Y, int32_t ldy, int64_t n, int32_t k, const 
   if (!Y || !V || !Z || n <= 0 || k < 1 || k > kP || m < 1 || m > kP || ldy < k || ldz < m ||
       static_cast<const void*>(Y) == Z)
     return FEAB_BAD_ARG;
-  FEAB_CUDA(cudaFuncSetAttribute(k_panel_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem));
-  const int64_t tiles = (n + kSmallRows - 1) / kSmallRows;
-  const int grid = (int)std::min<int64_t>(tiles, 2 * (int64_t)sm_count());
-  k_panel_small<T><<<grid, kPThreads, kSmallSmem, s>>>(Y, ldy, n, k, V, m, Z, ldz);
+  const int64_t groups = (n + 7) / 8, blocks = (groups + kPThreads / 32 - 1) / (kPThreads / 32);
+  const dim3 grid((unsigned)std::min<int64_t>(blocks, 4 * (int64_t)sm_count()), (m + 15) / 16);
+  const bool vec = k == kP && (reinterpret_cast<uintptr_t>(Y) & 15) == 0 && (ldy * sizeof(T)) % 16 == 0;
+  if (vec) k_panel_small<T, true><<<grid, kPThreads, 0, s>>>(Y, ldy, n, k, V, m, Z, ldz);
+  else k_panel_small<T, false><<<grid, kPThreads, 0, s>>>(Y, ldy, n, k, V, m, Z, ldz);
   count_launches(1);
   FEAB_CHECK_LAUNCH();
   return FEAB_OK;
