@@ -6,12 +6,15 @@
 //   elem_e = sum_q |detJ| w val_q / sum_q |detJ| w,
 // and optionally the von Mises stress of both (recovery.py:386-420).
 //
-// Two kernels.  k_recover_elements: 8 threads per element, thread q first evaluates Gauss point q
-// (val_q, |detJ| w) into shared memory, then thread c projects onto corner c, writing the
-// element's corner record (6 numerators + denominator, padded to 64 bytes) to scratch, and
-// threads 0-5 form the element average.  k_recover_nodes: one thread per node adds the corner
-// records of its elements (16-byte loads) in ascending element order, the order of the
-// reference's np.add.at over the connectivity, so the result is deterministic with no atomics.
+// Two kernels.  k_recover_elements: 8 lanes per element, lane q holding the corner with the signs of
+// Gauss point q.  The trilinear shape functions are products of one function per direction, so the
+// derivatives of the coordinates and displacements at the Gauss points are three exchanges between
+// the two lanes that differ in one sign (a difference along one direction, interpolations along the
+// others), and the projection sum_q N_c(q) w_q val_q is three more with the same two weights.
+// Everything stays in registers.  The element's corner records (6 numerators + denominator, padded
+// to 64 bytes) go to scratch.  k_recover_nodes: one thread per node adds the corner records of its
+// elements (16-byte loads) in ascending element order, the order of the reference's np.add.at over
+// the connectivity, so the result is deterministic with no atomics.
 #include "feab_hex8.cuh"
 
 namespace feab {
@@ -21,12 +24,30 @@ constexpr int kRecElems = 16;                 // elements per 128-thread block
 constexpr int kRecThreads = kRecElems * 8;
 constexpr int kRecord = 8;                    // doubles per (element, corner): 6 numerators, denominator, pad
 
+// The two values of the linear shape functions (1 -+ xi) / 2 at the Gauss abscissas: the nearer corner's
+// and the farther one's.
+constexpr double kNear = 0.5 * (1.0 + FEAB_GAUSS2), kFar = 0.5 * (1.0 - FEAB_GAUSS2);
 
-// Trilinear shape function of corner c at Gauss point q (elements/solids.py:133-142).
-__device__ __forceinline__ double shape_at(int c, int q) {
-  double xi, eta, zeta;
-  gauss_point(q, xi, eta, zeta);
-  return 0.125 * (1.0 + xi * xi_sign(c)) * (1.0 + eta * eta_sign(c)) * (1.0 + zeta * zeta_sign(c));
+// Corner with the signs of Gauss point q (xi: bit 2, eta: bit 1, zeta: bit 0).
+__device__ __forceinline__ int corner_of(int q) {
+  return ((q & 1) << 2) | ((q & 2) ? ((q & 4) ? 2 : 3) : ((q & 4) ? 1 : 0));
+}
+
+// The value of the lane whose sign along the direction of `bit` is the other one.
+__device__ __forceinline__ double other(double v, int bit) { return __shfl_xor_sync(FEAB_FULL_MASK, v, bit); }
+__device__ __forceinline__ double interpolate(double v, double o) { return fma(kNear, v, kFar * o); }
+
+// Natural derivatives, at the lane's Gauss point, of the trilinear field with corner values v.  h_*: 1/2 times the
+// lane's sign along each direction.
+__device__ __forceinline__ void natural_gradient(double v, double h_xi, double h_eta, double h_zeta, double (&d)[3]) {
+  const double ox = other(v, 4);
+  const double dx = h_xi * (v - ox), ix = interpolate(v, ox);
+  const double odx = other(dx, 2), oix = other(ix, 2);
+  const double dxi = interpolate(dx, odx), dy = h_eta * (ix - oix), iy = interpolate(ix, oix);
+  const double ody = other(dy, 1), oiy = other(iy, 1);
+  d[0] = interpolate(dxi, other(dxi, 1));
+  d[1] = interpolate(dy, ody);
+  d[2] = h_zeta * (iy - oiy);
 }
 
 __device__ __forceinline__ double mises(const double (&s)[6]) {
@@ -34,105 +55,82 @@ __device__ __forceinline__ double mises(const double (&s)[6]) {
   return sqrt(0.5 * (a * a + b * b + c * c) + 3.0 * (s[3] * s[3] + s[4] * s[4] + s[5] * s[5]));
 }
 
+// What bounds it: FP64 arithmetic (about 230 operations per Gauss point, with shape function tables and every
+// derivative summed over the 8 corners it was some 450), the exchanges (114 per warp) and the 64-byte
+// records.  rec may be NULL (element values only).
 __global__ void __launch_bounds__(kRecThreads) k_recover_elements(const double* __restrict__ coords,
                                                                   const int32_t* __restrict__ conn, int64_t n_elem,
                                                                   Mat6 D, int use_d, const double* __restrict__ u,
                                                                   double* __restrict__ rec, double* __restrict__ elem,
                                                                   double* __restrict__ elem_vm,
                                                                   feab_device_status* st) {
-  __shared__ double sX[kRecElems][8][3];
-  __shared__ double sU[kRecElems][8][3];
-  __shared__ double sV[kRecElems][8][7];       // per Gauss point: val (6), |detJ| w
-  const int le = threadIdx.x >> 3, t = threadIdx.x & 7;
-  const int64_t e = (int64_t)blockIdx.x * kRecElems + le;
-  const bool live = e < n_elem;
-  if (live) {
-    const int64_t n = conn[e * 8 + t];
+  const int q = threadIdx.x & 7;
+  const int64_t e0 = (int64_t)blockIdx.x * kRecElems + (threadIdx.x >> 3);
+  const bool live = e0 < n_elem;
+  const int64_t e = live ? e0 : n_elem - 1;    // spare lanes repeat the last element and write nothing
+  const int c = corner_of(q);
+  const int64_t node = conn[e * 8 + c];
+  const double h_xi = (q & 4) ? 0.5 : -0.5, h_eta = (q & 2) ? 0.5 : -0.5, h_zeta = (q & 1) ? 0.5 : -0.5;
+  double J[3][3], G[3][3], inv[3][3];          // J[i][j] = d X_j / d xi_i, G[i][j] = d u_j / d xi_i
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      sX[le][t][j] = coords[n * 3 + j];
-      sU[le][t][j] = u[n * 3 + j];
-    }
+  for (int j = 0; j < 3; ++j) {
+    double d[3];
+    natural_gradient(coords[node * 3 + j], h_xi, h_eta, h_zeta, d);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) J[i][j] = d[i];
+    natural_gradient(u[node * 3 + j], h_xi, h_eta, h_zeta, d);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) G[i][j] = d[i];
   }
-  __syncthreads();
-  if (live) {
-    // thread t = Gauss point q
-    double X[8][3];
+  const double det = invert3(J, inv);
+  if (live && !(fabs(det) >= 1e-300)) set_status(reinterpret_cast<int*>(st), FEAB_DEGENERATE_ELEMENT, e);
+  // H[i][j] = d u_j / d x_i
+  double H[3][3];
 #pragma unroll
-    for (int k = 0; k < 8; ++k)
+  for (int i = 0; i < 3; ++i)
 #pragma unroll
-      for (int j = 0; j < 3; ++j) X[k][j] = sX[le][k][j];
-    double xi, eta, zeta, inv[3][3];
-    gauss_point(t, xi, eta, zeta);
-    const double det = jacobian_inverse(X, xi, eta, zeta, inv);
-    if (!(fabs(det) >= 1e-300)) set_status(reinterpret_cast<int*>(st), FEAB_DEGENERATE_ELEMENT, e);
-    double eps[6] = {0, 0, 0, 0, 0, 0};
+    for (int j = 0; j < 3; ++j) H[i][j] = fma(inv[i][0], G[0][j], fma(inv[i][1], G[1][j], inv[i][2] * G[2][j]));
+  // rows xx, yy, zz, xy, yz, xz with engineering shear (recovery.py:169-193)
+  const double eps[6] = {H[0][0], H[1][1], H[2][2], H[1][0] + H[0][1], H[2][1] + H[1][2], H[2][0] + H[0][2]};
+  const double w = fabs(det);                  // Gauss weights are 1
+  double v[7];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      double a, b, c;
-      dshape(k, xi, eta, zeta, a, b, c);
-      const double gx = inv[0][0] * a + inv[0][1] * b + inv[0][2] * c;
-      const double gy = inv[1][0] * a + inv[1][1] * b + inv[1][2] * c;
-      const double gz = inv[2][0] * a + inv[2][1] * b + inv[2][2] * c;
-      const double ux = sU[le][k][0], uy = sU[le][k][1], uz = sU[le][k][2];
-      // B rows xx, yy, zz, xy, yz, xz with engineering shear (recovery.py:169-193)
-      eps[0] += gx * ux;
-      eps[1] += gy * uy;
-      eps[2] += gz * uz;
-      eps[3] += gy * ux + gx * uy;
-      eps[4] += gz * uy + gy * uz;
-      eps[5] += gz * ux + gx * uz;
+  for (int s = 0; s < 6; ++s) {
+    double x = eps[s];
+    if (use_d) {
+      x = 0.0;
+#pragma unroll
+      for (int j = 0; j < 6; ++j) x += D.d[s * 6 + j] * eps[j];
     }
-#pragma unroll
-    for (int s = 0; s < 6; ++s) {
-      double v = eps[s];
-      if (use_d) {
-        v = 0.0;
-#pragma unroll
-        for (int j = 0; j < 6; ++j) v += D.d[s * 6 + j] * eps[j];
-      }
-      sV[le][t][s] = v;
-    }
-    sV[le][t][6] = fabs(det);  // Gauss weights are 1
+    v[s] = w * x;
   }
-  __syncthreads();
-  if (live) {
-    // thread t = corner c: sum over the Gauss points in rule order
-    double num[6] = {0, 0, 0, 0, 0, 0}, den = 0.0;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const double wn = sV[le][q][6] * shape_at(t, q);
-#pragma unroll
-      for (int s = 0; s < 6; ++s) num[s] += wn * sV[le][q][s];
-      den += wn;
-    }
-    double2* r = reinterpret_cast<double2*>(rec + (e * 8 + t) * kRecord);
-    r[0] = make_double2(num[0], num[1]);
-    r[1] = make_double2(num[2], num[3]);
-    r[2] = make_double2(num[4], num[5]);
-    r[3] = make_double2(den, 0.0);
-  }
+  v[6] = w;
   if (elem || elem_vm) {
-    // thread t < 6: component t of the element average (every lane takes part in the shuffles)
-    double avg = 0.0;
-    if (live) {
-      double acc = 0.0, vol = 0.0;
-      const int s = t < 6 ? t : 0;
+    double m[7];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        acc += sV[le][q][6] * sV[le][q][s];
-        vol += sV[le][q][6];
-      }
-      avg = acc / vol;
-      if (elem && t < 6) elem[e * 6 + t] = avg;
+    for (int s = 0; s < 7; ++s) {
+      m[s] = v[s];
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) m[s] += __shfl_xor_sync(FEAB_FULL_MASK, m[s], o);
     }
-    if (elem_vm) {
-      // the 8 threads of an element are 8 consecutive lanes of one warp
-      double s6[6];
-      const int base = threadIdx.x & 31 & ~7;
+    double avg[6];
 #pragma unroll
-      for (int j = 0; j < 6; ++j) s6[j] = __shfl_sync(FEAB_FULL_MASK, avg, base + j);
-      if (live && t == 0) elem_vm[e] = mises(s6);
+    for (int s = 0; s < 6; ++s) avg[s] = m[s] / m[6];
+    if (live && elem && q < 6)
+      elem[e * 6 + q] = q == 0 ? avg[0] : q == 1 ? avg[1] : q == 2 ? avg[2] : q == 3 ? avg[3] : q == 4 ? avg[4] : avg[5];
+    if (live && elem_vm && q == 0) elem_vm[e] = mises(avg);
+  }
+  if (rec) {
+#pragma unroll
+    for (int s = 0; s < 7; ++s)
+#pragma unroll
+      for (int bit = 4; bit > 0; bit >>= 1) v[s] = interpolate(v[s], other(v[s], bit));
+    if (live) {
+      double2* r = reinterpret_cast<double2*>(rec + (e * 8 + c) * kRecord);
+      r[0] = make_double2(v[0], v[1]);
+      r[1] = make_double2(v[2], v[3]);
+      r[2] = make_double2(v[4], v[5]);
+      r[3] = make_double2(v[6], 0.0);
     }
   }
 }
@@ -198,8 +196,8 @@ extern "C" int32_t feab_hex8_recover(const double* coords, const int32_t* conn, 
   for (int i = 0; i < 36; ++i) D.d[i] = D_host ? D_host[i] : 0.0;
   double* rec = static_cast<double*>(scratch);
   const int64_t grid = (n_elem + kRecElems - 1) / kRecElems;
-  k_recover_elements<<<(unsigned)grid, kRecThreads, 0, s>>>(coords, conn, n_elem, D, D_host ? 1 : 0, u, rec, elem,
-                                                             elem_vm, status);
+  k_recover_elements<<<(unsigned)grid, kRecThreads, 0, s>>>(coords, conn, n_elem, D, D_host ? 1 : 0, u,
+                                                             nodal || nodal_vm ? rec : nullptr, elem, elem_vm, status);
   if (nodal || nodal_vm) {
     const int threads = 256;
     k_recover_nodes<<<(n_nodes + threads - 1) / threads, threads, 0, s>>>(conn, inc_ptr, inc_elem, n_nodes, rec, nodal,
