@@ -114,6 +114,17 @@ __device__ __forceinline__ bool last_of_problem(uint32_t* ticket, int n_items_p,
 #endif
 constexpr int kBRun = FEAB_BLOCK_BRUN;
 
+// Columns of problem p in use, 1 .. K.  The panel is as wide as the widest problem needs, rounded up to a
+// power of two; nothing reads what a step would write to the columns behind a problem's own.
+template <int K>
+__device__ __forceinline__ int live_columns(const BArgs& A, int p) {
+  return min(max(__ldg(A.prob_cols + p), 1), K);
+}
+
+// A problem that uses at most half of the panel's columns has its vector passes (and from 16 columns on,
+// where stated, its SpMM) on that half.
+constexpr int narrow_panel(int K) { return K >= 16 ? K / 2 : K; }
+
 // Block-wide per-column sums: thread t contributes v to column t % K (blockDim multiple of K).
 template <int K>
 __device__ __forceinline__ void block_col_sums(double v, double* sm) {
@@ -852,14 +863,20 @@ __global__ void __launch_bounds__(kThreads, TILES ? FEAB_BLOCK_MINB : FEAB_BLOCK
 // 16-byte load, one for each of two tiles (an even and an odd one of every 16 columns); C 8 x 8, lane
 // l holds row l / 4, so with both tiles four adjacent panel columns.
 //
-// What bounds it: the FP64 tensor rate (37 TFLOP/s) on the pair's 8 x 108 operand, 56 % of it nonzeros.
-// In the group and tile paths every value reached the lanes as its own shared-memory broadcast, and
-// the L1 data path set the pace; here a value is one lane's register.
+// What bounds it: the latency of the gathers at the 16 warps per SM that the sums' registers leave (at 418,176 rows
+// and 64 columns the operand's tensor work is 27 % of the kernel's time, its HBM bytes 10 %).  In the group and tile paths
+// every value reached the lanes as its own shared-memory broadcast, and the L1 data path set the pace;
+// here a value is one lane's register.  A whole FP64 block step at 418,176 rows, in us, with row groups
+// and with pairs: 8 columns 196 and 144, 16: 312 and 264, 32: 482 and 449, 64: 838 and 798.
+//
+// Columns of the records applied before the next gathers, and blocks per SM: by measurement (16 columns,
+// 8 and 2: 264 us, 4 and 4: 266 but 60 more with the residual replacements' spills; 64 columns, 1 and 2:
+// 795, 2 and 2: 907; 8 columns, 4 and 4: 146, 8 and 2: 168).
 #ifndef FEAB_PAIR_UNROLL
-#define FEAB_PAIR_UNROLL(K) ((K) == 64 ? 2 : ((K) == 32 ? 4 : 8))
+#define FEAB_PAIR_UNROLL(K) ((K) == 64 ? 1 : ((K) == 16 ? 8 : 4))
 #endif
 #ifndef FEAB_PAIR_MINB
-#define FEAB_PAIR_MINB(K) 2
+#define FEAB_PAIR_MINB(K) ((K) == 8 ? 4 : 2)
 #endif
 
 __device__ __forceinline__ void dmma884(double (&d)[2], double a, double b) {
@@ -905,10 +922,10 @@ __device__ __forceinline__ bool pair_wait(PairStage& st, int buf, unsigned parit
 }
 
 // acc += the staged records times the panel rows of src.
-template <int K>
+template <int K, int KC>
 __device__ __forceinline__ void pair_apply(const PairRecord* __restrict__ rec, int steps, int lane,
-                                           const double* __restrict__ src, double (&acc)[K / 8][2]) {
-  constexpr int U = FEAB_PAIR_UNROLL(K), NL = pair_loads(K);
+                                           const double* __restrict__ src, double (&acc)[KC / 8][2]) {
+  constexpr int U = FEAB_PAIR_UNROLL(KC), NL = pair_loads(KC);
   const int t = lane & 3, n = lane >> 2;
   for (int s = 0; s < steps; s += U) {
     double2 b[U][NL];
@@ -916,10 +933,10 @@ __device__ __forceinline__ void pair_apply(const PairRecord* __restrict__ rec, i
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (s + u < steps) {   // the same for the whole warp
-        const double* row = src + (int64_t)rec[s + u].col[K >= 16 ? lane >> 3 : t] * K;
+        const double* row = src + (int64_t)rec[s + u].col[KC >= 16 ? lane >> 3 : t] * K;
 #pragma unroll
         for (int j = 0; j < NL; ++j) {
-          if (K >= 16) b[u][j] = __ldg(reinterpret_cast<const double2*>(row + 16 * j) + (lane & 7));
+          if (KC >= 16) b[u][j] = __ldg(reinterpret_cast<const double2*>(row + 16 * j) + (lane & 7));
           else b[u][j] = make_double2(__ldg(row + n), 0.0);
         }
         a[u] = lane < 24 ? rec[s + u].val[lane] : 0.0;
@@ -930,7 +947,7 @@ __device__ __forceinline__ void pair_apply(const PairRecord* __restrict__ rec, i
       if (s + u < steps) {
 #pragma unroll
         for (int j = 0; j < NL; ++j) {
-          if constexpr (K >= 16) {
+          if constexpr (KC >= 16) {
             // eight lanes read one 128-byte line; the fragment wants row l % 4, columns 2 (l / 4) + {0, 1}
             const double x = __shfl_sync(FEAB_FULL_MASK, b[u][j].x, 8 * t + n);
             const double y = __shfl_sync(FEAB_FULL_MASK, b[u][j].y, 8 * t + n);
@@ -945,12 +962,122 @@ __device__ __forceinline__ void pair_apply(const PairRecord* __restrict__ rec, i
   }
 }
 
+// Item it's rows of the first KC panel columns, and the warp's column sums in sums.
+template <int K, int KC>
+__device__ __forceinline__ void pair_item(const BArgs& A, int it, int p, bool reliable, PairStage& st, int& buf,
+                                          unsigned (&parity)[2], double* sums) {
+  constexpr int NL = pair_loads(KC), W = KC >= 16 ? 4 : 2;   // adjacent columns of a lane, NL times
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, t = lane & 3, r = lane >> 2;
+  const double* __restrict__ src = reliable ? A.X : A.P0;
+  double* __restrict__ dst = reliable ? A.R : A.AP;
+  bool arrived = true;
+  double part[NL][W];
+#pragma unroll
+  for (int j = 0; j < NL; ++j)
+#pragma unroll
+    for (int e = 0; e < W; ++e) part[j][e] = 0.0;
+  int t0, t1;
+  item_tiles(A, it, t0, t1);
+  // the warp's pairs 2 t0 + w, + 8, ..., 32 at a time: lane i holds the i-th one's records and rows
+  for (int q0 = 2 * t0 + w; q0 < 2 * t1; q0 += 32 * kWarps) {
+    const int q = q0 + lane * kWarps;
+    int first = 0, last = 0, row0 = 0, rows = 0;
+    if (q < 2 * t1) {
+      const int g = A.t_g0[q >> 1] + 2 * (q & 1), gn = min(2, A.t_g0[(q >> 1) + 1] - g);
+      if (gn > 0) {
+        first = __ldg(A.pairs.off + q);
+        last = __ldg(A.pairs.off + q + 1);
+        row0 = A.group_ptr[g];
+        rows = A.group_ptr[g + gn] - row0;
+      }
+    }
+    const int count = min(32, (2 * t1 - q0 + kWarps - 1) / kWarps);
+    int pi = 0, s = 0, e = 0;                              // the next chunk to fetch: pair pi, from record s
+    auto open = [&] {                                      // the first pair from pi on that has records
+      for (; pi < count; ++pi) {
+        s = __shfl_sync(FEAB_FULL_MASK, first, pi);
+        e = __shfl_sync(FEAB_FULL_MASK, last, pi);
+        if (e > s) return;
+      }
+    };
+    auto fetch = [&](int b) {                              // issues the chunk, moves on; its steps (0: none left)
+      if (pi >= count) return 0;
+      const int n = min(kPairChunk, e - s);
+      if (lane == 0) pair_copy(st, b, A.pairs.rec + s, n);
+      s += n;
+      if (s >= e) {
+        ++pi;
+        open();
+      }
+      return n;
+    };
+    open();
+    double acc[KC / 8][2];
+#pragma unroll
+    for (int j = 0; j < KC / 8; ++j) acc[j][0] = acc[j][1] = 0.0;
+    int cur = pi, steps = fetch(buf);
+    while (steps > 0) {
+      const int nxt = pi, more = fetch(buf ^ 1);           // pair and steps of the chunk behind this one
+      arrived = pair_wait(st, buf, parity[buf]) && arrived;
+      parity[buf] ^= 1u;
+      pair_apply<K, KC>(st.rec[buf], steps, lane, src, acc);
+      __syncwarp();                                        // every lane is done with the chunk
+      if (more == 0 || nxt != cur) {                       // the pair's last chunk: its rows
+        const int r0 = __shfl_sync(FEAB_FULL_MASK, row0, cur), m = __shfl_sync(FEAB_FULL_MASK, rows, cur);
+        if (r < m) {
+          const int64_t base = (int64_t)(r0 + r) * K + W * t;
+#pragma unroll
+          for (int j = 0; j < NL; ++j) {
+            double v[W];
+            if constexpr (KC >= 16) {
+              v[0] = acc[2 * j][0];
+              v[1] = acc[2 * j + 1][0];
+              v[2] = acc[2 * j][1];
+              v[3] = acc[2 * j + 1][1];
+            } else {
+              v[0] = acc[j][0];
+              v[1] = acc[j][1];
+            }
+#pragma unroll
+            for (int e2 = 0; e2 < W; e2 += 2) {
+              const int64_t idx = base + 16 * j + e2;
+              // AP and p.Ap; a reliable step R = B - K X and r.r
+              const double2 in = reliable ? make_double2(A.B[idx], A.B[idx + 1])   // the caller's: 8-byte aligned
+                                          : *reinterpret_cast<const double2*>(A.P0 + idx);
+              const double y0 = reliable ? in.x - v[e2] : v[e2], y1 = reliable ? in.y - v[e2 + 1] : v[e2 + 1];
+              *reinterpret_cast<double2*>(dst + idx) = make_double2(y0, y1);
+              part[j][e2] += (reliable ? y0 : in.x) * y0;
+              part[j][e2 + 1] += (reliable ? y1 : in.y) * y1;
+            }
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < KC / 8; ++j) acc[j][0] = acc[j][1] = 0.0;
+      }
+      cur = nxt;
+      steps = more;
+      buf ^= 1;
+    }
+  }
+  if (!arrived && lane == 0) atomicCAS(&A.ps[p].status, FEAB_OK, FEAB_CUDA_ERROR);
+  // the rows' lanes of each column
+#pragma unroll
+  for (int j = 0; j < NL; ++j)
+#pragma unroll
+    for (int e = 0; e < W; ++e) {
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) part[j][e] += __shfl_xor_sync(FEAB_FULL_MASK, part[j][e], o);
+      if (r == 0) sums[16 * j + W * t + e] = part[j][e];
+    }
+  if (KC < K)
+    for (int c = KC + lane; c < K; c += 32) sums[c] = 0.0;
+}
+
 template <int K, bool MIXED>
 __global__ void __launch_bounds__(kThreads, FEAB_PAIR_MINB(K)) k_bstep_a_pairs(BArgs A) {
-  constexpr int NL = pair_loads(K), W = K >= 16 ? 4 : 2;   // adjacent columns of a lane, NL times
   __shared__ double sm[kWarps][K];
   extern __shared__ __align__(16) unsigned char dyn_stage[];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, t = lane & 3, r = lane >> 2;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   PairStage& st = reinterpret_cast<PairStage*>(dyn_stage)[w];
   if (lane < 2)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(&st.full[lane])) : "memory");
@@ -963,112 +1090,41 @@ __global__ void __launch_bounds__(kThreads, FEAB_PAIR_MINB(K)) k_bstep_a_pairs(B
     const ProbState P = A.ps[p];
     if (P.done) continue;
     const bool reliable = MIXED && P.mode == kModeReliable;
-    const double* __restrict__ src = reliable ? A.X : A.P0;
-    bool arrived = true;
-    double part[NL][W];
-#pragma unroll
-    for (int j = 0; j < NL; ++j)
-#pragma unroll
-      for (int e = 0; e < W; ++e) part[j][e] = 0.0;
-    int t0, t1;
-    item_tiles(A, it, t0, t1);
-    // the warp's pairs 2 t0 + w, + 8, ..., 32 at a time: lane i holds the i-th one's records and rows
-    for (int q0 = 2 * t0 + w; q0 < 2 * t1; q0 += 32 * kWarps) {
-      const int q = q0 + lane * kWarps;
-      int first = 0, last = 0, row0 = 0, rows = 0;
-      if (q < 2 * t1) {
-        const int g = A.t_g0[q >> 1] + 2 * (q & 1), gn = min(2, A.t_g0[(q >> 1) + 1] - g);
-        if (gn > 0) {
-          first = __ldg(A.pairs.off + q);
-          last = __ldg(A.pairs.off + q + 1);
-          row0 = A.group_ptr[g];
-          rows = A.group_ptr[g + gn] - row0;
-        }
-      }
-      const int count = min(32, (2 * t1 - q0 + kWarps - 1) / kWarps);
-      int pi = 0, s = 0, e = 0;                              // the next chunk to fetch: pair pi, from record s
-      auto open = [&] {                                      // the first pair from pi on that has records
-        for (; pi < count; ++pi) {
-          s = __shfl_sync(FEAB_FULL_MASK, first, pi);
-          e = __shfl_sync(FEAB_FULL_MASK, last, pi);
-          if (e > s) return;
-        }
-      };
-      auto fetch = [&](int b) {                              // issues the chunk, moves on; its steps (0: none left)
-        if (pi >= count) return 0;
-        const int n = min(kPairChunk, e - s);
-        if (lane == 0) pair_copy(st, b, A.pairs.rec + s, n);
-        s += n;
-        if (s >= e) {
-          ++pi;
-          open();
-        }
-        return n;
-      };
-      open();
-      double acc[K / 8][2];
-#pragma unroll
-      for (int j = 0; j < K / 8; ++j) acc[j][0] = acc[j][1] = 0.0;
-      int cur = pi, steps = fetch(buf);
-      while (steps > 0) {
-        const int nxt = pi, more = fetch(buf ^ 1);           // pair and steps of the chunk behind this one
-        arrived = pair_wait(st, buf, parity[buf]) && arrived;
-        parity[buf] ^= 1u;
-        pair_apply<K>(st.rec[buf], steps, lane, src, acc);
-        __syncwarp();                                        // every lane is done with the chunk
-        if (more == 0 || nxt != cur) {                       // the pair's last chunk: its rows
-          const int r0 = __shfl_sync(FEAB_FULL_MASK, row0, cur), m = __shfl_sync(FEAB_FULL_MASK, rows, cur);
-          if (r < m) {
-            const int64_t base = (int64_t)(r0 + r) * K + W * t;
-#pragma unroll
-            for (int j = 0; j < NL; ++j) {
-              double v[W];
-              if constexpr (K >= 16) {
-                v[0] = acc[2 * j][0];
-                v[1] = acc[2 * j + 1][0];
-                v[2] = acc[2 * j][1];
-                v[3] = acc[2 * j + 1][1];
-              } else {
-                v[0] = acc[j][0];
-                v[1] = acc[j][1];
-              }
-#pragma unroll
-              for (int e2 = 0; e2 < W; e2 += 2) {
-                const int64_t idx = base + 16 * j + e2;
-                if (reliable) {   // R = B - K X and r.r
-                  const double b0 = A.B[idx] - v[e2], b1 = A.B[idx + 1] - v[e2 + 1];
-                  *reinterpret_cast<double2*>(A.R + idx) = make_double2(b0, b1);
-                  part[j][e2] += b0 * b0;
-                  part[j][e2 + 1] += b1 * b1;
-                } else {          // AP and p.Ap
-                  const double2 pv = *reinterpret_cast<const double2*>(A.P0 + idx);
-                  *reinterpret_cast<double2*>(A.AP + idx) = make_double2(v[e2], v[e2 + 1]);
-                  part[j][e2] += pv.x * v[e2];
-                  part[j][e2 + 1] += pv.y * v[e2 + 1];
-                }
-              }
-            }
-          }
-#pragma unroll
-          for (int j = 0; j < K / 8; ++j) acc[j][0] = acc[j][1] = 0.0;
-        }
-        cur = nxt;
-        steps = more;
-        buf ^= 1;
-      }
-    }
-    if (!arrived && lane == 0) atomicCAS(&A.ps[p].status, FEAB_OK, FEAB_CUDA_ERROR);
-    // the rows' lanes of each column
-#pragma unroll
-    for (int j = 0; j < NL; ++j)
-#pragma unroll
-      for (int e = 0; e < W; ++e) {
-#pragma unroll
-        for (int o = 4; o < 32; o <<= 1) part[j][e] += __shfl_xor_sync(FEAB_FULL_MASK, part[j][e], o);
-        if (r == 0) sm[w][16 * j + W * t + e] = part[j][e];
-      }
+    // 64 problems of 4 to 16 columns, 849,747 rows: 456 us per step, 480 on whole panels.  Wider panels lose more to
+    // registers than a half saves (32 columns: 553 us for 448).
+    if (K == 16 && live_columns<K>(A, p) <= K / 2) pair_item<K, narrow_panel(K)>(A, it, p, reliable, st, buf, parity, sm[w]);
+    else pair_item<K, K>(A, it, p, reliable, st, buf, parity, sm[w]);
     __syncthreads();
     finish_step_a<K>(A, it, p, reliable, sm);
+  }
+}
+
+// P = M R + beta P on rows [r0, r1) of the first KC columns: two adjacent columns per thread with
+// 16-byte accesses, four pairs per trip.
+template <int K, int KC>
+__device__ __forceinline__ void p_rows(const BArgs& A, int p, int r0, int r1) {
+  constexpr int kRows = kThreads / (KC / 2);   // rows of a trip's quarter
+  const int cp = threadIdx.x % (KC / 2), live = live_columns<K>(A, p);
+  if (2 * cp >= live) return;
+  const double b0 = A.cs[(int64_t)p * K + 2 * cp].beta, b1 = A.cs[(int64_t)p * K + 2 * cp + 1].beta;
+  double2* __restrict__ P2 = reinterpret_cast<double2*>(A.P0) + cp;
+  const double2* __restrict__ R2 = reinterpret_cast<const double2*>(A.R) + cp;
+  for (int row = r0 + threadIdx.x / (KC / 2); row < r1; row += 4 * kRows) {
+    double2 rv[4], pv[4];
+    double dv[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = row + u * kRows;
+      const bool ok = i < r1;
+      rv[u] = ok ? R2[(int64_t)i * (K / 2)] : make_double2(0.0, 0.0);
+      pv[u] = ok ? P2[(int64_t)i * (K / 2)] : make_double2(0.0, 0.0);
+      dv[u] = ok ? __ldg(A.dinv + i) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = row + u * kRows;
+      if (i < r1) P2[(int64_t)i * (K / 2)] = make_double2(dv[u] * rv[u].x + b0 * pv[u].x, dv[u] * rv[u].y + b1 * pv[u].y);
+    }
   }
 }
 
@@ -1088,29 +1144,8 @@ __global__ void __launch_bounds__(kThreads) k_bstep_p(BArgs A) {
     if (P.done || !P.pending) continue;
     const int r0 = A.group_ptr[A.item_g0[it]], r1 = A.group_ptr[A.item_g1[it2 - 1]];
     if constexpr (K >= 2) {
-      // two adjacent columns per thread with 16-byte accesses, four pairs per trip
-      const int c2 = 2 * (threadIdx.x % (K / 2));
-      const double b0 = A.cs[(int64_t)p * K + c2].beta, b1 = A.cs[(int64_t)p * K + c2 + 1].beta;
-      const int64_t q0 = (int64_t)r0 * (K / 2) + threadIdx.x, q1 = (int64_t)r1 * (K / 2);
-      double2* __restrict__ P2 = reinterpret_cast<double2*>(P0);
-      const double2* __restrict__ R2 = reinterpret_cast<const double2*>(R);
-      for (int64_t q = q0; q < q1; q += 4 * kThreads) {
-        double2 rv[4], pv[4];
-        double dv[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int64_t e = q + (int64_t)u * kThreads;
-          const bool ok = e < q1;
-          rv[u] = ok ? R2[e] : make_double2(0.0, 0.0);
-          pv[u] = ok ? P2[e] : make_double2(0.0, 0.0);
-          dv[u] = ok ? __ldg(A.dinv + e / (K / 2)) : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int64_t e = q + (int64_t)u * kThreads;
-          if (e < q1) P2[e] = make_double2(dv[u] * rv[u].x + b0 * pv[u].x, dv[u] * rv[u].y + b1 * pv[u].y);
-        }
-      }
+      if (live_columns<K>(A, p) <= K / 2) p_rows<K, narrow_panel(K)>(A, p, r0, r1);
+      else p_rows<K, K>(A, p, r0, r1);
     } else {
       const double beta = A.cs[(int64_t)p].beta;
       const int64_t e0 = (int64_t)r0 + threadIdx.x, e1 = (int64_t)r1;
@@ -1131,6 +1166,75 @@ __global__ void __launch_bounds__(kThreads) k_bstep_p(BArgs A) {
       }
     }
    }
+  }
+}
+
+// Step B on rows [r0, r1) of the first KC columns, and the run's column sums to its row of the partials: two
+// adjacent columns per thread with 16-byte accesses, kVecU pairs per trip, every load of the trip
+// issued before any store.
+template <int K, int KC>
+__device__ __forceinline__ void b_rows(const BArgs& A, int it, int p, int r0, int r1, bool reliable,
+                                       double (&smv)[2][2 * kThreads]) {
+  constexpr int kRows = kThreads / (KC / 2);   // rows of one pair per thread
+  const int cp = threadIdx.x % (KC / 2), live = live_columns<K>(A, p);
+  const double al0 = A.cs[(int64_t)p * K + 2 * cp].alpha, al1 = A.cs[(int64_t)p * K + 2 * cp + 1].alpha;
+  double rr0 = 0.0, rr1 = 0.0, rz0 = 0.0, rz1 = 0.0;
+  const double2* __restrict__ P2 = reinterpret_cast<const double2*>(A.P0) + cp;
+  const double2* __restrict__ AP2 = reinterpret_cast<const double2*>(A.AP) + cp;
+  double2* __restrict__ X2 = reinterpret_cast<double2*>(A.X) + cp;
+  double2* __restrict__ R2 = reinterpret_cast<double2*>(A.R) + cp;
+  const int end = 2 * cp < live ? r1 : r0;
+  for (int row = r0 + threadIdx.x / (KC / 2); row < end; row += kVecU * kRows) {
+    double2 xv[kVecU], pv[kVecU], rv[kVecU], av[kVecU];
+    double dv[kVecU];
+#pragma unroll
+    for (int u = 0; u < kVecU; ++u) {
+      const int i = row + u * kRows;
+      const int64_t e = (int64_t)i * (K / 2);
+      const bool ok = i < end;
+      rv[u] = ok ? R2[e] : make_double2(0.0, 0.0);
+      dv[u] = ok ? __ldg(A.dinv + i) : 0.0;
+      if (!reliable) {
+        xv[u] = ok ? X2[e] : make_double2(0.0, 0.0);
+        pv[u] = ok ? P2[e] : make_double2(0.0, 0.0);
+        av[u] = ok ? AP2[e] : make_double2(0.0, 0.0);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kVecU; ++u) {
+      const int i = row + u * kRows;
+      const int64_t e = (int64_t)i * (K / 2);
+      if (i >= end) break;
+      double ri0 = rv[u].x, ri1 = rv[u].y;
+      if (!reliable) {
+        X2[e] = make_double2(xv[u].x + al0 * pv[u].x, xv[u].y + al1 * pv[u].y);
+        ri0 = rv[u].x - al0 * av[u].x;
+        ri1 = rv[u].y - al1 * av[u].y;
+        R2[e] = make_double2(ri0, ri1);
+      }
+      const double zi0 = dv[u] * ri0, zi1 = dv[u] * ri1;
+      rr0 += ri0 * ri0;
+      rr1 += ri1 * ri1;
+      rz0 += ri0 * zi0;
+      rz1 += ri1 * zi1;
+    }
+  }
+  // per-column sums: entry 2t + h holds column (2t + h) % KC; fold entries s apart (s >= KC)
+  smv[0][2 * threadIdx.x] = rr0;
+  smv[0][2 * threadIdx.x + 1] = rr1;
+  smv[1][2 * threadIdx.x] = rz0;
+  smv[1][2 * threadIdx.x + 1] = rz1;
+  for (int sh = kThreads; sh >= KC; sh >>= 1) {
+    __syncthreads();
+    if (threadIdx.x < sh) {
+      smv[0][threadIdx.x] += smv[0][threadIdx.x + sh];
+      smv[1][threadIdx.x] += smv[1][threadIdx.x + sh];
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < KC) {
+    A.part[(int64_t)it * 2 * K + threadIdx.x] = smv[0][threadIdx.x];
+    A.part[(int64_t)it * 2 * K + K + threadIdx.x] = smv[1][threadIdx.x];
   }
 }
 
@@ -1160,66 +1264,8 @@ __global__ void __launch_bounds__(kThreads, FEAB_BLOCK_B_MINB) k_bstep_b(BArgs A
     const double* __restrict__ AP = A.AP;
     const int r0 = A.group_ptr[A.item_g0[it]], r1 = A.group_ptr[A.item_g1[it2 - 1]];
     if constexpr (K >= 2 && FEAB_BLOCK_VECB) {
-      // two adjacent columns c2, c2 + 1 per thread with 16-byte accesses, kVecU pairs per trip,
-      // every load of the trip issued before any store
-      const int c2 = 2 * (threadIdx.x % (K / 2));
-      const double al0 = A.cs[(int64_t)p * K + c2].alpha, al1 = A.cs[(int64_t)p * K + c2 + 1].alpha;
-      double rr0 = 0.0, rr1 = 0.0, rz0 = 0.0, rz1 = 0.0;
-      const int64_t q0 = (int64_t)r0 * (K / 2) + threadIdx.x, q1 = (int64_t)r1 * (K / 2);
-      const double2* __restrict__ P2 = reinterpret_cast<const double2*>(pc);
-      const double2* __restrict__ AP2 = reinterpret_cast<const double2*>(AP);
-      double2* __restrict__ X2 = reinterpret_cast<double2*>(X);
-      double2* __restrict__ R2 = reinterpret_cast<double2*>(R);
-      for (int64_t q = q0; q < q1; q += kVecU * kThreads) {
-        double2 xv[kVecU], pv[kVecU], rv[kVecU], av[kVecU];
-        double dv[kVecU];
-#pragma unroll
-        for (int u = 0; u < kVecU; ++u) {
-          const int64_t e = q + (int64_t)u * kThreads;
-          const bool ok = e < q1;
-          rv[u] = ok ? R2[e] : make_double2(0.0, 0.0);
-          dv[u] = ok ? __ldg(A.dinv + e / (K / 2)) : 0.0;
-          if (!reliable) {
-            xv[u] = ok ? X2[e] : make_double2(0.0, 0.0);
-            pv[u] = ok ? P2[e] : make_double2(0.0, 0.0);
-            av[u] = ok ? AP2[e] : make_double2(0.0, 0.0);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < kVecU; ++u) {
-          const int64_t e = q + (int64_t)u * kThreads;
-          if (e >= q1) break;
-          double ri0 = rv[u].x, ri1 = rv[u].y;
-          if (!reliable) {
-            X2[e] = make_double2(xv[u].x + al0 * pv[u].x, xv[u].y + al1 * pv[u].y);
-            ri0 = rv[u].x - al0 * av[u].x;
-            ri1 = rv[u].y - al1 * av[u].y;
-            R2[e] = make_double2(ri0, ri1);
-          }
-          const double zi0 = dv[u] * ri0, zi1 = dv[u] * ri1;
-          rr0 += ri0 * ri0;
-          rr1 += ri1 * ri1;
-          rz0 += ri0 * zi0;
-          rz1 += ri1 * zi1;
-        }
-      }
-      // per-column sums: entry 2t + h holds column (2t + h) % K; fold entries s apart (s >= K)
-      smv[0][2 * threadIdx.x] = rr0;
-      smv[0][2 * threadIdx.x + 1] = rr1;
-      smv[1][2 * threadIdx.x] = rz0;
-      smv[1][2 * threadIdx.x + 1] = rz1;
-      for (int sh = kThreads; sh >= K; sh >>= 1) {
-        __syncthreads();
-        if (threadIdx.x < sh) {
-          smv[0][threadIdx.x] += smv[0][threadIdx.x + sh];
-          smv[1][threadIdx.x] += smv[1][threadIdx.x + sh];
-        }
-      }
-      __syncthreads();
-      if (threadIdx.x < K) {
-        A.part[(int64_t)it * 2 * K + c] = smv[0][c];
-        A.part[(int64_t)it * 2 * K + K + c] = smv[1][c];
-      }
+      if (live_columns<K>(A, p) <= K / 2) b_rows<K, narrow_panel(K)>(A, it, p, r0, r1, reliable, smv);
+      else b_rows<K, K>(A, it, p, r0, r1, reliable, smv);
     } else {
       const double alpha = A.cs[(int64_t)p * K + c].alpha;
       double rr = 0.0, rz = 0.0;
