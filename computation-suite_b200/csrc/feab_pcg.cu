@@ -407,6 +407,44 @@ __global__ void __launch_bounds__(kThreads) k_step_p(PcgArgs A) {
   if ((A.n & 1) && t0 == 0) A.p0[A.n - 1] = A.z[A.n - 1] + beta * A.p0[A.n - 1];
 }
 
+// A mixed reliable step: the FP64 residual r = b - K64 x through the CSR values; the thread's share of r.r.
+__device__ __forceinline__ double sell_reliable_residual(const PcgArgs& A, int lane) {
+  double rr = 0.0;
+  for_each_group<8>(A, lane, [&](const Group& gr) {
+    double acc[3];
+    const int hl = lane % 8;
+    group_spmv<8, double>(A, A.vals64, gr, hl, [&](int j) { return __ldg(A.x + j); }, acc);
+    if (hl < gr.f) {
+      const int i = gr.r0 + hl;
+      const double ri = A.b[i] - pick3(acc, hl);
+      A.r[i] = ri;
+      rr += ri * ri;
+    }
+  });
+  return rr;
+}
+
+// The end of a sliced step A: from the sum of `part` over the grid, alpha (a CG step) or r.r.
+__device__ __forceinline__ void finish_step_a(const PcgArgs& A, double (&part)[1], bool cg) {
+  PcgState* S = A.S_;
+  double tot[1];
+  if (grid_reduce<1>(part, A.partials, &S->ticket[0], tot) && threadIdx.x == 0) {
+    if (!cg) {
+      S->rr64 = tot[0];
+    } else {
+      if (FEAB_SELL_FUSED_P && S->p_pending) S->psel ^= 1;
+      S->p_pending = 0;
+      S->pAp = tot[0];
+      if (!(tot[0] > 0.0)) {  // p^T A p <= 0: A is not SPD (iterative_solvers.py:450-454)
+        S->status = FEAB_NOT_SPD;
+        S->done = 1;
+      } else {
+        S->alpha = S->rz_old / tot[0];
+      }
+    }
+  }
+}
+
 // Sliced path, kernel A: Ap = K p and p.Ap through the SELL-32 operator (PREC = its kind); in a
 // mixed reliable step, the FP64 residual r = b - K64 x through the CSR values instead.
 template <int PREC, bool IDX16>
@@ -417,17 +455,7 @@ __global__ void __launch_bounds__(kThreads, SellTuning<PREC>::kMinBlocks) k_step
   const int lane = threadIdx.x & 31;
   double part[1] = {0.0};
   if (PREC == FEAB_PREC_MIXED && mode == kModeReliable) {
-    for_each_group<8>(A, lane, [&](const Group& gr) {
-      double acc[3];
-      const int hl = lane % 8;
-      group_spmv<8, double>(A, A.vals64, gr, hl, [&](int j) { return __ldg(A.x + j); }, acc);
-      if (hl < gr.f) {
-        const int i = gr.r0 + hl;
-        const double ri = A.b[i] - pick3(acc, hl);
-        A.r[i] = ri;
-        part[0] += ri * ri;
-      }
-    });
+    part[0] = sell_reliable_residual(A, lane);
   } else if (FEAB_SELL_FUSED_P) {
     // p_new = z + beta p_old formed inside the gathers (two gathers per column) and written for
     // the lane's own rows into the other half of the p ping-pong; no separate P pass
@@ -470,22 +498,208 @@ __global__ void __launch_bounds__(kThreads, SellTuning<PREC>::kMinBlocks) k_step
       }
     }
   }
-  double tot[1];
-  if (grid_reduce<1>(part, A.partials, &S->ticket[0], tot) && threadIdx.x == 0) {
-    if (mode == kModeReliable && PREC != FEAB_PREC_FP64) {
-      S->rr64 = tot[0];
-    } else {
-      if (FEAB_SELL_FUSED_P && S->p_pending) S->psel ^= 1;
-      S->p_pending = 0;
-      S->pAp = tot[0];
-      if (!(tot[0] > 0.0)) {  // p^T A p <= 0: A is not SPD (iterative_solvers.py:450-454)
-        S->status = FEAB_NOT_SPD;
-        S->done = 1;
-      } else {
-        S->alpha = S->rz_old / tot[0];
+  finish_step_a(A, part, mode != kModeReliable || PREC == FEAB_PREC_FP64);
+}
+
+// ---------------------------------------------------------------- sliced step A through a ring
+// The step's product with the operator streamed through shared memory: a warp walks its slices as in
+// k_step_a_sell, but the blocks of 4 column steps (2-byte columns and values) come in by bulk copies,
+// kStages of them under way in a ring of the warp's own, so that a block's latency from HBM is not
+// followed by its gathers' latency 21 times in a slice, and no registers hold what is under way.
+//
+// What bounds it: at 128x32x32, 4,356 slices are one wave of warps, and the register path took 39 us
+// whatever the bytes (mixed in 246 MB; at 96x24x24 mixed was slower than FP64); with the ring the HBM's
+// rate sets the pace, and a part of K that L2 can hold beside the vectors is read without the
+// evict-first hint, so that it is still there in the next iteration.  The best part is that of some 68 MB
+// with nine vectors, about half of L2: at 128x32x32 mixed 88.2 ms per solve without, 85.2 with 46 MB of
+// K kept, 87.7 with 62 MB, 99 with 123 MB.
+// Whole solves, register path -> ring: 128x32x32 mixed (1e-9) 91.7 -> 85.2 ms, FP64 (1e-10) 109.7 -> 103.8;
+// 96x24x24 mixed 50.4 -> 38.2, FP64 44.0 -> 37.5.
+//
+// Stages and CTAs per SM, ms per solve (128 mixed, 128 FP64, 96 mixed, 96 FP64): 2 and 4: 85.2, 106.4,
+// 37.8, 37.3; 3 and 3: 91.6, -, 37.4, -; 3 and 2: -, 101.0, -, 36.0; 4 and 2: 86.2, 99.0, 37.7, 37.0; 1 and 4:
+// 84.1, 103.3, 44.0, 45.1.  Slices cut into equal runs of blocks for the CTAs' warps lost what they
+// balanced to the sums between the warps (97, 108, 38.5, 38.6).
+#ifndef FEAB_RING_STAGES_MIXED
+#define FEAB_RING_STAGES_MIXED 2
+#endif
+#ifndef FEAB_RING_MINB_MIXED
+#define FEAB_RING_MINB_MIXED 4
+#endif
+#ifndef FEAB_RING_STAGES_FP64
+#define FEAB_RING_STAGES_FP64 4
+#endif
+#ifndef FEAB_RING_MINB_FP64
+#define FEAB_RING_MINB_FP64 2
+#endif
+constexpr int kRingWarps = kThreads / 32;
+
+template <int KIND>
+struct RingTuning {
+  static constexpr int kValBytes = KIND == FEAB_PREC_FP64 ? 3072 : 2304;   // of a block of 4 steps
+  static constexpr int kBytes = kValBytes + 256;                            // with its 2-byte columns
+  static constexpr int kStages = KIND == FEAB_PREC_FP64 ? FEAB_RING_STAGES_FP64 : FEAB_RING_STAGES_MIXED;
+  static constexpr int kMinBlocks = KIND == FEAB_PREC_FP64 ? FEAB_RING_MINB_FP64 : FEAB_RING_MINB_MIXED;
+  static constexpr int kSmem = kRingWarps * kStages * kBytes;
+};
+
+constexpr int kRingSpinLimit = 1 << 22;   // polls of one copy's barrier (seconds)
+
+__device__ __forceinline__ void ring_copy(unsigned char* dst, const void* src, uint32_t bytes, uint32_t bar,
+                                          bool stream, unsigned long long first) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  if (stream)
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+        ::"r"(d), "l"(src), "r"(bytes), "r"(bar), "l"(first)
+        : "memory");
+  else
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(d), "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
+__device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity) {
+  for (int spin = 0; spin < kRingSpinLimit; ++spin) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
+template <int PREC>
+__global__ void __launch_bounds__(kThreads, RingTuning<PREC>::kMinBlocks) k_step_a_ring(PcgArgs A) {
+  using R = RingTuning<PREC>;
+  constexpr int kStages = R::kStages;
+  extern __shared__ __align__(128) unsigned char ring_smem[];
+  __shared__ unsigned long long full[kRingWarps][kStages];
+  PcgState* S = A.S_;
+  if (S->done) return;
+  const int mode = S->mode, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double part[1] = {0.0};
+  bool arrived = true;   // every copy waited for came in
+  if (PREC == FEAB_PREC_MIXED && mode == kModeReliable) {
+    part[0] = sell_reliable_residual(A, lane);
+  } else {
+    const SellView& V = A.sell;
+    unsigned char* const ring = ring_smem + (size_t)warp * kStages * R::kBytes;
+    if (lane < kStages)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;"
+                   ::"r"((uint32_t)__cvta_generic_to_shared(&full[warp][lane]))
+                   : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    __syncwarp();
+    unsigned long long first;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
+    const int nw = gridDim.x * kRingWarps, me = blockIdx.x * kRingWarps + warp;
+    // the next block to fetch: slice ps, step pb of steps up to pe
+    int ps = me, pb = 0, pe = 0;
+    if (ps < V.n_slices) {
+      pb = __ldg(V.soff + ps);
+      pe = __ldg(V.soff + ps + 1);
+    }
+    auto fetch = [&](int buf) {
+      while (pb >= pe) {
+        ps += nw;
+        if (ps >= V.n_slices) return;
+        pb = __ldg(V.soff + ps);
+        pe = __ldg(V.soff + ps + 1);
+      }
+      if (lane == 0) {
+        const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&full[warp][buf]);
+        unsigned char* const dst = ring + buf * R::kBytes;
+        const bool stream = (ps & 31) >= V.keep;
+        const size_t b = (size_t)pb;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(R::kBytes) : "memory");
+        ring_copy(dst + R::kValBytes, V.tcol16 + b * 32, 256, bar, stream, first);
+        if (PREC == FEAB_PREC_FP64) {
+          ring_copy(dst, V.v64 + 3 * b * 32, 3072, bar, stream, first);
+        } else {
+          ring_copy(dst, V.vhi + 3 * b * 32, 1536, bar, stream, first);
+          ring_copy(dst + 1536, V.vlo + 3 * b * 32, 768, bar, stream, first);
+        }
+      }
+      pb += 4;
+    };
+#pragma unroll
+    for (int q = 0; q < kStages; ++q) fetch(q);
+    int buf = 0;
+    uint32_t parity = 0;
+    const double* __restrict__ p = A.p0;
+    for (int sl = me; sl < V.n_slices; sl += nw) {
+      const SellLane L = sell_lane(V, sl, lane);
+      const int W = __ldg(V.soff + sl + 1) - __ldg(V.soff + sl);
+      double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+      for (int j = 0; j < W; j += 4) {
+        arrived = ring_wait((uint32_t)__cvta_generic_to_shared(&full[warp][buf]), parity) && arrived;
+        const unsigned char* blk = ring + buf * R::kBytes;
+        uint2 tq = reinterpret_cast<const uint2*>(blk + R::kValBytes)[lane];
+        SellBlock<PREC> B;
+        if constexpr (PREC == FEAB_PREC_FP64) {
+          // a lane's 32 bytes of a row, its two halves in an order that keeps eight lanes off each other's banks
+          const int swap = (lane >> 2) & 1;
+          if (swap) tq = make_uint2(tq.y, tq.x);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            const double2* vp = reinterpret_cast<const double2*>(blk + 1024 * k) + 2 * lane;
+            const double2 q0 = vp[swap], q1 = vp[swap ^ 1];
+            B.v[k][0] = q0.x;
+            B.v[k][1] = q0.y;
+            B.v[k][2] = q1.x;
+            B.v[k][3] = q1.y;
+          }
+        } else {
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            B.h[k] = reinterpret_cast<const uint4*>(blk)[32 * k + lane];
+            B.l[k] = reinterpret_cast<const uint2*>(blk + 1536)[32 * k + lane];
+          }
+        }
+        const double* __restrict__ pr = p + L.r0;
+        const double d[4] = {__ldg(pr + (int)(int16_t)(tq.x & 0xffffu)), __ldg(pr + (int)(int16_t)(tq.x >> 16)),
+                             __ldg(pr + (int)(int16_t)(tq.y & 0xffffu)), __ldg(pr + (int)(int16_t)(tq.y >> 16))};
+        __syncwarp();   // every lane has read the block
+        fetch(buf);
+        sell_use_block<PREC>(B, d, a0, a1, a2);
+        if (++buf == kStages) {
+          buf = 0;
+          parity ^= 1u;
+        }
+      }
+      double acc[3] = {a0, a1, a2};
+      double own[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) own[k] = k < L.f ? __ldg(p + L.r0 + k) : 0.0;
+      if (PREC == FEAB_PREC_MIXED) {
+        // the own-node term: own DOF j is row popc(mask below j) of the group
+        const double* __restrict__ Sp = V.S + (int64_t)L.r0 * 3;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const double x = ((L.mask >> j) & 1) ? pick3(own, __popc(L.mask & ((1 << j) - 1))) : 0.0;
+#pragma unroll
+          for (int k = 0; k < 3; ++k)
+            if (k < L.f) acc[k] += __ldg(Sp + 3 * k + j) * x;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        if (k < L.f) {
+          A.Ap[L.r0 + k] = acc[k];
+          part[0] += own[k] * acc[k];
+        }
       }
     }
   }
+  if (!arrived && lane == 0) {   // a copy did not come in
+    S->status = FEAB_CUDA_ERROR;
+    S->done = 1;
+  }
+  finish_step_a(A, part, mode != kModeReliable || PREC == FEAB_PREC_FP64);
 }
 
 // Step kernel B.
@@ -840,10 +1054,33 @@ int sell_grid(const PcgArgs& A) {
   return std::max(1, std::min((A.sell.n_slices + wpb - 1) / wpb, max_grid()));
 }
 
+// The ring takes operators with 2-byte columns whose arrays start on the bulk copies' 16 bytes.
+bool sell_ring(const PcgArgs& A, int prec) {
+  auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+  const SellView& V = A.sell;
+  return V.tcol16 && al(V.tcol16) && (prec == FEAB_PREC_FP64 ? al(V.v64) : al(V.vhi) && al(V.vlo));
+}
+
+template <int PREC>
+int ring_grid(const PcgArgs& A) {
+  const int ctas = (A.sell.n_slices + kRingWarps - 1) / kRingWarps;
+  return std::max(1, std::min(ctas, sm_count() * RingTuning<PREC>::kMinBlocks));
+}
+
+template <int PREC>
+cudaError_t ring_attributes() {
+  const auto fn = k_step_a_ring<PREC>;
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, RingTuning<PREC>::kSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  return e;
+}
+
 template <int PREC>
 void launch_step_sell(const PcgArgs& A, const Grids& gr, cudaStream_t s) {
   if (!FEAB_SELL_FUSED_P) k_step_p<<<gr.b, kThreads, 0, s>>>(A);
-  if (A.sell.tcol16) k_step_a_sell<PREC, true><<<sell_grid(A), kThreads, 0, s>>>(A);
+  if (sell_ring(A, PREC)) k_step_a_ring<PREC><<<ring_grid<PREC>(A), kThreads, RingTuning<PREC>::kSmem, s>>>(A);
+  else if (A.sell.tcol16) k_step_a_sell<PREC, true><<<sell_grid(A), kThreads, 0, s>>>(A);
   else k_step_a_sell<PREC, false><<<sell_grid(A), kThreads, 0, s>>>(A);
   k_step_b<PREC><<<gr.b, kThreads, 0, s>>>(A);
 }
@@ -981,9 +1218,12 @@ int32_t run_pcg(const PcgArgs& A, int prec, int chunk, int maxiter, int lpg, fea
   }
   if (!resident && rc == FEAB_OK) do {
     if (fail(graphs.events(ev))) break;
+    if (A.use_sell &&
+        fail(prec == FEAB_PREC_MIXED ? ring_attributes<FEAB_PREC_MIXED>() : ring_attributes<FEAB_PREC_FP64>()))
+      break;
     // the chunk's launches bake in A, the launch shapes and the chunk length
     const uint64_t topo = topo_signature({prec, chunk, lpg, A.use_sell, gr.a, gr.b, A.use_sell ? sell_grid(A) : 0,
-                                          FEAB_SELL_FUSED_P});
+                                          A.use_sell && sell_ring(A, prec) ? 1 : 0, FEAB_SELL_FUSED_P});
     auto record = [&](cudaStream_t cs) {
       for (int c = 0; c < chunk; ++c) {
         if (prec == FEAB_PREC_FP32) launch_step<FEAB_PREC_FP32>(A, gr, lpg, cs);
@@ -1068,6 +1308,9 @@ void fill_matrix(const feab_csr* M, PcgArgs* A) {
 
 void fill_sell(const feab_csr* M, const feab_sell_operator* D, PcgArgs* A) {
   A->sell = sell_view(M, D);
+  // the slices that the ring has L2 keep: 68 MB less nine vectors, of K's 26 or 20 bytes per 3 rows' entry
+  const double room = 68e6 - 72.0 * M->n, bytes = (D->kind == FEAB_PREC_FP64 ? 26.0 : 20.0) / 3.0 * (double)M->nnz;
+  A->sell.keep = room <= 0.0 || bytes <= 0.0 ? 0 : (int)std::min(32.0, 32.0 * room / bytes);
   A->use_sell = 1;
 }
 

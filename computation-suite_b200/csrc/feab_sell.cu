@@ -214,6 +214,7 @@ SellView sell_view(const feab_csr* A, const feab_sell_operator* op) {
   V.gmask = op->gmask;
   V.S = op->S;
   V.group_ptr = A->group_ptr;
+  V.keep = 0;
   return V;
 }
 

@@ -94,6 +94,7 @@ struct SellView {
   const uint8_t* gmask;
   const double* S;
   const int32_t* group_ptr;
+  int keep;                 // of 32 slices, those that the PCG asks L2 to keep between iterations
 };
 
 // The lane's group: rows r0 .. r0+f-1 and (difference form) its free-DOF mask.
