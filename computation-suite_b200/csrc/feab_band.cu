@@ -115,7 +115,7 @@ static_assert(sizeof(BandState) <= FEAB_BAND_HEADER_BYTES, "band header");
 // pivots take 6.5 (a reciprocal square root, a product and a difference, 16 cycles each, one after
 // the other), the two products 3.2, the inverse 2.7.  Measured, three launches per block column ->
 // one kernel: 64x16x16 elements (867 block columns, 28 bands) 74.2 -> 12.6 ms, 96x24x24 (2,813, 59
-// bands, bound by the workers at 22 TFLOP/s) 335 -> 118 ms, 33x9x8 (140, 9 bands) 10.6 -> 2.0 ms.
+// bands, bound by the workers at 22 TFLOP/s) 335 -> 118 ms (45.7 with the nodes in layers, 31 bands), 33x9x8 (140, 9 bands) 10.6 -> 2.0 ms.
 
 struct BandWork {
   double* tiles;
@@ -682,7 +682,7 @@ __global__ void __launch_bounds__(kBandThreads, 1) k_band_factor(BandWork B) {
 // reduction, and one hop to another SM), while a CTA's tiles per block row (bands / C) come in
 // faster than that; wide bands are bound by what 16 SMs read (about 1.4 TB/s).  Measured, two
 // launches per block row -> one kernel, both directions: 64x16x16 elements (867 block rows, 28
-// bands) 19.0 -> 2.1 ms, 96x24x24 (2,813, 59 bands) 63.3 -> 8.3 ms, 33x9x8 (140, 9) 2.07 -> 0.36 ms.
+// bands) 19.0 -> 2.1 ms, 96x24x24 (2,813, 59 bands) 63.3 -> 8.3 ms (6.5 with 31 bands), 33x9x8 (140, 9) 2.07 -> 0.36 ms.
 constexpr int kSolveWarps = 16;
 constexpr int kSolveThreads = 32 * kSolveWarps;       // that compute; one more warp fetches the tiles
 constexpr int kSolveCta = kSolveThreads + 32;

@@ -31,8 +31,9 @@
 //   37x11x9          139   18.5 ->  7.6    20.5 ->  8.4
 //   64x16x16         578   20.1 -> 10.0    29.4 -> 10.4
 //   80x20x20        1103   22.9 -> 19.6    35.3 -> 18.1
-// Above 8 slices per SM most of K comes from L2 or HBM in every iteration and the step kernels,
-// with more warps to wait for it, are as fast (96x24x24, FP64: 30.6 us).
+// Above 8 slices per SM most of K comes from L2 or HBM in every iteration, and the step kernels stream it through
+// their ring with more warps to wait for it.  Below, they lose to the launches: whole solves at 80x20x20,
+// resident against the steps with the ring, FP64 21.2 and 25.7 ms, mixed 18.6 and 26.8 ms.
 #pragma once
 
 namespace feab {

@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kThreads, SellTuning<KIND>::kMinBlocks) k_sell
 }  // namespace
 
 SellView sell_view(const feab_csr* A, const feab_sell_operator* op) {
-  SellView V;
+  SellView V{};   // no stray bytes: the launch arguments are a key of the graph cache
   V.kind = op->kind;
   V.n_slices = op->n_slices;
   V.n_groups = A->n_groups;
