@@ -54,6 +54,7 @@ struct ColState {  // per (problem, column)
 
 struct BArgs {
   int32_t n, n_groups, n_problems, n_items, k;
+  int32_t brun;            // work items of a run of the vector passes
   const int32_t* row_ptr;
   const int32_t* col_idx;
   const int32_t* group_ptr;
@@ -108,13 +109,19 @@ __device__ __forceinline__ bool last_of_problem(uint32_t* ticket, int n_items_p,
   return last;
 }
 
-// The vector passes P and B take runs of up to kBRun consecutive work items of one problem as
+// The vector passes P and B take runs of up to A.brun consecutive work items of one problem as
 // one contiguous row range (the items of a problem cover consecutive row groups), which cuts
-// their per-item block reductions and tickets; the SpMM keeps the finer items for its balance.
-#ifndef FEAB_BLOCK_BRUN
-#define FEAB_BLOCK_BRUN 4
-#endif
-constexpr int kBRun = FEAB_BLOCK_BRUN;
+// their per-item block reductions and tickets; the SpMM keeps the finer items for its balance.  One
+// problem's runs are as long as there are two for every SM, at most kMaxRun: 289 items with 64 columns at
+// 55,488 rows took 31 us in P and in B as 73 runs of four, now 24 and 21.  A batch keeps runs of four: there the
+// tuner would take larger items, of which too few are left when most problems are done.
+constexpr int kMaxRun = 4;
+
+int items_per_run(int n_items, int n_problems) {
+  int run = kMaxRun;
+  while (n_problems == 1 && run > 1 && n_items < 2 * run * sm_count()) run >>= 1;
+  return run;
+}
 
 // Columns of problem p in use, 1 .. K.  The panel is as wide as the widest problem needs, rounded up to a
 // power of two; nothing reads what a step would write to the columns behind a problem's own.
@@ -143,13 +150,13 @@ __device__ __forceinline__ void block_col_sums(double v, double* sm) {
 // flight, then the threads of a column are added as a tree; a fixed order.  In threads < K.  One
 // thread per column walking the rows one after the other took longer than the step's vector passes
 // when a problem has many items (250 of 621 us per step at 4,352 items).  HEADS: only the first
-// item of each run of kBRun has a row.
+// item of each run of `run` has a row.
 template <int K, int NV, bool HEADS>
-__device__ __forceinline__ void problem_totals(const double* part, int i0, int i1, double (&s)[NV]) {
+__device__ __forceinline__ void problem_totals(const double* part, int i0, int i1, int run, double (&s)[NV]) {
   __shared__ double sm[NV][kThreads];
   const int c = threadIdx.x % K, h = threadIdx.x / K;
   constexpr int H = kThreads / K, U = 8;
-  const int rows = HEADS ? (i1 - 1) / kBRun - i0 / kBRun + 1 : i1 - i0;
+  const int rows = HEADS ? (i1 - 1) / run - i0 / run + 1 : i1 - i0;
 #pragma unroll
   for (int k = 0; k < NV; ++k) s[k] = 0.0;
   for (int m0 = h; m0 < rows; m0 += U * H) {
@@ -157,7 +164,7 @@ __device__ __forceinline__ void problem_totals(const double* part, int i0, int i
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int m = m0 + u * H;
-      const int row = HEADS && m > 0 ? (i0 / kBRun + m) * kBRun : i0 + m;
+      const int row = HEADS && m > 0 ? (i0 / run + m) * run : i0 + m;
 #pragma unroll
       for (int k = 0; k < NV; ++k) v[u][k] = m < rows ? __ldcg(&part[(int64_t)row * 2 * K + k * K + c]) : 0.0;
     }
@@ -686,7 +693,7 @@ __global__ void __launch_bounds__(kThreads) k_bsetup(BArgs A) {
     const int i0 = A.prob_items[p], n_it = A.prob_items[p + 1] - i0;
     if (last_of_problem(&A.ps[p].ticket_a, n_it)) {
       double tot[2];
-      problem_totals<K, 2, false>(A.part, i0, i0 + n_it, tot);
+      problem_totals<K, 2, false>(A.part, i0, i0 + n_it, A.brun, tot);
       if (threadIdx.x < K) {
         const double s0 = tot[0], s1 = tot[1];
         ColState& C = A.cs[(int64_t)p * K + c];
@@ -736,7 +743,7 @@ __device__ __forceinline__ void finish_step_a(const BArgs& A, int it, int p, boo
   const int i0 = A.prob_items[p], n_it = A.prob_items[p + 1] - i0;
   if (last_of_problem(&A.ps[p].ticket_a, n_it)) {
     double tot[1];
-    problem_totals<K, 1, false>(A.part, i0, i0 + n_it, tot);
+    problem_totals<K, 1, false>(A.part, i0, i0 + n_it, A.brun, tot);
     if (threadIdx.x < K) {
       const int c = threadIdx.x;
       const double s = tot[0];
@@ -1154,9 +1161,9 @@ __global__ void __launch_bounds__(kThreads) k_bstep_p(BArgs A) {
   double* __restrict__ P0 = A.P0;
   double* __restrict__ X = A.X;
   const double* __restrict__ R = A.R;
-  for (int ru = blockIdx.x; ru * kBRun < A.n_items; ru += gridDim.x) {
-   const int it_end = min(A.n_items, (ru + 1) * kBRun);
-   for (int it = ru * kBRun, it2 = it; it < it_end; it = it2) {
+  for (int ru = blockIdx.x; ru * A.brun < A.n_items; ru += gridDim.x) {
+   const int it_end = min(A.n_items, (ru + 1) * A.brun);
+   for (int it = ru * A.brun, it2 = it; it < it_end; it = it2) {
     const int p = A.item_problem[it];
     for (it2 = it + 1; it2 < it_end && A.item_problem[it2] == p; ++it2) {
     }
@@ -1265,9 +1272,9 @@ __global__ void __launch_bounds__(kThreads, FEAB_BLOCK_B_MINB) k_bstep_b(BArgs A
   __shared__ double smv[2][2 * kThreads];
   __shared__ int flag_any, flag_all;
   const int c = threadIdx.x % K;
-  for (int ru = blockIdx.x; ru * kBRun < A.n_items; ru += gridDim.x) {
-   const int it_end = min(A.n_items, (ru + 1) * kBRun);
-   for (int it = ru * kBRun, it2 = it; it < it_end; it = it2) {
+  for (int ru = blockIdx.x; ru * A.brun < A.n_items; ru += gridDim.x) {
+   const int it_end = min(A.n_items, (ru + 1) * A.brun);
+   for (int it = ru * A.brun, it2 = it; it < it_end; it = it2) {
     const int p = A.item_problem[it];
     for (it2 = it + 1; it2 < it_end && A.item_problem[it2] == p; ++it2) {
     }
@@ -1327,7 +1334,7 @@ __global__ void __launch_bounds__(kThreads, FEAB_BLOCK_B_MINB) k_bstep_b(BArgs A
         flag_all = 1;
       }
       double tot[2];
-      problem_totals<K, 2, true>(A.part, i0, i0 + n_it, tot);
+      problem_totals<K, 2, true>(A.part, i0, i0 + n_it, A.brun, tot);
       if (threadIdx.x < K) {
         const double s0 = tot[0], s1 = tot[1];
         ColState& C = A.cs[(int64_t)p * K + c];
@@ -1495,7 +1502,8 @@ template <int K>
 int32_t run_block(BArgs A, int prec, int chunk, int maxiter, cudaStream_t s, int32_t* host_iters, double* host_relres,
                   int32_t* host_status) {
   const int grid = std::max(1, std::min(A.n_items, sm_count() * 4));
-  const int grid_pb = std::max(1, std::min((A.n_items + kBRun - 1) / kBRun, sm_count() * 4));  // P and B runs
+  A.brun = items_per_run(A.n_items, A.n_problems);
+  const int grid_pb = std::max(1, std::min((A.n_items + A.brun - 1) / A.brun, sm_count() * 4));  // P and B runs
   cudaMemsetAsync(A.ps, 0, sizeof(ProbState) * A.n_problems, s);
   int32_t np = A.n_problems;
   cudaMemcpyAsync(A.remaining, &np, sizeof(int32_t), cudaMemcpyHostToDevice, s);
