@@ -6,8 +6,8 @@ splu of K_ff, a singularity test on its pivots (min |U_ii| < tol max |U_ii|, tol
 lu.solve.  K_ff is SPD, so its LU factorisation without pivoting is the Cholesky factorisation
 K_ff = L L^T with U_ii = L_ii^2; the same pivot test is made on the Cholesky pivots.
 
-The free DOFs are renumbered node by node, layer by layer along the mesh's longest extent or in reverse
-Cuthill-McKee order of the node graph (on the host, as SuperLU's column ordering is in the
+The free DOFs are renumbered node by node, layer by layer along the axis with most layers of nodes or in
+reverse Cuthill-McKee order of the node graph (on the host, as SuperLU's column ordering is in the
 reference), so that the band of the renumbered K_ff is narrow; the band is factored and solved on the GPU with the
 feab_band_* kernels (64 x 64 tiles).  The factor of an operator is computed once and reused for
 every right-hand side.
@@ -62,11 +62,18 @@ def coordinate_order(op, coords):
 
 
 def layer_order(op, coords, sample=2048):
-    """Node row groups sorted layer by layer along the mesh's longest extent, within a layer by the
-    other two, and the number of layers: the coordinates in units of the mesh's own spacing along each
+    """Node row groups sorted layer by layer along the axis with most layers, within a layer by the other
+    two, and the number of layers: the coordinates in units of the mesh's own spacing along each
     axis (the mean length of the longer edges of some nodes), rounded.  Unlike the coordinates
     themselves, whole layers stay together when the nodes are not exactly in their planes, so the
-    band is one cross-section of nodes wide and not two.  On the operator's device."""
+    band is one cross-section of nodes wide and not two; and the smallest cross-section is the one across
+    the axis of most layers, whatever its length.  On the operator's device."""
+    order, n_layers = _layers(op, coords, sample)
+    return order, int(n_layers[2])
+
+
+def _layers(op, coords, sample=2048):
+    """The order of layer_order, and the layers along the three axes, ascending."""
     p = op.pattern
     dev = op.vals64.device
     gp, rp = p.group_ptr.to(torch.int64), p.row_ptr.to(torch.int64)
@@ -82,13 +89,12 @@ def layer_order(op, coords, sample=2048):
     d = (key[nbr] - key[some[src]]).abs()
     long = d > 0.5 * d.amax(0)
     h = torch.where(long, d, torch.zeros_like(d)).sum(0) / long.sum(0).clamp_min(1)
-    lo, hi = key.amin(0), key.amax(0)
+    lo = key.amin(0)
     q = ((key - lo) / torch.where(h > 0, h, torch.ones_like(h))).round().to(torch.int64)
-    n_layers = q.amax(0) + 1
-    ext, n_layers = torch.stack([hi - lo, n_layers.to(torch.float64)]).cpu().numpy()     # one read-back
-    ax = np.argsort(ext)
+    n_layers = (q.amax(0) + 1).cpu().numpy()
+    ax = np.argsort(n_layers, kind="stable")      # fewest first: neighbours within a layer stay closest
     code = (q[:, ax[2]] * int(n_layers[ax[1]]) + q[:, ax[1]]) * int(n_layers[ax[0]]) + q[:, ax[0]]
-    return torch.argsort(code, stable=True), int(n_layers[ax[2]])
+    return torch.argsort(code, stable=True), n_layers[ax]
 
 
 def dof_permutation(op, order):
@@ -103,43 +109,61 @@ def dof_permutation(op, order):
     return (first[group] + torch.arange(op.n, device=dev) - gp[group]).to(torch.int32)
 
 
+def narrowest_order(op, coords, width):
+    """(iperm, bandwidth, name) of the node order with the narrowest band; width(iperm) is an order's band.
+    coords: the mesh's node coordinates (N, 3), if known: the ordering in layers is then tried first, and
+    unless its band is known to be about as narrow as any, the ordering by coordinates and reverse
+    Cuthill-McKee beside it."""
+    best = None
+
+    def consider(name, order):
+        nonlocal best
+        iperm = dof_permutation(op, order)
+        bw = int(width(iperm))
+        if best is None or bw < best[1]:
+            best = (iperm, bw, name)
+
+    done = False
+    if coords is not None:
+        order, n_layers = _layers(op, coords)
+        consider("axis", order)
+        # No order's band is narrower than the rows divided by the steps between the two nodes farthest
+        # apart.  On a whole box these are the layers of its longest axis; within half as much again (a layer
+        # and the line of nodes beside the next one's nearest) the other orders are not tried: reverse
+        # Cuthill-McKee takes 30 ms of host time at 96x24x24 elements and is 1.2 to 2.7 times as wide on boxes.
+        # A box has a node in every place of the lattice and every one of its 27 neighbours; a bent, branched,
+        # slit or graded mesh lacks some, and its farthest nodes may be many layers apart.
+        nl = n_layers.astype(np.float64)
+        G = op.pattern.n_groups
+        box = G >= 0.99 * np.prod(nl) > 0 and op.pattern.nnz >= 0.99 * (op.n / G) ** 2 * np.prod(3 * nl - 2)
+        done = box and best[1] <= 1.5 * op.n / nl[2] + 6
+    if not done:
+        if coords is not None:
+            consider("axis", coordinate_order(op, coords))
+        consider("rcm", node_order(op))
+    return best
+
+
 class BandCholesky:
     """K_ff = L L^T on the device, in the renumbered order.  Raises MemoryError when the band
     would take more than `max_fraction` of the device's free memory."""
 
     def __init__(self, op, coords=None, max_fraction=0.6):
-        """coords: the mesh's node coordinates (N, 3), if known: the ordering in layers along the longest
-        axis is then tried first, and unless its band is about one layer wide, the ordering by
-        coordinates and reverse Cuthill-McKee beside it, and the narrowest band is kept."""
+        """coords: the mesh's node coordinates (N, 3), if known, for the order (see narrowest_order)."""
         self.op = op
         dev = op.vals64.device
         if op.pattern.group_ptr is None:
             raise ValueError("the direct solve needs node row groups (an assembled K_ff)")
         csr = op.csr_struct()
         scratch = torch.zeros(2, dtype=torch.int32, device=dev)
-        best = None
 
-        def consider(name, order):
-            nonlocal best
-            iperm = dof_permutation(op, order)
+        def width(iperm):
             bw = C.c_int32(0)
             rc = L.lib.feab_band_width(C.byref(csr), L.dptr(iperm), L.dptr(scratch), C.byref(bw), L.stream_ptr(dev))
             L.raise_for(rc, "band width")
-            if best is None or bw.value < best[1]:
-                best = (iperm, int(bw.value), name)
+            return bw.value
 
-        layers = 0
-        if coords is not None:
-            order, layers = layer_order(op, coords)
-            consider("axis", order)
-        # The rows of one layer bound the band of an ordering layer by layer from below.  Within half
-        # as much again the other orderings are not tried: on the box meshes reverse Cuthill-McKee's
-        # band is 2.7 times as wide, and it takes 30 ms of host time at 96x24x24 elements.
-        if coords is None or best[1] > 1.5 * op.n / layers + 6:
-            if coords is not None:
-                consider("axis", coordinate_order(op, coords))
-            consider("rcm", node_order(op))
-        self.iperm, self.bandwidth, self.ordering = best
+        self.iperm, self.bandwidth, self.ordering = narrowest_order(op, coords, width)
         nbytes = int(L.lib.feab_band_bytes(op.n, self.bandwidth))
         free, _ = torch.cuda.mem_get_info(dev)
         if nbytes > max_fraction * free:

@@ -73,3 +73,47 @@ def test_layer_order_on_graded_spacing_is_a_bijection():
     order, layers = layer_order(op, X)
     assert sorted(order.tolist()) == list(range(len(starts))) and layers >= 1
     assert sorted(dof_permutation(op, order).tolist()) == list(range(op.n))
+
+
+def _chosen(X, el, fixed):
+    """The band that the direct solve chooses, by its ordering, and the bands of the orderings that it had
+    before the one in layers."""
+    from feab200.direct import coordinate_order, dof_permutation, narrowest_order, node_order
+    op, K, starts = _operator(X, el, fixed)
+    iperm, bw, _ = narrowest_order(op, X, lambda ip: _band(K, ip.numpy()))
+    assert bw == _band(K, iperm.numpy()) and sorted(iperm.tolist()) == list(range(op.n))
+    return bw, [_band(K, dof_permutation(op, o).numpy()) for o in (coordinate_order(op, X), node_order(op))]
+
+
+@pytest.mark.parametrize("shape,size", [((4, 48, 48), (2.0, 0.4, 0.4)), ((4, 60, 10), (2.0, 1.0, 0.4)),
+                                        ((6, 24, 24), (2.0, 0.4, 0.4)), ((10, 30, 30), (2.0, 0.4, 0.4)),
+                                        ((2, 2, 40), (2.0, 1.0, 0.4)), ((33, 9, 8), (2.0, 0.4, 0.4)),
+                                        ((25, 25, 2), (2.0, 0.4, 0.4)), ((7, 1, 1), (1.0, 0.1, 0.1)),
+                                        ((12, 12, 12), (1.0, 1.0, 1.0))])
+def test_the_chosen_band_is_the_narrowest(shape, size):
+    """Flat and stretched boxes among them: the longest axis is not always that of most layers."""
+    X, el = O.box_mesh(*size, *shape)
+    bw, others = _chosen(X, el, O.fixed_dofs_on_plane(X, 0, 0.0))
+    assert bw <= min(others)
+
+
+@pytest.mark.parametrize("kind", ["bent", "slit"])
+def test_the_chosen_band_is_the_narrowest_on_other_meshes(kind):
+    """Two legs side by side, and a plate that slits of one element's width make one long strip: the layers
+    of the bounding box cross the strip many times, an order along it once."""
+    nx, ny = (24, 20) if kind == "bent" else (40, 40)
+    X, el = O.box_mesh(float(nx), float(ny), 1.0, nx, ny, 1)
+    c = X[el].mean(axis=1)
+    if kind == "bent":
+        keep = (c[:, 0] > nx - 3) | (c[:, 1] < 3) | (c[:, 1] > ny - 3)
+    else:
+        leg = np.floor(c[:, 1]).astype(int)
+        turn = np.where((leg // 8) % 2 == 0, c[:, 0] > nx - 7, c[:, 0] < 7)
+        keep = (leg % 8 != 7) | turn
+    el = el[keep]
+    used = np.unique(el)
+    new = np.full(len(X), -1)
+    new[used] = np.arange(len(used))
+    X, el = X[used], new[el]
+    bw, others = _chosen(X, el, O.fixed_dofs_on_plane(X, 0, 0.0)[:30])
+    assert bw <= min(others)
