@@ -820,11 +820,30 @@ __global__ void __cluster_dims__(kJacCluster, 1, 1) __launch_bounds__(kJacThread
     ++sweep;
   }
   if (cta == 0) {
-    // descending order: an eigenvalue's place is the number of those before it
+    // descending order: an eigenvalue's place is the number of those before it.  A NaN is neither before nor
+    // behind any, so that places would be taken twice and others left unwritten: a selection sort then.
+    const bool unordered = __syncthreads_or(tid < k && !(S.a[tid][tid] == S.a[tid][tid]));
+    if (unordered) {
+      if (tid == 0) {
+        for (int i = 0; i < k; ++i) S.place[i] = i;   // here: the index at each place
+        for (int i = 0; i < k; ++i) {
+          int best = i;
+          for (int j = i + 1; j < k; ++j)
+            if (S.a[S.place[j]][S.place[j]] > S.a[S.place[best]][S.place[best]]) best = j;
+          const int t = S.place[i];
+          S.place[i] = S.place[best];
+          S.place[best] = t;
+        }
+      }
+      __syncthreads();
+    }
     if (tid < k) {
       const double x = S.a[tid][tid];
       int at = 0;
-      for (int j = 0; j < k; ++j) at += S.a[j][j] > x || (!(S.a[j][j] < x) && j < tid) ? 1 : 0;
+      if (unordered)
+        while (S.place[at] != tid) ++at;
+      else
+        for (int j = 0; j < k; ++j) at += S.a[j][j] > x || (!(S.a[j][j] < x) && j < tid) ? 1 : 0;
       w[at] = scalbn(x, e);
       for (int r = 1; r < kJacCluster; ++r) {
         const uint32_t dst = jac_map(&S.place[tid], r);

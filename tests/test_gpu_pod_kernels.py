@@ -64,3 +64,21 @@ def test_fit_does_not_depend_on_the_layout_of_the_snapshots(k, dtype):
         p = PodBasis().fit(other, n_modes=5)
         assert np.array_equal(p.singular_values, base.singular_values) and torch.equal(p.V, base.V)
     assert torch.equal(X, before)
+
+
+@pytest.mark.parametrize("k", [1, 3, 32, 63, 64])
+@pytest.mark.parametrize("where", ["first", "middle", "all"])
+def test_symeig_writes_every_output_where_a_value_is_nan(k, where):
+    """A diagonal matrix with NaN among its entries needs no rotation: its entries come out, each once, and
+    the unit vectors in the same order."""
+    from feab200 import _lib as L
+    d = np.random.default_rng(k).permutation(k) + 1.0
+    d[{"first": slice(0, 1), "middle": slice(k // 3, k // 3 + 2), "all": slice(None)}[where]] = np.nan
+    A = torch.as_tensor(np.diag(d)).cuda()
+    w = torch.full((k,), 1e9, dtype=torch.float64, device="cuda")
+    V = torch.full((k, k), 1e9, dtype=torch.float64, device="cuda")
+    assert L.lib.feab_symeig_jacobi(L.dptr(A), k, L.dptr(w), L.dptr(V), 40, None, L.stream_ptr(A.device)) == L.FEAB_OK
+    w, V = w.cpu().numpy(), V.cpu().numpy()
+    assert np.array_equal(np.sort(w), np.sort(d), equal_nan=True)
+    assert np.array_equal(np.sort(V, axis=0)[-1], np.ones(k)) and np.array_equal(V.sum(0), np.ones(k))
+    assert np.array_equal(d[V.argmax(0)], w, equal_nan=True)
