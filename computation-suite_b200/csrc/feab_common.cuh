@@ -20,6 +20,12 @@
     if (_e != cudaSuccess) return FEAB_CUDA_ERROR;           \
   } while (0)
 
+// Cycles after which a wait on the device gives up (0 in the tests' own builds: a wait gives up when its
+// first poll fails).
+#ifndef FEAB_WAIT_CYCLES
+#define FEAB_WAIT_CYCLES (1ll << 32)
+#endif
+
 namespace feab {
 
 // Records the first device-side error: status word 0 -> code, plus the offending index.
@@ -67,6 +73,22 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double* sh) {
   }
   __syncthreads();
 }
+
+// The end of a wait: one object per wait, over() after every poll that failed.  True once the wait has taken
+// some seconds of the SM's clock.  The clock is read every 64 polls, and a span counts a 64th of a second at
+// most: the time in which the context is switched out is not the wait's.
+struct WaitLimit {
+  static constexpr long long kCycles = FEAB_WAIT_CYCLES, kSpan = 1ll << 25;
+  long long last = 0, spent = 0;
+  int polls = 0;
+  __device__ __forceinline__ bool over() {
+    if ((++polls & 63) != 0 && kCycles > 0) return false;
+    const long long now = clock64(), span = now - last;
+    if (last != 0) spent += span >= 0 && span < kSpan ? span : kSpan;
+    last = now;
+    return spent >= kCycles;
+  }
+};
 
 // Number of SMs of the current device, cached per process.
 int sm_count();

@@ -610,6 +610,7 @@ __global__ void __launch_bounds__(32 * kReduceWarps) k_gram_reduce(const double*
 // rotations to its 2 x 2 block.  The matrix is first scaled by a power of two to entries of at most
 // one.  CTAs 1 and 2 turn half of V's rows each, some rounds behind: a round's (c, s) go into their
 // shared memory (st.async), where a sweep's rounds have a place each, and the CTAs meet after each sweep.
+// Their waits are bounded: one that gives up makes the outputs NaN and the sweeps -1.
 //
 // What bounds it: a round's chain of some 20 dependent FP64 operations (16 cycles each, 45 for a
 // reciprocal square root), two barriers and the update's shared-memory accesses.  Measured for a POD
@@ -790,17 +791,18 @@ __global__ void __cluster_dims__(kJacCluster, 1, 1) __launch_bounds__(kJacThread
       JacPair own(min(pos, half - 1), kk);
       for (int round = 0; round < rounds; ++round) {
         const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&S.full[round]);
-        for (int spin = 0; !*(volatile int*)&S.bad; ++spin) {
-          uint32_t ok;
+        uint32_t ok = 0;
+        for (WaitLimit limit; !*(volatile int*)&S.bad;) {
           asm volatile(
               "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
               : "=r"(ok)
               : "r"(bar), "r"(sweep & 1)
               : "memory");
           if (ok) break;
-          if (spin > (1 << 22)) *(volatile int*)&S.bad = 1;   // seconds: V becomes NaN below
+          if (limit.over()) *(volatile int*)&S.bad = 1;   // the outputs become NaN and the sweeps -1 below
         }
-        if (tid == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(16 * half) : "memory");
+        if (tid == 0 && ok)   // this phase is over: the next sweep's
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(16 * half) : "memory");
         if (tid < 512 && pos < half) {
           const double2 cs = S.rot[round][pos];
           const int p = own.lo(), q = own.hi();
@@ -855,6 +857,13 @@ __global__ void __cluster_dims__(kJacCluster, 1, 1) __launch_bounds__(kJacThread
   jac_meet();
   if (cta != 0 && V) {
     const int row0 = (cta - 1) * kJacVRows;
+    if (S.bad) {   // behind CTA 0's own writes: the cluster has met since
+      // rotations not waited for may still be on their way into this CTA's memory: 0.1 ms for them
+      for (const long long t0 = clock64(); clock64() - t0 < 200000;) {
+      }
+      if (tid < k) w[tid] = __longlong_as_double(0x7ff8000000000000ll);
+      if (tid == 0 && sweeps_out) *sweeps_out = -1;
+    }
     for (int i = tid; i < kJacVRows * k; i += kJacThreads) {
       const int r = i / k, c = i % k;
       if (row0 + r < k)

@@ -24,21 +24,22 @@ import torch
 from .batched import block_pcg, panel_width
 from .device import ReducedOperator
 from .panel import block_spmm, panel_gram, panel_small
-from .pod import symeig
+from .pod import _check_symeig, _symeig
 
 
 def _generalized_eig(Kr, Mr):
     """Eigenpairs of Kr v = lambda Mr v (Kr, Mr symmetric, Mr positive definite), lambda ascending
-    and V^T Mr V = I."""
-    lm, Q = symeig(Mr)
+    and V^T Mr V = I, and the sweeps of the second eigensolve."""
+    lm, Q, sweeps = _symeig(Mr)
     if not bool((lm > 0).all()):
+        _check_symeig(sweeps)
         raise np.linalg.LinAlgError("solve_modal: the subspace lost rank (M-Gram matrix not positive definite)")
     S = Q * lm.rsqrt()[None, :]
     A = S.t() @ Kr @ S
     A = 0.5 * (A + A.t())
-    w, W = symeig(A)
+    w, W, sweeps = _symeig(A)
     order = torch.argsort(w)
-    return w[order], S @ W[:, order]
+    return w[order], S @ W[:, order], sweeps
 
 
 def subspace_iteration(Kop: ReducedOperator, Mop: ReducedOperator, n_modes, subspace=None, tol=1e-12, maxiter=300,
@@ -64,12 +65,14 @@ def subspace_iteration(Kop: ReducedOperator, Mop: ReducedOperator, n_modes, subs
         block_spmm(Mop, X, out=B)
         Y, res = block_pcg(Kop, np.array([0, n]), B, [p], tol=pcg_tol)
         if not (res.status == 0).all():
+            if it > 1:
+                _check_symeig(sweeps)     # X is NaN after a wait that timed out
             raise RuntimeError(f"solve_modal: the inner block-PCG did not converge (status {res.status.tolist()})")
         block_spmm(Kop, Y, out=KY)
         block_spmm(Mop, Y, out=MY)
         Kr = panel_gram(Y[:, :p], KY[:, :p])
         Mr = panel_gram(Y[:, :p], MY[:, :p])
-        lam, V = _generalized_eig(0.5 * (Kr + Kr.t()), 0.5 * (Mr + Mr.t()))
+        lam, V, sweeps = _generalized_eig(0.5 * (Kr + Kr.t()), 0.5 * (Mr + Mr.t()))
         X[:, :p] = panel_small(Y[:, :p], V)
         low = lam[:n_modes]
         if lam_old is not None:

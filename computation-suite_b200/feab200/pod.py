@@ -100,7 +100,13 @@ def gram_fp64(X, workspace=None):
 
 
 def symeig(G, vectors=True, max_sweeps=40):
-    """Eigenvalues (descending) and eigenvectors of a symmetric FP64 device matrix (k <= 64)."""
+    """Eigenvalues (descending) and eigenvectors of a symmetric FP64 device matrix (k <= 64).  Asynchronous:
+    all are NaN if a bounded wait timed out on the device (PodBasis.fit and solve_modal raise then)."""
+    return _symeig(G, vectors, max_sweeps)[:2]
+
+
+def _symeig(G, vectors=True, max_sweeps=40):
+    """symeig's results and the device int of the sweeps, -1 after a wait that timed out."""
     k = G.shape[0]
     A = G.contiguous().clone()
     w = torch.empty(k, dtype=torch.float64, device=G.device)
@@ -109,7 +115,12 @@ def symeig(G, vectors=True, max_sweeps=40):
     rc = L.lib.feab_symeig_jacobi(L.dptr(A), k, L.dptr(w), L.dptr(V), int(max_sweeps), L.dptr(sweeps),
                                   L.stream_ptr(G.device))
     L.raise_for(rc, "symeig_jacobi")
-    return w, V
+    return w, V, sweeps
+
+
+def _check_symeig(sweeps):
+    if int(sweeps.item()) < 0:
+        raise RuntimeError("symeig_jacobi: a bounded wait timed out on the device")
 
 
 def _select_rank(S, n_modes, energy_threshold):
@@ -158,9 +169,11 @@ class PodBasis:
             Xp = torch.zeros((n, MAX_SNAPSHOTS), dtype=dt, device=dev)
             Xp[:, :k] = X.to(dt)
         G = {"bf16x3": gram_bf16x3, "int8": gram_int8, "fp64": gram_fp64}[gram](Xp)
-        w, V = symeig(G)
+        w, V, sweeps = _symeig(G)
         S = torch.sqrt(torch.clamp(w[: min(k, n)], min=0.0))
         S_host = S.cpu().numpy()
+        if np.isnan(S_host).any():                           # NaN snapshots, or no result
+            _check_symeig(sweeps)
         r = _select_rank(S_host, n_modes, energy_threshold)
         Vk = V[:k, :r]                                       # eigenvectors of the k x k Gram block
         inv = torch.where(S[:r] > 0, 1.0 / S[:r], torch.zeros_like(S[:r]))

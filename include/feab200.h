@@ -450,9 +450,10 @@ int32_t feab_panel_small(const double* Y, int32_t ldy, int64_t n, int32_t k, con
 int32_t feab_panel_small_f32(const float* Y, int32_t ldy, int64_t n, int32_t k, const double* V, int32_t m, double* Z,
                              int32_t ldz, cudaStream_t stream);
 
-/* Cyclic Jacobi eigensolver (one CTA, FP64) for a symmetric k x k matrix (k <= 64) in device
+/* Cyclic Jacobi eigensolver (a cluster of three CTAs, FP64) for a symmetric k x k matrix (k <= 64) in device
  * memory: eigenvalues descending into evals, eigenvectors (columns) into evecs (may be NULL).
- * A may be overwritten.  *sweeps_out (device int, may be NULL) receives the sweeps used. */
+ * A may be overwritten.  *sweeps_out (device int, may be NULL) receives the sweeps used, or -1 when a
+ * bounded wait timed out (evals and evecs are NaN then).  Asynchronous. */
 int32_t feab_symeig_jacobi(double* A, int32_t k, double* evals, double* evecs, int32_t max_sweeps,
                            int32_t* sweeps_out, cudaStream_t stream);
 
