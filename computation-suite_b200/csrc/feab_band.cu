@@ -16,6 +16,7 @@
 // factors, in one kernel of one cluster (k_band_solve).
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include "feab_common.cuh"
 
@@ -95,8 +96,10 @@ struct BandState {
   int32_t status;
   int32_t bad;                          // assembly: an entry outside the band
   int32_t next_task, abort_flag;        // factorisation
+  int32_t solve_error;                  // of solves without an error flag of their own
 };
 static_assert(sizeof(BandState) <= FEAB_BAND_HEADER_BYTES, "band header");
+static_assert(offsetof(BandState, solve_error) == FEAB_BAND_ERROR_BYTE, "band header");
 
 // The factorisation is one cooperative kernel, so that a block column costs what its dependences
 // cost and not three launches.  CTA 0 walks the diagonal (the chain): for block row J it forms
@@ -675,8 +678,8 @@ __global__ void __launch_bounds__(kBandThreads, 1) k_band_factor(BandWork B) {
 // memory (bulk copies).
 // Vector q + 32 goes where vector q was: every CTA sends a vector between the two (it has a row among
 // any 16, and at most 31 vectors lie between its last row forward and its first backward), and it
-// has taken in all vectors before the one that it sends.  Every wait is bounded: a warp whose wait
-// runs out goes on without waiting, so that barriers stay matched, and sends NaN.
+// has taken in all vectors before the one that it sends.  Every wait is bounded: a CTA whose wait runs out
+// goes on without waiting, so that barriers stay matched, sends NaN and sets the solve's error flag.
 //
 // What bounds it: latency, 1.1 us per block row (two 64 x 64 products by 512 threads, each with its
 // reduction, and one hop to another SM), while a CTA's tiles per block row (bands / C) come in
@@ -711,28 +714,41 @@ __device__ __forceinline__ void mbar_expect(unsigned long long* m, uint32_t byte
 __device__ __forceinline__ void mbar_arrive(unsigned long long* m) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(m)) : "memory");
 }
+__device__ __forceinline__ bool mbar_done(unsigned long long* m, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(done)
+      : "r"(smem_u32(m)), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+
 __device__ __forceinline__ unsigned long long now_ns() {
   unsigned long long v;
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(v));
   return v;
 }
 constexpr unsigned long long kSolveLimitNs = 4000000000ull;
+constexpr int kSolveLate = 4096;                       // polls beyond it: the context may have been switched out
 
-// False when the phase does not end within kSolveLimitNs, or another wait of the CTA has given up.
+// False when the wait runs out, or another wait of the CTA has.  (A clock that leaves such time out, and telling
+// the other CTAs, each cost the wide bands 2 to 4 %: it is code in every wait.)
 __device__ __forceinline__ bool mbar_wait(unsigned long long* m, uint32_t parity, volatile int* abort_flag) {
   const uint32_t a = smem_u32(m);
   unsigned long long began = 0;
+  int late = 0;
   while (true) {
     uint32_t done;
     asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        "{\n .reg .pred p;\n " FEAB_MBAR_TRY ".parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
         : "=r"(done)
         : "r"(a), "r"(parity)
         : "memory");
     if (done) return true;
-    if (*abort_flag) return false;
+    if (*abort_flag || FEAB_WAIT_CYCLES == 0) break;
     if (began == 0) began = now_ns();
-    else if (now_ns() - began > kSolveLimitNs) break;
+    else if (now_ns() - began > kSolveLimitNs && ++late > kSolveLate) break;
   }
   *abort_flag = 1;
   return false;
@@ -747,6 +763,7 @@ struct SolveArgs {
   const double* inv;
   const double* b;
   double* x;      // y after the forward pass, then the solution
+  int32_t* error_flag;
   int32_t bands, n_tiles;
 };
 
@@ -848,6 +865,7 @@ __global__ void __launch_bounds__(kSolveCta, 1) k_band_solve(SolveArgs A) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   cluster_sync_all();
+  int issued = 0;   // tiles (the fetching thread)
   if (tid >= kSolveThreads) {
     // the tiles, each into the next free place of the ring
     if ((tid & 31) == 0) {
@@ -856,8 +874,10 @@ __global__ void __launch_bounds__(kSolveCta, 1) k_band_solve(SolveArgs A) {
       bool ok = true;
       solve_tiles(A, c, C, [&](const double* src) {
         if (!ok) return;
-        ok = mbar_wait(&S.empty[slot], phase ^ 1, abort_flag);
+        // a warp that gave up on a tile leaves its place all the same: the tile may still be on its way
+        ok = mbar_wait(&S.empty[slot], phase ^ 1, abort_flag) && !*abort_flag;
         if (!ok) return;
+        ++issued;
         mbar_expect(&S.full[slot], kTile * 8);
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                          smem_u32(S.ring[slot])),
@@ -1028,6 +1048,18 @@ __global__ void __launch_bounds__(kSolveCta, 1) k_band_solve(SolveArgs A) {
   }
   __syncwarp();
   cluster_sync_all();
+  if (*abort_flag) {
+    // what nobody waited for may still be on its way into this CTA's memory: the tiles, and 0.1 ms for vectors
+    for (int i = 0; i < kSolveRing; ++i) {
+      const int uses = issued / kSolveRing + (i < issued % kSolveRing ? 1 : 0);
+      DrainLimit limit;
+      while (uses > 0 && !mbar_done(&S.full[i], (uses - 1) & 1) && !limit.over()) {
+      }
+    }
+    for (const long long t0 = clock64(); clock64() - t0 < 200000;) {
+    }
+    if (tid == 0) *A.error_flag = 1;
+  }
 }
 
 // Wider bands than the cluster kernel's pending rows: one launch per block row.
@@ -1216,7 +1248,12 @@ extern "C" int32_t feab_band_cholesky(feab_band* B, double* pivots_out, cudaStre
 }
 
 extern "C" int32_t feab_band_solve(const feab_band* B, const double* b, double* x, double* work, cudaStream_t s) {
-  if (!band_ok(B) || !b || !x || !work || x == b || x == work || b == work) return FEAB_BAD_ARG;
+  return feab_band_solve_flag(B, b, x, work, B && B->storage ? &band_state(B)->solve_error : nullptr, s);
+}
+
+extern "C" int32_t feab_band_solve_flag(const feab_band* B, const double* b, double* x, double* work,
+                                        int32_t* error_flag, cudaStream_t s) {
+  if (!band_ok(B) || !b || !x || !work || !error_flag || x == b || x == work || b == work) return FEAB_BAD_ARG;
   const double* tiles = band_tiles(B);
   const double* inv = band_inv(B);
   const int NT = B->n_tiles, bands = B->bands;
@@ -1224,7 +1261,7 @@ extern "C" int32_t feab_band_solve(const feab_band* B, const double* b, double* 
   // CTA and block row.
   const int C = bands > 8 ? kSolveMaxCluster : 8, rows = (bands + C - 1) / C;
   if (rows <= kSolveMaxRows) {
-    SolveArgs A{tiles, inv, b, x, bands, NT};
+    SolveArgs A{tiles, inv, b, x, error_flag, bands, NT};
     const void* fn = rows <= 1 ? (const void*)k_band_solve<1> : rows <= 2 ? (const void*)k_band_solve<2>
                    : rows <= 4 ? (const void*)k_band_solve<4> : (const void*)k_band_solve<kSolveMaxRows>;
     FEAB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SolveShared)));

@@ -25,6 +25,11 @@
 #ifndef FEAB_WAIT_CYCLES
 #define FEAB_WAIT_CYCLES (1ll << 32)
 #endif
+#if FEAB_WAIT_CYCLES > 0
+#define FEAB_MBAR_TRY "mbarrier.try_wait"
+#else
+#define FEAB_MBAR_TRY "mbarrier.test_wait"
+#endif
 
 namespace feab {
 
@@ -77,18 +82,21 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double* sh) {
 // The end of a wait: one object per wait, over() after every poll that failed.  True once the wait has taken
 // some seconds of the SM's clock.  The clock is read every 64 polls, and a span counts a 64th of a second at
 // most: the time in which the context is switched out is not the wait's.
+template <long long CYCLES = FEAB_WAIT_CYCLES>
 struct WaitLimit {
-  static constexpr long long kCycles = FEAB_WAIT_CYCLES, kSpan = 1ll << 25;
+  static constexpr long long kSpan = 1ll << 25;
   long long last = 0, spent = 0;
   int polls = 0;
   __device__ __forceinline__ bool over() {
-    if ((++polls & 63) != 0 && kCycles > 0) return false;
+    if ((++polls & 63) != 0 && CYCLES > 0) return false;
     const long long now = clock64(), span = now - last;
     if (last != 0) spent += span >= 0 && span < kSpan ? span : kSpan;
     last = now;
-    return spent >= kCycles;
+    return spent >= CYCLES;
   }
 };
+// Before a CTA that gave up on a wait leaves: its own copies, whatever FEAB_WAIT_CYCLES.
+using DrainLimit = WaitLimit<(1ll << 32)>;
 
 // Number of SMs of the current device, cached per process.
 int sm_count();

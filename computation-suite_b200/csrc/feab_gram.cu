@@ -792,7 +792,7 @@ __global__ void __cluster_dims__(kJacCluster, 1, 1) __launch_bounds__(kJacThread
       for (int round = 0; round < rounds; ++round) {
         const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&S.full[round]);
         uint32_t ok = 0;
-        for (WaitLimit limit; !*(volatile int*)&S.bad;) {
+        for (WaitLimit<> limit; !*(volatile int*)&S.bad;) {
           asm volatile(
               "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
               : "=r"(ok)

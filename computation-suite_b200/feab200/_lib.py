@@ -148,6 +148,7 @@ SIGNATURES = {
     "feab_band_assemble": (_I32, [C.POINTER(CSR), _P, _I32, C.POINTER(Band), _P]),
     "feab_band_cholesky": (_I32, [C.POINTER(Band), C.POINTER(_D), _P]),
     "feab_band_solve": (_I32, [C.POINTER(Band), _P, _P, _P, _P]),
+    "feab_band_solve_flag": (_I32, [C.POINTER(Band), _P, _P, _P, _P, _P]),
 }
 
 

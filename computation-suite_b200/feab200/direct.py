@@ -181,6 +181,7 @@ class BandCholesky:
             raise np.linalg.LinAlgError("banded Cholesky: a pivot <= 0 -- K_ff is not SPD")
         L.raise_for(rc, "banded Cholesky")
         self.padded = int(self.band.n_tiles) * TILE
+        self._error = torch.zeros(1, dtype=torch.int32, pin_memory=True)     # set by a solve whose wait timed out
 
     @property
     def near_singular(self):
@@ -189,7 +190,9 @@ class BandCholesky:
         return not (lo >= PIVOT_TOL * hi)
 
     def solve(self, b):
-        """x = K_ff^{-1} b (b: (n,) host or device array; returns an FP64 device tensor)."""
+        """x = K_ff^{-1} b (b: (n,) host or device array; returns an FP64 device tensor).  Asynchronous.
+        Where a bounded wait times out on the device x is NaN, and check() or the next solve raises."""
+        self._raise_if_timed_out()
         op = self.op
         dev = op.vals64.device
         b = torch.as_tensor(b, dtype=torch.float64).to(dev).reshape(-1)
@@ -199,6 +202,17 @@ class BandCholesky:
         bp[self.iperm.long()] = b
         xp = torch.empty_like(bp)
         work = torch.empty_like(bp)
-        rc = L.lib.feab_band_solve(C.byref(self.band), L.dptr(bp), L.dptr(xp), L.dptr(work), L.stream_ptr(dev))
+        rc = L.lib.feab_band_solve_flag(C.byref(self.band), L.dptr(bp), L.dptr(xp), L.dptr(work), L.dptr(self._error),
+                                        L.stream_ptr(dev))
         L.raise_for(rc, "banded Cholesky solve")
         return xp[self.iperm.long()]
+
+    def check(self):
+        """Waits for the solves on the current stream; raises when a bounded wait of one timed out."""
+        torch.cuda.current_stream(self.op.vals64.device).synchronize()
+        self._raise_if_timed_out()
+
+    def _raise_if_timed_out(self):
+        if int(self._error[0]):
+            self._error.zero_()
+            L.raise_for(L.FEAB_CUDA_ERROR, "banded Cholesky solve: a bounded wait timed out on the device")

@@ -504,6 +504,8 @@ class FESystem:
         x = fac.solve(b)
         bn = float(torch.linalg.norm(b)) or 1.0
         rel = float(torch.linalg.norm(b - spmv(op, x, lanes_per_group=16))) / bn
+        if rel != rel:               # NaN in the load, or no result
+            fac.check()
         return x, SolveInfo(L.FEAB_OK, 0, 0, rel, bn, "direct")
 
     def _rigid_null_space(self, device):

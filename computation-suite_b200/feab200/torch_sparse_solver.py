@@ -89,7 +89,7 @@ def fesystem_solve_static_torch(sysobj, method="cg", device="cpu", tol=1e-8, max
     else:
         # a direct solve, as the reference's torch_dense_solve: the banded Cholesky of K_ff
         # (feab200.direct); a K_ff that is not SPD, or singular, goes to a tight PCG instead
-        x = None
+        x = fac = None
         try:
             fac = op.direct_factor(coords=getattr(sysobj.mesh, "nodes", None))
             if not fac.near_singular:
@@ -102,6 +102,8 @@ def fesystem_solve_static_torch(sysobj, method="cg", device="cpu", tol=1e-8, max
                 raise RuntimeError("fesystem_solve_static_torch: method='dense' found K_ff not SPD or singular, "
                                    "and the tight PCG it falls back to did not converge")
             L.raise_for(info.status, "fesystem_solve_static_torch")
+        else:
+            fac.check()
         U[free] = x.cpu().numpy()
         return U
     L.raise_for(info.status, "fesystem_solve_static_torch")

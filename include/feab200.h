@@ -584,6 +584,13 @@ int32_t feab_band_cholesky(feab_band* B, double* pivots_out, cudaStream_t stream
  * memory; the entries of b past n must be 0, and those of x past n are 0).  Asynchronous. */
 int32_t feab_band_solve(const feab_band* B, const double* b, double* x, double* work, cudaStream_t stream);
 
+/* The same with an error flag of its own (an int32 that the device can write, pinned host memory
+ * included; zero it first), set if a bounded wait timed out: x is NaN then.  feab_band_solve sets the int32
+ * at byte FEAB_BAND_ERROR_BYTE of the storage, which the factorisation clears.  Asynchronous. */
+#define FEAB_BAND_ERROR_BYTE 32
+int32_t feab_band_solve_flag(const feab_band* B, const double* b, double* x, double* work, int32_t* error_flag,
+                             cudaStream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -37,3 +37,51 @@ def test_eigensolver(tmp_path, monkeypatch):
         PodBasis().fit(torch.as_tensor(rng.standard_normal((500, 64))).cuda(), n_modes=3)
     monkeypatch.undo()
     assert PodBasis().fit(torch.as_tensor(rng.standard_normal((500, 64))).cuda(), n_modes=3).V.shape == (500, 3)
+
+
+@pytest.mark.parametrize("shape", [(6, 2, 2), (24, 8, 8), (40, 12, 12)])
+def test_band_solve(tmp_path, monkeypatch, shape):
+    """Bands of 1, 5 and 9 tiles: clusters of 8 and of 16 CTAs."""
+    import ctypes as C
+    import feab200
+    from feab200 import _lib as L
+    from feab200 import torch_sparse_solver as ts
+    lib = wait_limits.build(tmp_path, "feab_band.cu")
+    if lib is None:
+        pytest.skip("no nvcc")
+    _declare(lib, "feab_band_solve", "feab_band_solve_flag")
+    mesh = feab200.box_mesh(2.0, 0.4, 0.4, *shape)
+    fs = feab200.FESystem(mesh, feab200.Hex8Solid3D(), sparse=True)
+    fs.assemble_stiffness(feab200.D_solid3d(feab200.Material(E=1.0, nu=0.3)), vectorized=True)
+    fs.fix_dofs(mesh.nodes_on_plane(0, 0.0), (0, 1, 2))
+    fs.add_nodal_force(mesh.nodes_on_plane(0, 2.0), 2, 1.0)
+    want = np.asarray(fs.solve_static())
+    fac = fs.reduced_operator(want32=False).direct_factor(coords=mesh.nodes)
+    st = L.stream_ptr(torch.device("cuda"))
+    b = torch.ones(fac.op.n, dtype=torch.float64, device="cuda")
+    x = fac.solve(b)
+    fac.check()
+    with monkeypatch.context() as m:
+        m.setattr(L.lib, "feab_band_solve_flag", lib.feab_band_solve_flag)
+        assert bool(fac.solve(b).isnan().any())
+        with pytest.raises(L.FeabError, match="timed out"):
+            fac.check()
+        fac.check()                                                # said once
+        fac.solve(b)
+        torch.cuda.synchronize()
+        with pytest.raises(L.FeabError, match="timed out"):
+            fac.solve(b)
+        with pytest.raises(L.FeabError, match="timed out"):
+            fs.solve_static()
+        with pytest.raises(L.FeabError, match="timed out"):
+            ts.fesystem_solve_static_torch(fs, method="dense")
+    # without a flag of its own a solve sets the header's
+    header = fac.storage[32:36].view(torch.int32)
+    bp = torch.zeros(fac.padded, dtype=torch.float64, device="cuda")
+    bp[:fac.op.n] = 1.0
+    xp, work = torch.empty_like(bp), torch.empty_like(bp)
+    for fn, flag in ((L.lib.feab_band_solve, 0), (lib.feab_band_solve, 1)):
+        assert fn(C.byref(fac.band), L.dptr(bp), L.dptr(xp), L.dptr(work), st) == L.FEAB_OK
+        assert int(header) == flag and bool(xp.isnan().any()) == bool(flag)
+    assert torch.equal(fac.solve(b), x)
+    assert np.array_equal(np.asarray(fs.solve_static()), want)
