@@ -1062,7 +1062,7 @@ __global__ void __launch_bounds__(kSolveCta, 1) k_band_solve(SolveArgs A) {
   }
 }
 
-// Wider bands than the cluster kernel's pending rows: one launch per block row.
+// Wider bands than the cluster kernel's pending rows, or no place for the cluster: one launch per block row.
 // Forward step K of L y = b: every CTA forms y_K = Linv_KK w_K (two threads per row), CTA 0 writes
 // it, and CTA i < n_below applies tile (K + 1 + i, i + 1): w_{K+1+i} -= L_{K+1+i,K} y_K.
 __global__ void __launch_bounds__(128) k_band_fwd(const double* __restrict__ tiles, const double* __restrict__ inv,
@@ -1226,10 +1226,19 @@ extern "C" int32_t feab_band_cholesky(feab_band* B, double* pivots_out, cudaStre
   int resident = 0;
   FEAB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_band_factor, kBandThreads, kFactorSmem));
   const int64_t tasks = B->bands >= 2 ? (int64_t)B->n_tiles * (B->bands + 1) : 0;
-  const int grid = (int)std::min<int64_t>((int64_t)sm_count() * std::min(resident, 1), 1 + tasks);
-  if (grid < (tasks > 0 ? 2 : 1)) return FEAB_CUDA_ERROR;
+  int grid = (int)std::min<int64_t>((int64_t)sm_count() * std::min(resident, 1), 1 + tasks);
+  const int least = tasks > 0 ? 2 : 1;
+  if (grid < least) return FEAB_CUDA_ERROR;
   void* args[1] = {&W};
-  FEAB_CUDA(cudaLaunchCooperativeKernel((const void*)k_band_factor, dim3(grid), dim3(kBandThreads), args, kFactorSmem, s));
+  // a context with fewer SMs at hand than the device has: any number of workers does
+  cudaError_t e;
+  while ((e = cudaLaunchCooperativeKernel((const void*)k_band_factor, dim3(grid), dim3(kBandThreads), args, kFactorSmem,
+                                          s)) == cudaErrorCooperativeLaunchTooLarge &&
+         grid > least) {
+    cudaGetLastError();
+    grid = std::max(least, grid / 2);
+  }
+  FEAB_CUDA(e);
   count_launches(1);
   FEAB_CHECK_LAUNCH();
   if (flag_bytes) FEAB_CUDA(cudaMemsetAsync(band_flags(B), 0, flag_bytes, s));   // left as it was
@@ -1264,8 +1273,6 @@ extern "C" int32_t feab_band_solve_flag(const feab_band* B, const double* b, dou
     SolveArgs A{tiles, inv, b, x, error_flag, bands, NT};
     const void* fn = rows <= 1 ? (const void*)k_band_solve<1> : rows <= 2 ? (const void*)k_band_solve<2>
                    : rows <= 4 ? (const void*)k_band_solve<4> : (const void*)k_band_solve<kSolveMaxRows>;
-    FEAB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SolveShared)));
-    FEAB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(C);
     cfg.blockDim = dim3(kSolveCta);
@@ -1278,9 +1285,14 @@ extern "C" int32_t feab_band_solve_flag(const feab_band* B, const double* b, dou
     cfg.attrs = at;
     cfg.numAttrs = 1;
     void* args[1] = {&A};
-    FEAB_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
-    count_launches(1);
-    return FEAB_OK;
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SolveShared));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaLaunchKernelExC(&cfg, fn, args);
+    if (e == cudaSuccess) {
+      count_launches(1);
+      return FEAB_OK;
+    }
+    cudaGetLastError();   // the cluster has no place (a part of a device): a launch per block row needs none
   }
   const size_t bytes = (size_t)NT * kT * sizeof(double);
   // forward: work = b, updated in place; y into x
