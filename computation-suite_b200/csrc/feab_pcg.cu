@@ -1054,8 +1054,10 @@ int sell_grid(const PcgArgs& A) {
   return std::max(1, std::min((A.sell.n_slices + wpb - 1) / wpb, max_grid()));
 }
 
-// The ring takes operators with 2-byte columns whose arrays start on the bulk copies' 16 bytes.
+// The ring takes operators with 2-byte columns whose arrays start on the bulk copies' 16 bytes, and a direction
+// that k_step_p has formed.
 bool sell_ring(const PcgArgs& A, int prec) {
+  if (FEAB_SELL_FUSED_P) return false;
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
   const SellView& V = A.sell;
   return V.tcol16 && al(V.tcol16) && (prec == FEAB_PREC_FP64 ? al(V.v64) : al(V.vhi) && al(V.vlo));

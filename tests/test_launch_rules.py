@@ -41,7 +41,7 @@ static cudaError_t fake_ex(const cudaLaunchConfig_t* c, const void*, void**) {
 """
 
 
-def _run(tmp_path, source, main):
+def _run(tmp_path, source, main, *flags):
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(nvcc):
         pytest.skip("no nvcc")
@@ -49,7 +49,7 @@ def _run(tmp_path, source, main):
     with open(src, "w") as fh:
         fh.write(FAKES + f'#include "{source}"\n' + main)
     subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=compute_100a", "-std=c++17", "--expt-relaxed-constexpr",
-                    "-I", os.path.join(ROOT, "include"), "-I", CSRC, src, "-o", exe], check=True, capture_output=True)
+                    "-I", os.path.join(ROOT, "include"), "-I", CSRC, *flags, src, "-o", exe], check=True, capture_output=True)
     # no device is visible: a launch that is not replaced ends on the host
     out = subprocess.run([exe], check=True, capture_output=True, text=True, env=dict(os.environ, CUDA_VISIBLE_DEVICES=""))
     return [[int(v) for v in line.split()] for line in out.stdout.splitlines()]
@@ -89,3 +89,24 @@ def test_band_factor_and_solve_on_a_part_of_a_device(tmp_path):
         # one cluster kernel, and a launch per block row and direction where it is refused or too wide
         assert rows[4] == ([0, 1, 1] if bands <= 128 else [0, 0, 600]), bands
         assert rows[5] == ([0, 1, 600] if bands <= 128 else [0, 0, 600]), bands
+
+
+@pytest.mark.parametrize("fused", [0, 1])
+def test_step_kernel_of_the_sliced_operator(tmp_path, fused):
+    """The direction formed inside step A's gathers (a build option) is not one that the ring can take."""
+    out = _run(tmp_path, "feab_pcg.cu", """
+    int main() {
+      using namespace feab;
+      char* at = (char*)aligned_alloc(256, 4096);
+      for (int off : {0, 2}) {
+        PcgArgs A{};
+        A.sell.tcol16 = (const int16_t*)(at + off);
+        A.sell.v64 = (double*)at;
+        A.sell.vhi = (uint32_t*)at;
+        A.sell.vlo = (uint16_t*)at;
+        printf("%d %d\\n", (int)sell_ring(A, FEAB_PREC_FP64), (int)sell_ring(A, FEAB_PREC_MIXED));
+      }
+      exit(0);
+    }
+    """, f"-DFEAB_SELL_FUSED_P={fused}", "-Xlinker", "--unresolved-symbols=ignore-all", "-Xcicc", "-O0")
+    assert out == [[1 - fused, 1 - fused], [0, 0]]
