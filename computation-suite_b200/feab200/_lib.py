@@ -7,6 +7,8 @@ reference raises for the same condition.
 from __future__ import annotations
 
 import ctypes as C
+import functools
+import hashlib
 import os
 
 import numpy as np
@@ -166,6 +168,13 @@ def _load():
 
 
 lib = _load()
+
+
+@functools.lru_cache(maxsize=None)
+def build_id(path=LIB_PATH):
+    """A name of the library's build: what was measured with another one does not hold for it."""
+    with open(path, "rb") as fh:
+        return hashlib.file_digest(fh, "sha256").hexdigest()[:16]
 
 
 def status_string(code):

@@ -204,7 +204,10 @@ def tuning_cache_path():
 
 
 def tuning_key(device_name, n, nnz, n_problems, k, precision):
-    return f"{device_name}|n={n}|nnz={nnz}|problems={n_problems}|k={k}|{precision}|spmm=tiles{TILE_GROUPS}p"
+    """What a tuned shape holds for: this shape of operator and panel, on this GPU, with this build of the
+    kernels (a shape tuned for another build's would be used without having been timed)."""
+    return (f"{device_name}|n={n}|nnz={nnz}|problems={n_problems}|k={k}|{precision}|spmm=tiles{TILE_GROUPS}|"
+            f"build={L.build_id()}")
 
 
 def load_tuning(path=None):
@@ -267,7 +270,7 @@ def tuned_block_shape(op, row_bounds, B_panel, cols, precision="fp64", candidate
     and right-hand sides over ITEM_GROUPS x {panel widths <= K} x {node tiles, row groups}; a
     tile narrower than K costs K / width tile steps.
     Cached in this process and in the JSON file of tuning_cache_path(), keyed by (GPU, n, nnz,
-    problems, K, precision)."""
+    problems, K, precision, build of the library)."""
     n, K = B_panel.shape
     P = len(row_bounds) - 1
     dev = op.vals64.device

@@ -172,6 +172,27 @@ def test_reference_arm_runs_whole_steps_without_the_cuda_library():
     assert set(line["config"]) == {"workload", "n_free", "nnz", "tol", "l2", "parallelism"}
 
 
+def test_block_tuning_of_another_build_is_not_taken(tmp_path, monkeypatch):
+    """A shape that was timed with other kernels is in the cache file under a key of its own."""
+    from feab200 import _lib
+    from feab200 import batched as bt
+    shape = ("NVIDIA B200", 418176, 32348142, 1, 64, "fp64")
+    keys = set()
+    for content in (b"one build", b"another build"):
+        lib = tmp_path / f"lib{len(content)}.so"
+        lib.write_bytes(content)
+        build = _lib.build_id(str(lib))
+        with monkeypatch.context() as m:
+            m.setattr(_lib, "build_id", lambda: build)
+            keys.add(bt.tuning_key(*shape))
+    keys.add(bt.tuning_key(*shape))
+    assert len(keys) == 3
+    path = str(tmp_path / "tuning.json")
+    for k in keys:
+        bt.save_tuning(k, bt.BlockShape(32, 64, 512.5), path)
+    assert set(bt.load_tuning(path)) == keys and bt.tuning_key(*shape) in keys
+
+
 def test_block_tuning_cache_round_trip(tmp_path):
     from feab200 import batched as bt
     path = str(tmp_path / "sub" / "tuning.json")
