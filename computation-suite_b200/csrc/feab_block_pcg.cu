@@ -1532,7 +1532,7 @@ int32_t run_block(BArgs A, int prec, int chunk, int maxiter, cudaStream_t s, int
     if (fail(cudaFuncSetAttribute(k_bstep_a<K, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)kStageBytes)))
       break;
-    if constexpr (K >= 8) {
+    if constexpr (K >= kPairPanel) {
       if (fail(cudaFuncSetAttribute(k_bstep_a_pairs<K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem)))
         break;
       if (fail(cudaFuncSetAttribute(k_bstep_a_pairs<K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem)))
@@ -1541,13 +1541,13 @@ int32_t run_block(BArgs A, int prec, int chunk, int maxiter, cudaStream_t s, int
     auto record = [&](cudaStream_t cs) {
       for (int q = 0; q < chunk; ++q) {
         k_bstep_p<K, false><<<grid_pb, kThreads, 0, cs>>>(A);
-        if constexpr (K >= 8) {
+        if constexpr (K >= kPairPanel) {
           if (A.pairs.off) {
             if (prec == FEAB_PREC_MIXED) k_bstep_a_pairs<K, true><<<grid, kThreads, kPairSmem, cs>>>(A);
             else k_bstep_a_pairs<K, false><<<grid, kThreads, kPairSmem, cs>>>(A);
           }
         }
-        const bool pairs = K >= 8 && A.pairs.off;
+        const bool pairs = K >= kPairPanel && A.pairs.off;
         if (prec == FEAB_PREC_MIXED) {
           if (pairs) {
           } else if (tiles) k_bstep_a<K, true, true><<<grid, kThreads, smem_a, cs>>>(A);

@@ -11,6 +11,11 @@
 
 namespace feab {
 
+// The least panel width that is multiplied through pair records: a tile of mma.sync.m8n8k4 is 8 columns.  The
+// records take 27 steps of 208 bytes per pair of nodes of a structured mesh, 2.8 KB per node beside the 1.9 KB
+// of its CSR values, and are not made for narrower panels.
+constexpr int kPairPanel = 8;
+
 struct __align__(16) PairRecord {
   double val[24];
   int32_t col[4];

@@ -13,8 +13,8 @@
 //   5. (build) one warp per group: each list entry finds its mask (binary searches in the tile's
 //      lists), its mask's run and its column there, and writes its rows' values at
 //      3 * (poff + upair + rank of the group among the mask's set bits) + row;
-//   6. (build) one warp per pair of a tile's groups (0, 1 and 2, 3): the pair records that the
-//      block-PCG's SpMM feeds to the FP64 tensor path (feab_pair.cuh).
+//   6. (build, for panels of kPairPanel columns or more) one warp per pair of a tile's groups (0, 1 and
+//      2, 3): the pair records that the block-PCG's SpMM feeds to the FP64 tensor path (feab_pair.cuh).
 #include <algorithm>
 #include <climits>
 #include "feab_common.cuh"
@@ -394,7 +394,7 @@ TileScratch scratch_layout(int32_t G, int32_t P, char* base) {
 }
 
 // Storage layout of the operator for n_tiles tiles, nu union columns, np (column, group) pairs and ns
-// steps of pair records.
+// steps of pair records (negative: none are kept).
 size_t storage_layout(int32_t n_tiles, int32_t G, int64_t nu, int64_t np, int64_t nch, int64_t ns, int prec,
                       char* base, feab_tile_operator* T) {
   size_t off = 0;
@@ -422,9 +422,9 @@ size_t storage_layout(int32_t n_tiles, int32_t G, int64_t nu, int64_t np, int64_
     lo2 = take(nv);
   }
   const size_t pairs = off;
-  take(pair_section_bytes(n_tiles, ns));
+  if (ns >= 0) take(pair_section_bytes(n_tiles, ns));
   if (T) {
-    T->reserved = (int32_t)(pairs / 256);   // see pair_view()
+    T->reserved = ns >= 0 ? (int32_t)(pairs / 256) : 0;   // see pair_view()
     T->tile_g0 = reinterpret_cast<int32_t*>(tg);
     T->group_tile = reinterpret_cast<int32_t*>(gt);
     T->uoff = reinterpret_cast<int32_t*>(uo);
@@ -456,10 +456,18 @@ extern "C" int32_t feab_tile_operator_build(const feab_csr* M, const feab_diff_o
                                             const int32_t* problem_groups, int32_t P, int32_t prec, void* scratch,
                                             size_t scratch_bytes, void* storage, size_t storage_bytes,
                                             size_t* bytes_out, feab_tile_operator* out, cudaStream_t s) {
+  return feab_tile_operator_build_k(M, D, problem_groups, P, prec, kPairPanel, scratch, scratch_bytes, storage,
+                                    storage_bytes, bytes_out, out, s);
+}
+
+extern "C" int32_t feab_tile_operator_build_k(const feab_csr* M, const feab_diff_operator* D,
+                                              const int32_t* problem_groups, int32_t P, int32_t prec, int32_t k,
+                                              void* scratch, size_t scratch_bytes, void* storage, size_t storage_bytes,
+                                              size_t* bytes_out, feab_tile_operator* out, cudaStream_t s) {
   if (!M || !problem_groups || P <= 0 || !scratch || !M->group_ptr || M->n_groups <= 0 || !M->row_ptr ||
       !M->col_idx || !M->vals64)
     return FEAB_BAD_ARG;
-  if (prec != FEAB_PREC_FP64 && prec != FEAB_PREC_MIXED) return FEAB_BAD_ARG;
+  if ((prec != FEAB_PREC_FP64 && prec != FEAB_PREC_MIXED) || k < 1) return FEAB_BAD_ARG;
   if (prec == FEAB_PREC_MIXED && (!D || !D->tcol || !D->goff || !D->voff || !D->vhi || !D->vlo || !D->vlo2))
     return FEAB_BAD_ARG;
   if (storage && (!out || (reinterpret_cast<uintptr_t>(storage) & 15u))) return FEAB_BAD_ARG;
@@ -502,14 +510,16 @@ extern "C" int32_t feab_tile_operator_build(const feab_csr* M, const feab_diff_o
   FEAB_CUDA(cudaStreamSynchronize(s));
   if (nu >= (int64_t)INT32_MAX || 3 * np >= (int64_t)INT32_MAX) return FEAB_CAPACITY;
   const int pw = kThreads / 32, pair_blocks = (2 * n_tiles + pw - 1) / pw;
-  k_pairs<<<pair_blocks, kThreads, 0, s>>>(2 * n_tiles, M->group_ptr, M->row_ptr, M->col_idx, M->vals64, X.tg0, X.scnt,
-                                           nullptr, nullptr);
-  count_launches(1);
-  FEAB_CHECK_LAUNCH();
-  int64_t ns = 0;
-  FEAB_CUDA(scan_exclusive_i32(X.scnt, X.scnt, 2 * (int64_t)n_tiles, X.scan, X.total, s));
-  FEAB_CUDA(cudaMemcpyAsync(&ns, X.total, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-  FEAB_CUDA(cudaStreamSynchronize(s));
+  int64_t ns = -1;
+  if (k >= kPairPanel) {
+    k_pairs<<<pair_blocks, kThreads, 0, s>>>(2 * n_tiles, M->group_ptr, M->row_ptr, M->col_idx, M->vals64, X.tg0, X.scnt,
+                                             nullptr, nullptr);
+    count_launches(1);
+    FEAB_CHECK_LAUNCH();
+    FEAB_CUDA(scan_exclusive_i32(X.scnt, X.scnt, 2 * (int64_t)n_tiles, X.scan, X.total, s));
+    FEAB_CUDA(cudaMemcpyAsync(&ns, X.total, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    FEAB_CUDA(cudaStreamSynchronize(s));
+  }
   const size_t need = storage_layout(n_tiles, G, nu, np, nch, ns, prec, nullptr, nullptr);
   if (bytes_out) *bytes_out = need;
   if (!storage) return FEAB_OK;
@@ -531,12 +541,14 @@ extern "C" int32_t feab_tile_operator_build(const feab_csr* M, const feab_diff_o
       G, Ls, M->vals64, D ? D->vhi : nullptr, D ? D->vlo : nullptr, D ? D->vlo2 : nullptr, D ? D->voff : nullptr,
       T.tile_g0, T.group_tile, T.uoff, T.poff, T.ucol, T.umask, T.upair, T.v64, T.vhi, T.vlo, T.vlo2, X.err);
   const PairView V = pair_view(&T);
-  FEAB_CUDA(cudaMemcpyAsync(const_cast<int32_t*>(V.off), X.scnt, sizeof(int32_t) * (2 * (size_t)n_tiles + 1),
-                            cudaMemcpyDeviceToDevice, s));
-  FEAB_CUDA(cudaMemsetAsync(const_cast<PairRecord*>(V.rec), 0, sizeof(PairRecord) * (size_t)ns, s));
-  k_pairs<<<pair_blocks, kThreads, 0, s>>>(2 * n_tiles, M->group_ptr, M->row_ptr, M->col_idx, M->vals64, T.tile_g0, nullptr,
-                                           V.off, const_cast<PairRecord*>(V.rec));
-  count_launches(4);
+  if (V.off) {
+    FEAB_CUDA(cudaMemcpyAsync(const_cast<int32_t*>(V.off), X.scnt, sizeof(int32_t) * (2 * (size_t)n_tiles + 1),
+                              cudaMemcpyDeviceToDevice, s));
+    FEAB_CUDA(cudaMemsetAsync(const_cast<PairRecord*>(V.rec), 0, sizeof(PairRecord) * (size_t)ns, s));
+    k_pairs<<<pair_blocks, kThreads, 0, s>>>(2 * n_tiles, M->group_ptr, M->row_ptr, M->col_idx, M->vals64, T.tile_g0,
+                                             nullptr, V.off, const_cast<PairRecord*>(V.rec));
+  }
+  count_launches(V.off ? 4 : 3);
   FEAB_CHECK_LAUNCH();
   FEAB_CUDA(cudaMemcpyAsync(&err, X.err, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
   FEAB_CUDA(cudaStreamSynchronize(s));

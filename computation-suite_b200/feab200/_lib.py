@@ -62,6 +62,7 @@ class TileOperator(C.Structure):
 
 
 TILE_GROUPS = 4   # FEAB_TILE_GROUPS: node row groups per tile of the block SpMM
+PAIR_PANEL = 8    # the least block-PCG panel width that runs on a tile operator's pair records
 
 
 class Batch(C.Structure):
@@ -123,6 +124,8 @@ SIGNATURES = {
     "feab_tile_scratch_bytes": (_SZ, [_I32, _I32]),
     "feab_tile_operator_build": (_I32, [C.POINTER(CSR), C.POINTER(DiffOperator), _P, _I32, _I32, _P, _SZ, _P, _SZ,
                                         C.POINTER(_SZ), C.POINTER(TileOperator), _P]),
+    "feab_tile_operator_build_k": (_I32, [C.POINTER(CSR), C.POINTER(DiffOperator), _P, _I32, _I32, _I32, _P, _SZ, _P,
+                                          _SZ, C.POINTER(C.c_size_t), C.POINTER(TileOperator), _P]),
     "feab_block_pcg_solve": (_I32, [C.POINTER(CSR), C.POINTER(DiffOperator), C.POINTER(TileOperator),
                                     C.POINTER(Batch), _P, _P, _P, C.POINTER(PcgParams), _P, _SZ, C.POINTER(_I32),
                                     C.POINTER(_D), C.POINTER(_I32), _P]),

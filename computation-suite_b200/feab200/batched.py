@@ -108,7 +108,7 @@ def _block_pcg_call(op, item_problem, g0, g1, prob_items, B_panel, cols, tol, ma
     B_panel = B_panel.to(dev, torch.float64).contiguous()
     prec = L.PREC_MIXED if precision == "mixed" else L.PREC_FP64
     diff = C.byref(op.diff_operator()) if precision == "mixed" else None
-    tiles = C.byref(op.tile_operator(precision, problem_groups)) if problem_groups is not None else None
+    tiles = C.byref(op.tile_operator(precision, problem_groups, K)) if problem_groups is not None else None
     params = L.PcgParams(float(tol), int(maxiter or 0), prec, float(reliable_delta), int(chunk), 1, 0, 0)
     iters = np.zeros(P * K, np.int32)
     relres = np.zeros(P * K, np.float64)

@@ -109,38 +109,52 @@ class ReducedOperator:
             self._diff = (storage, d)
         return self._diff[1]
 
-    def tile_operator(self, precision="fp64", problem_groups=None):
-        """Node tiles of the block SpMM (feab_tile_operator_build): FEAB_TILE_GROUPS consecutive
+    def tile_operator(self, precision="fp64", problem_groups=None, panel=1):
+        """Node tiles of the block SpMM (feab_tile_operator_build_k): FEAB_TILE_GROUPS consecutive
         row groups whose column lists are merged, with "fp64" (CSR) or "mixed" (difference-form,
         44-bit) values.  Tiles never cross the boundaries in problem_groups (the first row group
-        of each problem, then n_groups; default one problem).  Cached per (precision, boundaries)."""
+        of each problem, then n_groups; default one problem).  panel: the widest block-PCG panel that
+        it is for; from PAIR_PANEL columns on it also holds the pair records, unless the device has no
+        room for them.  Cached per (precision, boundaries, records)."""
         if precision not in ("fp64", "mixed"):
             raise ValueError("the tile operator holds 'fp64' or 'mixed' values")
         p = self.pattern
         if p.group_ptr is None:
             raise ValueError("the tile operator needs node row groups (an assembled K_ff)")
         pg = np.asarray([0, p.n_groups] if problem_groups is None else problem_groups, dtype=np.int32)
-        key = (precision, pg.tobytes())
+        plain = (precision, pg.tobytes())
+        wide = plain + ("pairs",)
         if self._tiles is None:
             self._tiles = {}
+        # an operator with the records serves narrow panels too
+        key = wide if panel >= L.PAIR_PANEL or (wide in self._tiles and plain not in self._tiles) else plain
         if key not in self._tiles:
-            dev = self.vals64.device
-            pg_t = torch.as_tensor(pg).to(dev)
-            n_prob = len(pg) - 1
-            diff = C.byref(self.diff_operator()) if precision == "mixed" else None
-            sbytes = int(L.lib.feab_tile_scratch_bytes(p.n_groups, n_prob))
-            scratch = torch.empty(max(sbytes, 1), dtype=torch.uint8, device=dev)
-            csr = self.csr_struct()
-            need = C.c_size_t(0)
-            args = (C.byref(csr), diff, L.dptr(pg_t), n_prob, PRECISIONS[precision], L.dptr(scratch), sbytes)
-            L.raise_for(L.lib.feab_tile_operator_build(*args, None, 0, C.byref(need), None, L.stream_ptr(dev)),
-                        "tile operator")
-            storage = torch.empty(need.value, dtype=torch.uint8, device=dev)
-            t = L.TileOperator()
-            L.raise_for(L.lib.feab_tile_operator_build(*args, L.dptr(storage), need.value, None, C.byref(t),
-                                                       L.stream_ptr(dev)), "tile operator")
-            self._tiles[key] = (storage, t)
+            try:
+                self._tiles[key] = self._build_tiles(precision, pg, L.PAIR_PANEL if key == wide else 1)
+            except torch.OutOfMemoryError:
+                if key == plain:
+                    raise
+                self._tiles[wide] = self._tiles[plain] if plain in self._tiles else self._build_tiles(precision, pg, 1)
         return self._tiles[key][1]
+
+    def _build_tiles(self, precision, pg, k):
+        p = self.pattern
+        dev = self.vals64.device
+        pg_t = torch.as_tensor(pg).to(dev)
+        n_prob = len(pg) - 1
+        diff = C.byref(self.diff_operator()) if precision == "mixed" else None
+        sbytes = int(L.lib.feab_tile_scratch_bytes(p.n_groups, n_prob))
+        scratch = torch.empty(max(sbytes, 1), dtype=torch.uint8, device=dev)
+        csr = self.csr_struct()
+        need = C.c_size_t(0)
+        args = (C.byref(csr), diff, L.dptr(pg_t), n_prob, PRECISIONS[precision], k, L.dptr(scratch), sbytes)
+        L.raise_for(L.lib.feab_tile_operator_build_k(*args, None, 0, C.byref(need), None, L.stream_ptr(dev)),
+                    "tile operator")
+        storage = torch.empty(need.value, dtype=torch.uint8, device=dev)
+        t = L.TileOperator()
+        L.raise_for(L.lib.feab_tile_operator_build_k(*args, L.dptr(storage), need.value, None, C.byref(t),
+                                                     L.stream_ptr(dev)), "tile operator")
+        return storage, t
 
     def max_row_len(self):
         rp = self.pattern.row_ptr

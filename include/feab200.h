@@ -382,6 +382,14 @@ int32_t feab_tile_operator_build(const feab_csr* A, const feab_diff_operator* di
                                  void* storage, size_t storage_bytes, size_t* bytes_out, feab_tile_operator* out,
                                  cudaStream_t stream);
 
+/* The same for block-PCG panels of up to k columns: below 8 columns without the pair records, which only
+ * wider panels use (2.8 KB per node of a structured mesh, 1.5 times the CSR's FP64 values).
+ * feab_tile_operator_build makes them.  Without them panels of any width run on the other arrays. */
+int32_t feab_tile_operator_build_k(const feab_csr* A, const feab_diff_operator* diff, const int32_t* problem_groups,
+                                   int32_t n_problems, int32_t precision, int32_t k, void* scratch,
+                                   size_t scratch_bytes, void* storage, size_t storage_bytes, size_t* bytes_out,
+                                   feab_tile_operator* out, cudaStream_t stream);
+
 /* tiles (optional, of the solve's precision, built with this batch's problem boundaries): the
  * SpMM of every CG step walks node tiles instead of single row groups; work items must then
  * start and end on tile boundaries (items of a multiple of FEAB_TILE_GROUPS groups from each

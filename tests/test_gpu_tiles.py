@@ -186,3 +186,53 @@ def test_tile_operator_rejects_bad_problem_boundaries():
     for pg in ([0, G // 2, G // 2, G], [1, G], [0, G - 1]):
         with pytest.raises(ValueError):
             op.tile_operator("fp64", pg)
+
+
+def _solve(b, B, precision, **kw):
+    from feab200.batched import block_pcg
+    X, r = block_pcg(b.op, b.row_bounds, B, np.minimum(b.cols, B.shape[1]), tol=1e-10, precision=precision, max_groups=8,
+                     tile_width=B.shape[1], tune=False, **kw)
+    assert (r.status == 0).all()
+    return X
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_pair_records_are_kept_for_wide_panels_only(precision):
+    b = _batch()
+    op = b.op
+    B = b.rhs_panel()
+    B4 = B[:, :4].contiguous()
+    B8 = torch.cat([B4, B4], 1)
+    ref = _solve(b, B4, precision, node_tiles=False)
+    X = _solve(b, B4, precision, node_tiles=True)
+    assert float(torch.linalg.norm(X - ref) / torch.linalg.norm(ref)) < 1e-8
+    (storage, t), = op._tiles.values()
+    assert t.reserved == 0
+    # the arrays of the layout test and no more: per tile, column and pair, each array padded to 256 bytes
+    last = max(getattr(t, n) or 0 for n in ("v64", "vlo2"))
+    pairs = int(_dev(storage, t.poff, t.n_tiles + 1, torch.int32)[-1])
+    assert storage.numel() - (last - storage.data_ptr()) < 3 * pairs * (8 if precision == "fp64" else 1) + 256
+    X8 = _solve(b, B8, precision, node_tiles=True)
+    assert len(op._tiles) == 2 and sorted(s[1].reserved > 0 for s in op._tiles.values()) == [False, True]
+    assert float(torch.linalg.norm(X8[:, :4] - ref) / torch.linalg.norm(ref)) < 1e-8
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_wide_panels_without_room_for_pair_records(precision, monkeypatch):
+    from feab200.device import ReducedOperator
+    b = _batch()
+    B4 = b.rhs_panel()[:, :4].contiguous()
+    B8 = torch.cat([B4, B4], 1)
+    ref = _solve(b, B8, precision, node_tiles=False)
+    build = ReducedOperator._build_tiles
+
+    def no_room(self, precision, pg, k):
+        if k >= 8:
+            raise torch.OutOfMemoryError("no room")
+        return build(self, precision, pg, k)
+
+    monkeypatch.setattr(ReducedOperator, "_build_tiles", no_room)
+    for _ in range(2):
+        X = _solve(b, B8, precision, node_tiles=True)
+        assert float(torch.linalg.norm(X - ref) / torch.linalg.norm(ref)) < 1e-8
+    assert all(t.reserved == 0 for _, t in b.op._tiles.values())
