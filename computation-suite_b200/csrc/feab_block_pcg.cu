@@ -763,12 +763,10 @@ __device__ __forceinline__ void finish_step_a(const BArgs& A, int it, int p, boo
       ProbState& Pm = A.ps[p];
       Pm.ticket_a = 0;
       Pm.x_pending = 0;
-      if (!reliable) {
-        Pm.pending = 0;
-        if (Pm.status != FEAB_OK) {
-          Pm.done = 1;
-          atomicSub(A.remaining, 1);
-        }
+      if (!reliable) Pm.pending = 0;
+      if (Pm.status != FEAB_OK) {
+        Pm.done = 1;
+        atomicSub(A.remaining, 1);
       }
     }
   }
@@ -919,10 +917,11 @@ __device__ __forceinline__ void pair_copy(PairStage& st, int buf, const PairReco
                : "memory");
 }
 
-// False when the copy does not arrive (some seconds).
+// False when the copy does not arrive.
+constexpr int kPairPolls = FEAB_WAIT_CYCLES > 0 ? 1 << 26 : 1;
 __device__ __forceinline__ bool pair_wait(PairStage& st, int buf, unsigned parity) {
   const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&st.full[buf]);
-  for (int spin = 0; spin < (1 << 22); ++spin) {
+  for (int poll = 0; poll < kPairPolls; ++poll) {
     uint32_t ok;
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
@@ -975,7 +974,8 @@ __device__ __forceinline__ void pair_apply(const PairRecord* __restrict__ rec, i
   }
 }
 
-// Item it's rows of the first KC panel columns, and the warp's column sums in sums.
+// Item it's rows of the first KC panel columns, and the warp's column sums in sums.  buf: the chunk to apply next,
+// or -1 once a copy has not come in, after which the warp does no more.
 template <int K, int KC>
 __device__ __forceinline__ void pair_item(const BArgs& A, int it, int p, bool reliable, PairStage& st, int& buf,
                                           unsigned (&parity)[2], double* sums) {
@@ -983,7 +983,6 @@ __device__ __forceinline__ void pair_item(const BArgs& A, int it, int p, bool re
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, t = lane & 3, r = lane >> 2;
   const double* __restrict__ src = reliable ? A.X : A.P0;
   double* __restrict__ dst = reliable ? A.R : A.AP;
-  bool arrived = true;
   double part[NL][W];
 #pragma unroll
   for (int j = 0; j < NL; ++j)
@@ -992,7 +991,7 @@ __device__ __forceinline__ void pair_item(const BArgs& A, int it, int p, bool re
   int t0, t1;
   item_tiles(A, it, t0, t1);
   // the warp's pairs 2 t0 + w, + 8, ..., 32 at a time: lane i holds the i-th one's records and rows
-  for (int q0 = 2 * t0 + w; q0 < 2 * t1; q0 += 32 * kWarps) {
+  for (int q0 = 2 * t0 + w; q0 < 2 * t1 && buf >= 0; q0 += 32 * kWarps) {
     const int q = q0 + lane * kWarps;
     int first = 0, last = 0, row0 = 0, rows = 0;
     if (q < 2 * t1) {
@@ -1031,7 +1030,10 @@ __device__ __forceinline__ void pair_item(const BArgs& A, int it, int p, bool re
     int cur = pi, steps = fetch(buf);
     while (steps > 0) {
       const int nxt = pi, more = fetch(buf ^ 1);           // pair and steps of the chunk behind this one
-      arrived = pair_wait(st, buf, parity[buf]) && arrived;
+      if (!__all_sync(FEAB_FULL_MASK, pair_wait(st, buf, parity[buf]))) {
+        buf = -1;
+        break;
+      }
       parity[buf] ^= 1u;
       pair_apply<K, KC>(st.rec[buf], steps, lane, src, acc);
       __syncwarp();                                        // every lane is done with the chunk
@@ -1072,7 +1074,7 @@ __device__ __forceinline__ void pair_item(const BArgs& A, int it, int p, bool re
       buf ^= 1;
     }
   }
-  if (!arrived && lane == 0) atomicCAS(&A.ps[p].status, FEAB_OK, FEAB_CUDA_ERROR);
+  if (buf < 0) atomicCAS(&A.ps[p].status, FEAB_OK, FEAB_CUDA_ERROR);
   // the rows' lanes of each column
 #pragma unroll
   for (int j = 0; j < NL; ++j)
@@ -1110,6 +1112,7 @@ __global__ void __launch_bounds__(kThreads, FEAB_PAIR_MINB(K)) k_bstep_a_pairs(B
     __syncthreads();
     finish_step_a<K>(A, it, p, reliable, sm);
   }
+  if (buf < 0) pause_for_copies();
 }
 
 // X += alpha P (x) and P = M R + beta P (dir) on rows [r0, r1) of the first KC columns: two adjacent

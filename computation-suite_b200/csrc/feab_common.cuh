@@ -97,6 +97,11 @@ struct WaitLimit {
 };
 // Before a CTA that gave up on a wait leaves: its own copies, whatever FEAB_WAIT_CYCLES.
 using DrainLimit = WaitLimit<(1ll << 32)>;
+// The same where it is not known which copies are under way: 2^21 cycles, a millisecond, for a microsecond's copies.
+__device__ __forceinline__ void pause_for_copies() {
+  for (const long long t0 = clock64(); clock64() - t0 < (1ll << 21);) {
+  }
+}
 
 // Number of SMs of the current device, cached per process.
 int sm_count();

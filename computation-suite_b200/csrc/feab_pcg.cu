@@ -429,6 +429,7 @@ __device__ __forceinline__ void finish_step_a(const PcgArgs& A, double (&part)[1
   PcgState* S = A.S_;
   double tot[1];
   if (grid_reduce<1>(part, A.partials, &S->ticket[0], tot) && threadIdx.x == 0) {
+    if (*(volatile int32_t*)&S->done) return;   // a copy of the ring's did not come in
     if (!cg) {
       S->rr64 = tot[0];
     } else {
@@ -543,8 +544,6 @@ struct RingTuning {
   static constexpr int kSmem = kRingWarps * kStages * kBytes;
 };
 
-constexpr int kRingSpinLimit = 1 << 22;   // polls of one copy's barrier (seconds)
-
 __device__ __forceinline__ void ring_copy(unsigned char* dst, const void* src, uint32_t bytes, uint32_t bar,
                                           bool stream, unsigned long long first) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
@@ -559,11 +558,13 @@ __device__ __forceinline__ void ring_copy(unsigned char* dst, const void* src, u
                  : "memory");
 }
 
+// False when the copy does not come in.
+constexpr int kRingPolls = FEAB_WAIT_CYCLES > 0 ? 1 << 22 : 1;
 __device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity) {
-  for (int spin = 0; spin < kRingSpinLimit; ++spin) {
+  for (int poll = 0; poll < kRingPolls; ++poll) {
     uint32_t ok;
     asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        "{\n .reg .pred p;\n " FEAB_MBAR_TRY ".parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
         : "=r"(ok)
         : "r"(bar), "r"(parity)
         : "memory");
@@ -582,7 +583,7 @@ __global__ void __launch_bounds__(kThreads, RingTuning<PREC>::kMinBlocks) k_step
   if (S->done) return;
   const int mode = S->mode, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double part[1] = {0.0};
-  bool arrived = true;   // every copy waited for came in
+  bool arrived = true;   // every copy waited for came in; after one that did not, the warp does no more
   if (PREC == FEAB_PREC_MIXED && mode == kModeReliable) {
     part[0] = sell_reliable_residual(A, lane);
   } else {
@@ -636,7 +637,8 @@ __global__ void __launch_bounds__(kThreads, RingTuning<PREC>::kMinBlocks) k_step
       const int W = __ldg(V.soff + sl + 1) - __ldg(V.soff + sl);
       double a0 = 0.0, a1 = 0.0, a2 = 0.0;
       for (int j = 0; j < W; j += 4) {
-        arrived = ring_wait((uint32_t)__cvta_generic_to_shared(&full[warp][buf]), parity) && arrived;
+        arrived = __all_sync(FEAB_FULL_MASK, ring_wait((uint32_t)__cvta_generic_to_shared(&full[warp][buf]), parity));
+        if (!arrived) break;
         const unsigned char* blk = ring + buf * R::kBytes;
         uint2 tq = reinterpret_cast<const uint2*>(blk + R::kValBytes)[lane];
         SellBlock<PREC> B;
@@ -671,6 +673,7 @@ __global__ void __launch_bounds__(kThreads, RingTuning<PREC>::kMinBlocks) k_step
           parity ^= 1u;
         }
       }
+      if (!arrived) break;
       double acc[3] = {a0, a1, a2};
       double own[3];
 #pragma unroll
@@ -695,9 +698,10 @@ __global__ void __launch_bounds__(kThreads, RingTuning<PREC>::kMinBlocks) k_step
       }
     }
   }
-  if (!arrived && lane == 0) {   // a copy did not come in
-    S->status = FEAB_CUDA_ERROR;
-    S->done = 1;
+  if (!arrived) {
+    pause_for_copies();
+    atomicExch(&S->status, FEAB_CUDA_ERROR);
+    atomicExch(&S->done, 1);
   }
   finish_step_a(A, part, mode != kModeReliable || PREC == FEAB_PREC_FP64);
 }

@@ -14,6 +14,16 @@ def _declare(lib, *names):
         f.restype, f.argtypes = L.SIGNATURES[n]
 
 
+def _cantilever(shape):
+    import feab200
+    mesh = feab200.box_mesh(2.0, 0.4, 0.4, *shape)
+    fs = feab200.FESystem(mesh, feab200.Hex8Solid3D(), sparse=True)
+    fs.assemble_stiffness(feab200.D_solid3d(feab200.Material(E=1.0, nu=0.3)), vectorized=True)
+    fs.fix_dofs(mesh.nodes_on_plane(0, 0.0), (0, 1, 2))
+    fs.add_nodal_force(mesh.nodes_on_plane(0, 2.0), 2, 1.0)
+    return fs
+
+
 def test_eigensolver(tmp_path, monkeypatch):
     from feab200 import _lib as L
     from feab200.pod import PodBasis
@@ -43,18 +53,14 @@ def test_eigensolver(tmp_path, monkeypatch):
 def test_band_solve(tmp_path, monkeypatch, shape):
     """Bands of 1, 5 and 9 tiles: clusters of 8 and of 16 CTAs."""
     import ctypes as C
-    import feab200
     from feab200 import _lib as L
     from feab200 import torch_sparse_solver as ts
     lib = wait_limits.build(tmp_path, "feab_band.cu")
     if lib is None:
         pytest.skip("no nvcc")
     _declare(lib, "feab_band_solve", "feab_band_solve_flag")
-    mesh = feab200.box_mesh(2.0, 0.4, 0.4, *shape)
-    fs = feab200.FESystem(mesh, feab200.Hex8Solid3D(), sparse=True)
-    fs.assemble_stiffness(feab200.D_solid3d(feab200.Material(E=1.0, nu=0.3)), vectorized=True)
-    fs.fix_dofs(mesh.nodes_on_plane(0, 0.0), (0, 1, 2))
-    fs.add_nodal_force(mesh.nodes_on_plane(0, 2.0), 2, 1.0)
+    fs = _cantilever(shape)
+    mesh = fs.mesh
     want = np.asarray(fs.solve_static())
     fac = fs.reduced_operator(want32=False).direct_factor(coords=mesh.nodes)
     st = L.stream_ptr(torch.device("cuda"))
@@ -85,3 +91,52 @@ def test_band_solve(tmp_path, monkeypatch, shape):
         assert int(header) == flag and bool(xp.isnan().any()) == bool(flag)
     assert torch.equal(fac.solve(b), x)
     assert np.array_equal(np.asarray(fs.solve_static()), want)
+
+
+def test_ring_of_the_sliced_pcg(tmp_path, monkeypatch):
+    """44,649 nodes: beyond the resident solve, so that step A streams through its ring."""
+    from feab200 import _lib as L
+    lib = wait_limits.build(tmp_path, "feab_pcg.cu", "feab_sell.cu", "feab_scan.cu")
+    if lib is None:
+        pytest.skip("no nvcc")
+    _declare(lib, "feab_pcg_solve")
+    fs = _cantilever((40, 32, 32))
+    for precision, tol in (("fp64", 1e-10), ("mixed", 1e-9)):
+        want = np.asarray(fs.solve_static(method="pcg", precision=precision, tol=tol))
+        with monkeypatch.context() as m:
+            m.setattr(L.lib, "feab_pcg_solve", lib.feab_pcg_solve)
+            with pytest.raises(L.FeabError):
+                fs.solve_static(method="pcg", precision=precision, tol=tol)
+            assert fs.last_solve_info.status == L.FEAB_CUDA_ERROR
+        assert np.array_equal(np.asarray(fs.solve_static(method="pcg", precision=precision, tol=tol)), want)
+
+
+def test_pair_records_of_the_block_pcg(tmp_path, monkeypatch):
+    """One problem that takes several chunks and two that take one: all report the error, none hangs."""
+    import oracle as O
+    from feab200 import _lib as L
+    from feab200.batched import ProblemBatch, block_pcg
+    lib = wait_limits.build(tmp_path, "feab_block_pcg.cu")
+    if lib is None:
+        pytest.skip("no nvcc")
+    _declare(lib, "feab_block_pcg_solve")
+    probs = []
+    rng = np.random.default_rng(3)
+    for sh in ((30, 6, 5), (3, 2, 2), (2, 1, 1)):
+        X, el = O.box_mesh(1.0, 0.5, 0.3, *sh)
+        probs.append((X, el, O.D_solid3d(5.0, 0.3), O.fixed_dofs_on_plane(X, 0, 0.0), rng.standard_normal((3 * len(X), 16))))
+    b = ProblemBatch(probs)
+    op, B = b.assemble(), b.rhs_panel()
+    kw = dict(max_groups=8, tune=False, node_tiles=True)
+    for precision in ("fp64", "mixed"):
+        for K in (8, 16):
+            Bk = B[:, :K].contiguous()
+            args = (op, b.row_bounds, Bk, [K, 3, K])
+            want, res = block_pcg(*args, tol=1e-9, precision=precision, tile_width=K, **kw)
+            assert (res.status == 0).all()
+            with monkeypatch.context() as m:
+                m.setattr(L.lib, "feab_block_pcg_solve", lib.feab_block_pcg_solve)
+                with pytest.raises(L.FeabError):
+                    block_pcg(*args, tol=1e-9, precision=precision, tile_width=K, **kw)
+            got, res = block_pcg(*args, tol=1e-9, precision=precision, tile_width=K, **kw)
+            assert (res.status == 0).all() and torch.equal(got, want)

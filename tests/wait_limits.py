@@ -22,7 +22,8 @@ void count_launches(uint64_t) {}
 
 
 def build(tmp, *sources):
-    """A ctypes library of these sources of csrc, or None without nvcc."""
+    """A ctypes library of these sources of csrc, or None without nvcc.  Its state (cached graphs) is its own
+    beside libfeab200's in the process: no unique symbols, its own definitions first."""
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(nvcc):
         return None
@@ -32,5 +33,6 @@ def build(tmp, *sources):
     subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-shared", "-Xcompiler",
                     "-fPIC", "--expt-relaxed-constexpr", "-DFEAB_WAIT_CYCLES=0", "-I", os.path.join(ROOT, "include"),
                     "-I", CSRC, "-o", lib, common, *[os.path.join(CSRC, s) for s in sources], "-cudart",
-                    "static"], check=True, capture_output=True)
+                    "static", "--threads", "4", "-Xcompiler",
+                    "-fno-gnu-unique", "-Xlinker", "-Bsymbolic"], check=True, capture_output=True)
     return C.CDLL(lib)
