@@ -72,6 +72,12 @@ def layer_order(op, coords, sample=2048):
     return order, int(n_layers[2])
 
 
+def _spread(G, count, dev):
+    """`count` of the indices 0 .. G - 1, evenly spread, the last among them.  In FP64: FP32 numbers are whole
+    multiples of 2 from 2^24 on, and the last could be G."""
+    return torch.linspace(0, G - 1, count, dtype=torch.float64, device=dev).to(torch.int64)
+
+
 def _layers(op, coords, sample=2048):
     """The order of layer_order, and the layers along the three axes, ascending."""
     p = op.pattern
@@ -80,7 +86,7 @@ def _layers(op, coords, sample=2048):
     G = gp.numel() - 1
     dof = torch.nonzero(p.free_map >= 0).flatten()
     key = torch.as_tensor(np.ascontiguousarray(coords, dtype=float)).to(dev)[dof[gp[:-1]] // 3]
-    some = torch.linspace(0, G - 1, min(G, int(sample)), device=dev).to(torch.int64)
+    some = _spread(G, min(G, int(sample)), dev)
     start = rp[gp[some]]
     lens = rp[gp[some] + 1] - start
     src = torch.repeat_interleave(torch.arange(some.numel(), device=dev), lens)

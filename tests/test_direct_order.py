@@ -75,6 +75,14 @@ def test_layer_order_on_graded_spacing_is_a_bijection():
     assert sorted(dof_permutation(op, order).tolist()) == list(range(op.n))
 
 
+@pytest.mark.parametrize("G", [1, 2, 2047, 2048, 2049, 2 ** 24 + 2, 20000004, 33554435, 79000001])
+def test_sampled_nodes_are_nodes(G):
+    from feab200.direct import _spread
+    s = _spread(G, min(G, 2048), "cpu")
+    assert len(s) == min(G, 2048) and int(s[0]) == 0 and int(s[-1]) == G - 1
+    assert bool((s[1:] > s[:-1]).all())
+
+
 def _chosen(X, el, fixed):
     """The band that the direct solve chooses, by its ordering, and the bands of the orderings that it had
     before the one in layers."""
