@@ -279,9 +279,10 @@ def spmv_bytes(op, precision):
 
 
 def spmv_roofline(op, precision, reps, peak_gbs):
-    """Average duration of the PCG's SpMV kernel (the sliced SELL-32 product for fp64 and mixed,
+    """Average duration of the stand-alone SpMV kernel (the sliced SELL-32 product for fp64 and mixed,
     the CSR one for fp32) with CUDA events on the launching stream; L2 is flushed before each
-    launch (L2Flush: a 256 MB write, then a 256 MB read)."""
+    launch (L2Flush: a 256 MB write, then a 256 MB read).  The PCG's step A streams the same sliced
+    operator, at this size through a ring of bulk copies (k_step_a_ring): pcg_iteration times that."""
     import torch
     from feab200.device import sell_spmv, spmv, tuned_lanes_per_group
     dev = op.vals64.device
@@ -313,7 +314,7 @@ def spmv_roofline(op, precision, reps, peak_gbs):
     kern = {"fp64": "k_sell_spmv<FP64>", "fp32": f"k_spmv<float, {lpg}>", "mixed": "k_sell_spmv<MIXED>"}[precision]
     return {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak_gbs, "unit": "GB/s",
             "frac": round(achieved / peak_gbs, 3), "traffic": None,
-            "kernel": f"{kern} (the SpMV of PCG step A, {precision})",
+            "kernel": f"{kern} (stand-alone SpMV, {precision})",
             "bytes_per_launch": int(nbytes),
             "csr_formula_bytes": int(bytes_csr), "launch_us": round(t * 1e6, 2)}
 

@@ -685,7 +685,8 @@ __global__ void __launch_bounds__(kBandThreads, 1) k_band_factor(BandWork B) {
 // reduction, and one hop to another SM), while a CTA's tiles per block row (bands / C) come in
 // faster than that; wide bands are bound by what 16 SMs read (about 1.4 TB/s).  Measured, two
 // launches per block row -> one kernel, both directions: 64x16x16 elements (867 block rows, 28
-// bands) 19.0 -> 2.1 ms, 96x24x24 (2,813, 59 bands) 63.3 -> 8.3 ms (6.5 with 31 bands), 33x9x8 (140, 9) 2.07 -> 0.36 ms.
+// bands) 19.0 -> 2.1 ms (1.84 with the 15 bands of nodes in layers), 96x24x24 (2,813, 59 bands) 63.3 -> 8.3 ms (6.4
+// with 31 bands), 33x9x8 (140, 9) 2.07 -> 0.36 ms (0.27 with 5 bands).
 constexpr int kSolveWarps = 16;
 constexpr int kSolveThreads = 32 * kSolveWarps;       // that compute; one more warp fetches the tiles
 constexpr int kSolveCta = kSolveThreads + 32;

@@ -19,10 +19,11 @@
 // deterministic.  Converged problems are skipped; the host polls a "problems remaining"
 // counter one CUDA-graph chunk behind.
 //
-// Precisions: FEAB_PREC_FP64 (reference recurrence) and FEAB_PREC_MIXED (SpMM on 7-byte values,
-// 44-bit mantissas, in difference form with FP64 vectors; per problem, an FP64 residual replacement with the
-// FP64 values whenever a column's residual dropped by reliable_delta; convergence on the FP64
-// residual).
+// Precisions: FEAB_PREC_FP64 (reference recurrence) and FEAB_PREC_MIXED (per problem, an FP64 residual
+// replacement with the FP64 values whenever a column's residual dropped by reliable_delta; convergence on
+// that residual).  The mixed SpMM is on 7-byte values, 44-bit mantissas, in difference form with FP64
+// vectors, except where step A has pair records: these hold the FP64 values, and the replacements are then
+// checks of a recurrence that is already on the exact K.
 #include <algorithm>
 #include <cmath>
 #include "feab_common.cuh"
@@ -875,11 +876,14 @@ __global__ void __launch_bounds__(kThreads, TILES ? FEAB_BLOCK_MINB : FEAB_BLOCK
 // and 64 columns the operand's tensor work is 27 % of the kernel's time, its HBM bytes 10 %).  In the group and tile paths
 // every value reached the lanes as its own shared-memory broadcast, and the L1 data path set the pace;
 // here a value is one lane's register.  A whole FP64 block step at 418,176 rows, in us, with row groups
-// and with pairs: 8 columns 196 and 144, 16: 312 and 264, 32: 482 and 449, 64: 838 and 798.
+// and with pairs: 8 columns 196 and 144, 16: 312 and 264, 32: 482 and 449, 64: 838 and 770; at 1,382,976
+// rows, 16: 1,276 and 839, 64: 2,977 and 2,658.
 //
-// Columns of the records applied before the next gathers, and blocks per SM: by measurement (16 columns,
-// 8 and 2: 264 us, 4 and 4: 266 but 60 more with the residual replacements' spills; 64 columns, 1 and 2:
-// 795, 2 and 2: 907; 8 columns, 4 and 4: 146, 8 and 2: 168).
+// Columns of the records applied before the next gathers, and blocks per SM: by measurement, us per step
+// at 418,176 rows (16 columns, 8 and 2: 264, 4 and 4: 266 but 60 more with the residual replacements'
+// spills; 64 columns, 1 and 2: 795, 2 and 2: 907; 8 columns, 4 and 4: 146, 8 and 2: 168; 32 columns, FP64
+// and mixed, 4 and 2: 454 and 448, 1 and 2: 435 and 445, 2 and 2: 472 and 478, 8 and 2: 515 and 527, 2 and
+// 3: 531 and 523, 4 and 1: 585 and 596).
 #ifndef FEAB_PAIR_UNROLL
 #define FEAB_PAIR_UNROLL(K) ((K) == 64 ? 1 : ((K) == 16 ? 8 : 4))
 #endif

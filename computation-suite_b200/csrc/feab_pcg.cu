@@ -512,8 +512,10 @@ __global__ void __launch_bounds__(kThreads, SellTuning<PREC>::kMinBlocks) k_step
 // whatever the bytes (mixed in 246 MB; at 96x24x24 mixed was slower than FP64); with the ring the HBM's
 // rate sets the pace, and a part of K that L2 can hold beside the vectors is read without the
 // evict-first hint, so that it is still there in the next iteration.  The best part is that of some 68 MB
-// with nine vectors, about half of L2: at 128x32x32 mixed 88.2 ms per solve without, 85.2 with 46 MB of
-// K kept, 87.7 with 62 MB, 99 with 123 MB.
+// with nine vectors, about half of L2.  us per iteration with a part of 68 MB, of 54 and 82, and without:
+//                 96x24x24                112x28x28               128x32x32               144x36x36
+//   mixed   28.4  28.4 29.3  30.1   35.5  35.9 36.6  39.4   48.9  49.5 50.6  51.7   70.7  71.6 74.5  73.0
+//   FP64    27.3  28.2 27.1  33.4   45.7  46.5 47.1  50.3   56.9  58.1 58.0  60.6   83.9  86.3 85.5  85.9
 // Whole solves, register path -> ring: 128x32x32 mixed (1e-9) 91.7 -> 85.2 ms, FP64 (1e-10) 109.7 -> 103.8;
 // 96x24x24 mixed 50.4 -> 38.2, FP64 44.0 -> 37.5.
 //
@@ -1314,7 +1316,8 @@ void fill_matrix(const feab_csr* M, PcgArgs* A) {
 
 void fill_sell(const feab_csr* M, const feab_sell_operator* D, PcgArgs* A) {
   A->sell = sell_view(M, D);
-  // the slices that the ring has L2 keep: 68 MB less nine vectors, of K's 26 or 20 bytes per 3 rows' entry
+  // the slices that the ring has L2 keep: 68 MB (see the ring) less nine vectors, of K's 26 or 20 bytes per
+  // 3 rows' entry
   const double room = 68e6 - 72.0 * M->n, bytes = (D->kind == FEAB_PREC_FP64 ? 26.0 : 20.0) / 3.0 * (double)M->nnz;
   A->sell.keep = room <= 0.0 || bytes <= 0.0 ? 0 : (int)std::min(32.0, 32.0 * room / bytes);
   A->use_sell = 1;

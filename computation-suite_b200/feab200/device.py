@@ -84,7 +84,7 @@ class ReducedOperator:
 
     def direct_factor(self, coords=None):
         """The banded Cholesky factor of K_ff (direct.BandCholesky; coords: the mesh's node
-        coordinates, for the ordering along the longest axis), cached."""
+        coordinates, for the ordering in layers), cached."""
         if self._direct is None:
             from .direct import BandCholesky
             self._direct = BandCholesky(self, coords=coords)
@@ -92,7 +92,8 @@ class ReducedOperator:
 
     def diff_operator(self):
         """The difference-form operator of the mixed block-PCG (7-byte values, 44-bit mantissas;
-        feab_diff_operator_build), cached."""
+        feab_diff_operator_build), cached.  Panels of 8 columns or more on node tiles need it to be given but
+        multiply with the tiles' FP64 pair records."""
         if self._diff is None:
             p = self.pattern
             if p.group_ptr is None or p.free_map.numel() == 0:

@@ -9,7 +9,7 @@ vectors) with a Rayleigh-Ritz step, every product on the GPU:
                                      M X by the block SpMM (feab_block_spmm)
     Kr = Y^T K Y,  Mr = Y^T M Y      block SpMMs and FP64 panel Grams (feab_panel_gram)
     Kr v = lambda Mr v               Mr = Q L Q^T, then the eigenpairs of L^-1/2 Q^T Kr Q L^-1/2
-                                     (feab_symeig_jacobi, one CTA, k <= 64; p x p products only)
+                                     (feab_symeig_jacobi, k <= 64; p x p products only)
     X  = Y V                         M-orthonormal Ritz vectors, lambda ascending (feab_panel_small)
 
 until the n_modes lowest Ritz values change by less than ``tol`` (relative), or stop decreasing

@@ -3,7 +3,7 @@
 ``PodBasis.fit`` keeps the reference's signature and rank rule (n_modes / energy_threshold,
 _select_rank pod.py:163-176).  The FP64 economy SVD of the reference (pod.py:140-147) is
 replaced by the method of snapshots: the 64 x 64 Gram matrix X^T X, its FP64 eigenvalues by a
-one-CTA Jacobi solver (feab_symeig_jacobi), singular values sqrt(lambda), and modes
+Jacobi solver on a cluster of three CTAs (feab_symeig_jacobi), singular values sqrt(lambda), and modes
 U = X V / sigma.  Three Gram kernels; the default ``gram="auto"`` takes the int8 one for FP32
 snapshots and the FP64 one for FP64 snapshots (whose values carry more bits than seven 7-bit
 digits keep):

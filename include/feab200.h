@@ -297,7 +297,7 @@ int32_t feab_sell_operator_build(const feab_csr* A, const int32_t* dof_of, int32
 int32_t feab_sell_spmv(const feab_csr* A, const feab_sell_operator* op, const double* x, double* y,
                        cudaStream_t stream);
 
-/* y = A x with the PCG's SpMV kernel (same code and launch shape as one PCG step's SpMV).
+/* y = A x on its own, by the product of the PCG's CSR steps or the stand-alone sliced one.
  * FEAB_PREC_FP64: x, y double, vals64; FEAB_PREC_FP32: x, y float, vals32;
  * FEAB_PREC_MIXED: x, y double, difference form through a MIXED sliced operator (sell);
  * FEAB_PREC_FP64 with an FP64 sliced operator: the sliced product instead of the CSR one.
@@ -393,7 +393,9 @@ int32_t feab_tile_operator_build_k(const feab_csr* A, const feab_diff_operator* 
 /* tiles (optional, of the solve's precision, built with this batch's problem boundaries): the
  * SpMM of every CG step walks node tiles instead of single row groups; work items must then
  * start and end on tile boundaries (items of a multiple of FEAB_TILE_GROUPS groups from each
- * problem's first group do).  The mixed solve's FP64 residual replacements use A and diff. */
+ * problem's first group do).  The mixed solve's FP64 residual replacements use A and diff.  With pair
+ * records, panels of 8 columns or more make every product with the FP64 values that A had when the tiles
+ * were built, residual replacements included. */
 int32_t feab_block_pcg_solve(const feab_csr* A, const feab_diff_operator* diff, const feab_tile_operator* tiles,
                              const feab_batch* batch, const double* dinv64, const double* B, double* X,
                              const feab_pcg_params* params, void* workspace, size_t workspace_bytes,
