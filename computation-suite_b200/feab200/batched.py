@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import ctypes as C
 import json
+import math
 import os
 import tempfile
 from dataclasses import dataclass
@@ -249,19 +250,38 @@ def save_tuning(key, shape, path=None):
         pass                   # a read-only home directory keeps the in-process cache only
 
 
-def _step_cost_us(op, items, B_panel, cols, precision, short=4, long=20, problem_groups=None):
-    """Device time of one block-PCG step over this panel: two runs of tol 0 (no column
-    converges) of `short` and `long` steps, timed with CUDA events; the difference over
-    long - short removes setup and graph capture."""
-    times = []
-    for steps in (short, long, short, long):
+def _step_cost_us(op, items, B_panel, cols, precision, short=4, long=20, problem_groups=None, reps=2):
+    """Device time of one block-PCG step over this panel: `reps` runs of tol 0 (no column
+    converges) of `short` and of `long` steps, timed with CUDA events; the difference of the shortest
+    over long - short removes setup and graph capture."""
+    times = {short: [], long: []}
+    for steps in (short, long) * reps:
         a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         a.record()
         _block_pcg_call(op, *items, B_panel, cols, 0.0, steps, precision, 0.1, 8, problem_groups)
         b.record()
         b.synchronize()
-        times.append(a.elapsed_time(b) * 1e3)
-    return max(1e-3, (min(times[1], times[3]) - min(times[0], times[2])) / (long - short))
+        times[steps].append(a.elapsed_time(b) * 1e3)
+    return max(1e-3, (min(times[long]) - min(times[short])) / (long - short))
+
+
+def _cheapest(candidates, cost):
+    """The candidate of least cost(candidate, steps, repetitions), and its cost.  Every candidate is timed
+    over 16 steps, twice.  A pause of the host of half a millisecond in both short runs makes 25 us of a
+    step of 130 disappear (one choice in eight was wrong for it: 64 columns at 55,488 rows, 147 ms a
+    solve for 128), so that those within 30 % of the least, and whichever leads then, are timed again,
+    three times over 8 ms or 64 steps."""
+    costs = {c: cost(c, 16, 2) for c in candidates}
+    near = 1.3 * min(costs.values())
+    again = [c for c in candidates if costs[c] <= near]
+    sure = set()
+    while again:
+        for c in again:
+            costs[c] = cost(c, int(min(64, max(16, math.ceil(8000.0 / costs[c])))), 3)
+            sure.add(c)
+        best = min(candidates, key=costs.get)
+        again = [] if best in sure else [best]
+    return best, costs[best]
 
 
 def tuned_block_shape(op, row_bounds, B_panel, cols, precision="fp64", candidates=None):
@@ -286,14 +306,16 @@ def tuned_block_shape(op, row_bounds, B_panel, cols, precision="fp64", candidate
     if candidates is None:
         candidates = [(g, w, nt) for g in ITEM_GROUPS for w in PANELS if 16 <= w <= K or w == K
                       for nt in (False, True) if not (nt and g % TILE_GROUPS)]
-    best = None
-    for g, w, nt in candidates:
-        items = _work_items(gp, np.asarray(row_bounds), g)
-        ct = np.clip(cols, 0, w)
-        pgroups = _problem_groups(gp, np.asarray(row_bounds)) if nt else None
-        cost = _step_cost_us(op, items, B_panel[:, :w].contiguous(), ct, precision, problem_groups=pgroups) * (K // w)
-        if best is None or cost < best.us_per_step:
-            best = BlockShape(g, w, cost, nt)
+    pgroups = _problem_groups(gp, np.asarray(row_bounds))
+
+    def cost(candidate, steps, reps):
+        g, w, nt = candidate
+        return _step_cost_us(op, _work_items(gp, np.asarray(row_bounds), g), B_panel[:, :w].contiguous(),
+                             np.clip(cols, 0, w), precision, short=4, long=4 + steps,
+                             problem_groups=pgroups if nt else None, reps=reps) * (K // w)
+
+    (g, w, nt), us = _cheapest(candidates, cost)
+    best = BlockShape(g, w, us, nt)
     _tuned_block[key] = best
     save_tuning(key, best)
     return best

@@ -172,6 +172,26 @@ def test_reference_arm_runs_whole_steps_without_the_cuda_library():
     assert set(line["config"]) == {"workload", "n_free", "nnz", "tol", "l2", "parallelism"}
 
 
+@pytest.mark.parametrize("disturbed", [None, (64, 64, False), (16, 16, False), (64, 64, True)])
+def test_block_tuning_survives_a_disturbed_timing(disturbed):
+    """One candidate's first timing is off, as by a pause of the host in its short or its long runs: the
+    least costly one is chosen all the same."""
+    from feab200 import batched as bt
+    true = {(g, w, nt): 110.0 + 25.0 * (g != 64) + 20.0 * (64 // w - 1) + 20.0 * (not nt)
+            for g in bt.ITEM_GROUPS for w in (16, 32, 64) for nt in (False, True)}
+    best = (64, 64, True)
+    calls = []
+
+    def cost(c, steps, reps):
+        calls.append(c)
+        pause = 400.0 if c == disturbed and calls.count(c) == 1 else 0.0     # us
+        return true[c] + (pause if c == best else -pause) / steps
+
+    shape, us = bt._cheapest(list(true), cost)
+    assert shape == best and us == true[best]
+    assert len(calls) <= 2 * len(true)
+
+
 def test_block_tuning_of_another_build_is_not_taken(tmp_path, monkeypatch):
     """A shape that was timed with other kernels is in the cache file under a key of its own."""
     from feab200 import _lib
